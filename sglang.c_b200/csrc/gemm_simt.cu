@@ -82,92 +82,112 @@ gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, const float
     }
   }
 }
-// Many rows and many features (a prompt portion of the 32-bit path): a block of 128 x 128 outputs,
-// a thread 8 x 8 of them (two 4 x 4 corners 64 apart each way, so that a warp's shared-memory reads
-// are two broadcasts and one contiguous run), which is four times the arithmetic per shared-memory
-// read of the 64 x 64 kernel (NW = 1: 128 x 64 outputs, 8 x 4 a thread, for products whose 128 x 128
-// blocks would leave most of the GPU idle).  The next k-tile is on its way from global memory into registers
-// while this one is multiplied.  One accumulator per output, k ascending: the same bits again.
-constexpr int LM = 128, LK = 16, LP = LM + 4;
+__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool on) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = on ? 16 : 0;                         // 0: the 16 bytes are filled with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int NW>
-__global__ void __launch_bounds__(256, 2)          // two blocks an SM: at most 128 registers a thread
-gemm_simt_large_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                       float* __restrict__ out, float* __restrict__ residual, int M, int N, int K, int lda,
-                       int ldo, int act) {
-  __shared__ __align__(16) float As[2][LK][LP];
-  constexpr int LN = 64 * NW;
-  __shared__ __align__(16) float Ws[2][LK][LN + 4];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  const int m0 = blockIdx.y * LM, n0 = blockIdx.x * LN;
-  const int lrow = tid / 4, lk = (tid % 4) * 4;      // rows lrow and lrow + 64, four k from lk
-  float4 ra[2], rw[NW];
-  auto gload = [&](int k0) {
-    const int k = k0 + lk;
+__device__ __forceinline__ float part(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// Many rows (a prompt portion of the 32-bit path), blocks of 64 x 64.  A warp has the 64 rows of 16 features, a lane
+// 8 x 4 outputs; rows of A and W lie in shared memory as they lie in memory (36 floats apart: eight rows' 16-byte
+// reads fall on all 32 banks), brought by asynchronous copies four k-tiles ahead, and leave it four k ahead of
+// their use.  A 16-byte read costs one pass for the eight rows all quarters of a warp share and four for the four
+// features, so the rows are on the side that costs one.  One accumulator per output, k ascending: the same
+// bits from every kernel of this file.
+// 672 x 768 x 768: 63.6 -> 32.6 us, over K 3,072 245 -> 111 us, 1,872 x 768 over K 3,072 347 -> 254 us (35 TFLOP/s).  Bound
+// by how many registers a multiply-add's operands can be read a cycle (ncu: 0.58 of the multiply-add pipe, issue
+// slots 0.70, warps ready): the pair kernel below is what gets around that where there are rows enough.
+constexpr int LK = 32, LPITCH = LK + 4;
+
+constexpr int TILE_M = 64, TILE_N = 64, TILE_ST = 4;
+
+__global__ void __launch_bounds__(128, 3)
+gemm_simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                      float* __restrict__ out, float* __restrict__ residual, int M, int N, int K, int lda,
+                      int ldo, int act) {
+  constexpr int BMT = TILE_M, BNT = TILE_N, TN = 4, ST = TILE_ST, STAGE = (BMT + BNT) * LPITCH;
+  constexpr int STEP = 16;                           // rows a pass of the block's 16-byte copies covers
+  extern __shared__ __align__(16) float ring[];      // [ST][BMT rows of A, then BNT of W][LPITCH]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = blockIdx.y * BMT, n0 = blockIdx.x * BNT;
+  const int n_tiles = (K + LK - 1) / LK;
+  const int crow = tid / 8, ck = (tid % 8) * 4;
+  // (rows beyond the last are copies of it: their outputs are not stored)
+  auto ask_w = [&](int tile, int st) {
+    float* to = ring + st * STAGE + BMT * LPITCH + crow * LPITCH + ck;
+    const int k = tile * LK + ck;
+    const bool on = k < K;                           // (K is a multiple of 4: a piece lies inside or outside)
+    const float* from = W + (on ? k : 0);
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int m = m0 + lrow + 64 * r;
-      ra[r] = (m < M && k < K) ? *reinterpret_cast<const float4*>(A + (size_t)m * lda + k)
-                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-#pragma unroll
-    for (int r = 0; r < NW; r++) {
-      const int n = n0 + lrow + 64 * r;
-      rw[r] = (n < N && k < K) ? *reinterpret_cast<const float4*>(W + (size_t)n * K + k)
-                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
+    for (int r = 0; r < BNT / STEP; r++)
+      cp_async16_zfill(to + r * STEP * LPITCH, from + (size_t)min(n0 + crow + r * STEP, N - 1) * K, on);
   };
-  auto sstore = [&](int buf) {
+  auto ask_a = [&](int tile, int st) {
+    float* to = ring + st * STAGE + crow * LPITCH + ck;
+    const int k = tile * LK + ck;
+    const bool on = k < K;
+    const float* from = A + (on ? k : 0);
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int c = lrow + 64 * r;
-      As[buf][lk + 0][c] = ra[r].x; As[buf][lk + 1][c] = ra[r].y;
-      As[buf][lk + 2][c] = ra[r].z; As[buf][lk + 3][c] = ra[r].w;
-    }
-#pragma unroll
-    for (int r = 0; r < NW; r++) {
-      const int c = lrow + 64 * r;
-      Ws[buf][lk + 0][c] = rw[r].x; Ws[buf][lk + 1][c] = rw[r].y;
-      Ws[buf][lk + 2][c] = rw[r].z; Ws[buf][lk + 3][c] = rw[r].w;
-    }
+    for (int r = 0; r < BMT / STEP; r++)
+      cp_async16_zfill(to + r * STEP * LPITCH, from + (size_t)min(m0 + crow + r * STEP, M - 1) * lda, on);
   };
-  float acc[8][4 * NW];
+  for (int t = 0; t < ST; t++) {
+    if (t < n_tiles) { ask_a(t, t); ask_w(t, t); }
+    cp_async_commit();
+  }
+  const int row = lane & 7, feat = warp * 4 * TN + (lane >> 3);     // + 8 i, + 4 j
+  float acc[8][TN];
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
-    for (int j = 0; j < 4 * NW; j++) acc[i][j] = 0.0f;
-  gload(0);
-  sstore(0);
+    for (int j = 0; j < TN; j++) acc[i][j] = 0.0f;
+  float4 a[2][8], w[2][TN];
+  auto take = [&](int to, int st, int k) {           // four k of this lane's rows and features into registers
+    const float* as = ring + st * STAGE + row * LPITCH + k;
+    const float* ws = ring + st * STAGE + (BMT + feat) * LPITCH + k;
+#pragma unroll
+    for (int j = 0; j < TN; j++) w[to][j] = *reinterpret_cast<const float4*>(ws + 4 * j * LPITCH);
+#pragma unroll
+    for (int i = 0; i < 8; i++) a[to][i] = *reinterpret_cast<const float4*>(as + 8 * i * LPITCH);
+  };
+  cp_async_wait<ST - 1>();
   __syncthreads();
-  for (int k0 = 0, buf = 0; k0 < K; k0 += LK, buf ^= 1) {
-    const bool more = k0 + LK < K;
-    if (more) gload(k0 + LK);
+  take(0, 0, 0);
+  int st = 0;
+  for (int tile = 0; tile < n_tiles; tile++) {
 #pragma unroll
-    for (int k = 0; k < LK; k++) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][k][ty * 4]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][k][64 + ty * 4]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      float w[4 * NW];
-#pragma unroll
-      for (int r = 0; r < NW; r++) {
-        const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][k][64 * r + tx * 4]);
-        w[4 * r] = w4.x; w[4 * r + 1] = w4.y; w[4 * r + 2] = w4.z; w[4 * r + 3] = w4.w;
+    for (int g = 0; g < LK / 4; g++) {
+      // the next group's values leave shared memory while this group's are multiplied
+      if (g + 1 < LK / 4) {
+        take((g + 1) & 1, st, (g + 1) * 4);
+      } else {
+        cp_async_wait<ST - 2>();
+        __syncthreads();                             // tile + 1 has landed; this tile's stage is free
+        if (tile + ST < n_tiles) { ask_a(tile + ST, st); ask_w(tile + ST, st); }
+        cp_async_commit();
+        if (++st == ST) st = 0;
+        take(0, st, 0);                              // (behind the last tile: a stage that is not used)
       }
 #pragma unroll
-      for (int i = 0; i < 8; i++)
+      for (int e = 0; e < 4; e++)
 #pragma unroll
-        for (int j = 0; j < 4 * NW; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+          for (int j = 0; j < TN; j++) acc[i][j] = fmaf(part(a[g & 1][i], e), part(w[g & 1][j], e), acc[i][j]);
     }
-    if (more) sstore(buf ^ 1);                       // (its readers passed the barrier of the tile before)
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 8; i++) {
-    const int m = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
+    const int m = m0 + row + 8 * i;
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4 * NW; j++) {
-      const int n = n0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
+    for (int j = 0; j < TN; j++) {
+      const int n = n0 + feat + 4 * j;
       if (n >= N) continue;
       float v = acc[i][j];
       if (bias) v += bias[n];
@@ -179,77 +199,325 @@ gemm_simt_large_kernel(const float* __restrict__ A, const float* __restrict__ W,
   }
 }
 
-// Up to 16 rows (a decode step of the 32-bit path): the product is a read of the weights once, so
-// what counts is bytes in flight.  A block takes 16 output features; the tiles of A (16 x 32 k)
-// and W (16 x 32 k) come through a ring of eight shared-memory stages by asynchronous 16-byte
-// copies, seven k-tiles ahead of the arithmetic.  A thread owns 2 rows of 1 feature and adds
-// k = 0..K-1 in ascending order with the same fused multiply-add as the kernel above, so an
-// output element has the same bits whichever of the two kernels computed it.
-constexpr int SM_ = 16, SN = 16, SK = 32, ST = 8, PITCH = SK + 4;
+// Few rows (a decode step of the 32-bit path): the weights are read once, and an output is a chain of K
+// dependent multiply-adds (four clocks each), which is what bounds the narrow products.  A block is one
+// warp with 4 MR rows of 8 NF features, a lane MR x NF outputs, with no barrier between warps, and few
+// instructions beside the chain.  Tiles of 64 k come through a ring of ST stages by asynchronous
+// 16-byte copies; the first stages' weights are asked for before the wait for the kernel ahead.  A
+// 16-byte read costs one pass for the eight features all quarters of the warp share and four for the
+// four rows (rows lie 68 floats apart: no bank conflicts).  k ascending, one accumulator: the same bits
+// as the kernels above.
+// 8 rows: 768 columns 7.4 -> 4.8 us, over K 3,072 23.6 -> 12.6 us (its chain alone 6.4), 50,257 columns 84 -> 44 us (154 MB:
+// 24 us at the copy rate).
+constexpr int SK = 64, PITCH = SK + 4;
 
-__device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, bool on) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const int n = on ? 16 : 0;                         // 0: the 16 bytes are filled with zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+template <int MR, int NF, int ST>
+__global__ void __launch_bounds__(32)
+gemm_simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                      float* __restrict__ out, float* __restrict__ residual, int M, int N, int K, int lda,
+                      int ldo, int act) {
+  constexpr int RA = 4 * MR, RW = 8 * NF, STAGE = (RA + RW) * PITCH;
+  extern __shared__ __align__(16) float ring[];      // [ST][RA rows, then RW weight rows][PITCH]
+  const int lane = threadIdx.x;
+  const int m0 = blockIdx.y * RA, n0 = blockIdx.x * RW;
+  const int n_tiles = (K + SK - 1) / SK;
+  const int crow = lane >> 4, ck = (lane & 15) * 4;  // a pass of the warp's copies: two rows
+  // Where this lane's pieces come from (one warp has to issue everything: what a tile costs beside its chain is
+  // kept to the copies themselves).  Weight rows beyond the last are copies of it, their outputs are not stored;
+  // token rows beyond the last are zeros (copies would have every block ask for the same lines again).
+  const float* pw[RW / 2];
+  const float* pa[RA / 2];
+  bool on_a[RA / 2];
+#pragma unroll
+  for (int r = 0; r < RW / 2; r++) pw[r] = W + (size_t)min(n0 + crow + 2 * r, N - 1) * K + ck;
+#pragma unroll
+  for (int r = 0; r < RA / 2; r++) {
+    const int m = m0 + crow + 2 * r;
+    on_a[r] = m < M;
+    pa[r] = A + (on_a[r] ? (size_t)m * lda : 0) + ck;
+  }
+  const unsigned to0 = (unsigned)__cvta_generic_to_shared(ring) + (crow * PITCH + ck) * 4;
+  auto copy = [](unsigned to, const float* from, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(from), "r"(on ? 16 : 0));
+  };
+  auto ask_w = [&](int tile, int st) {
+    const bool on = tile * SK + ck < K;              // (K is a multiple of 4: a piece lies inside or outside)
+    const int at = on ? tile * SK : 0;
+#pragma unroll
+    for (int r = 0; r < RW / 2; r++) copy(to0 + (st * STAGE + (RA + 2 * r) * PITCH) * 4, pw[r] + (on ? at : -ck), on);
+  };
+  auto ask_a = [&](int tile, int st) {
+    const bool on = tile * SK + ck < K;
+    const int at = on ? tile * SK : 0;
+#pragma unroll
+    for (int r = 0; r < RA / 2; r++) copy(to0 + (st * STAGE + 2 * r * PITCH) * 4, pa[r] + (on ? at : -ck), on && on_a[r]);
+  };
+  for (int t = 0; t < ST - 1; t++) {
+    if (t < n_tiles) { ask_w(t, t); ask_a(t, t); }
+    cp_async_commit();
+  }
+  float acc[MR][NF];
+#pragma unroll
+  for (int i = 0; i < MR; i++)
+#pragma unroll
+    for (int j = 0; j < NF; j++) acc[i][j] = 0.0f;
+  const int row = lane >> 3, feat = lane & 7;        // + 4 i, + 8 j
+  int st = 0, st_in = ST - 1;
+  for (int tile = 0; tile < n_tiles; tile++) {
+    cp_async_wait<ST - 2>();
+    __syncwarp();                                    // tile `tile` has landed; the stage of tile-1 is free
+    if (tile + ST - 1 < n_tiles) { ask_w(tile + ST - 1, st_in); ask_a(tile + ST - 1, st_in); }
+    cp_async_commit();
+    const float* as = ring + st * STAGE + row * PITCH;
+    const float* ws = ring + st * STAGE + (RA + feat) * PITCH;
+    if (++st == ST) st = 0;
+    if (++st_in == ST) st_in = 0;
+#pragma unroll(NF * MR > 8 ? 4 : 16)
+    for (int k = 0; k < SK; k += 4) {
+      float4 a[MR], w[NF];
+#pragma unroll
+      for (int i = 0; i < MR; i++) a[i] = *reinterpret_cast<const float4*>(as + 4 * i * PITCH + k);
+#pragma unroll
+      for (int j = 0; j < NF; j++) w[j] = *reinterpret_cast<const float4*>(ws + 8 * j * PITCH + k);
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+#pragma unroll
+        for (int i = 0; i < MR; i++)
+#pragma unroll
+          for (int j = 0; j < NF; j++) acc[i][j] = fmaf(part(a[i], e), part(w[j], e), acc[i][j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MR; i++) {
+    const int m = m0 + row + 4 * i;
+#pragma unroll
+    for (int j = 0; j < NF; j++) {
+      const int n = n0 + feat + 8 * j;
+      if (m >= M || n >= N) continue;
+      float v = acc[i][j];
+      if (bias) v += bias[n];
+      v = apply_act(v, act);
+      const size_t o = (size_t)m * ldo + n;
+      if (residual) residual[o] = residual[o] + v;
+      else out[o] = v;
+    }
+  }
 }
 
-__global__ void __launch_bounds__(128)
-gemm_simt_small_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
-                       float* __restrict__ out, float* __restrict__ residual, int M, int N, int K, int lda,
-                       int ldo, int act) {
-  __shared__ __align__(16) float As[ST][SM_][PITCH];
-  __shared__ __align__(16) float Ws[ST][SN][PITCH];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  const int m0 = blockIdx.y * SM_, n0 = blockIdx.x * SN;
-  const int lrow = tid / 8, lk = (tid % 8) * 4;      // this thread's 16-byte piece of a tile row
-  const int n_tiles = (K + SK - 1) / SK;
-  auto issue = [&](int tile) {
-    if (tile < n_tiles) {
-      const int st = tile % ST, k = tile * SK + lk;
-      const bool kin = k < K;                        // (K is a multiple of 4: a piece lies inside or outside)
-      const int m = m0 + lrow;
-      cp_async16_zfill(&As[st][lrow][lk], A + (size_t)(m < M ? m : 0) * lda + (kin ? k : 0), kin && m < M);
-      const int n = n0 + lrow;
-      cp_async16_zfill(&Ws[st][lrow][lk], W + (size_t)(n < N ? n : 0) * K + (kin ? k : 0), kin && n < N);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+// A load that stays where it is written: ahead of the arithmetic that covers its way from memory.
+__device__ __forceinline__ float4 load_early(const float* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+constexpr int PK = 16;
+
+// Many rows and features: blocks of 128 x 64 or 128 x 128, a thread 8 x 8 outputs (runs of 4, so that a warp's reads are
+// broadcasts and contiguous), the tiles turned to k-major on their way through registers.  Two features of a row
+// are one packed multiply-add, each half rounded as a single one, which reads its operands as pairs.  1,872 rows:
+// 2,304 columns 170 -> 155 us (43 TFLOP/s of the 73.6 that packed multiply-adds alone reach here), 3,072 columns
+// 264 -> 204 us.
+template <int BMT, int BNT, int BLOCKS>
+__global__ void __launch_bounds__(BMT / 8 * (BNT / 8), BLOCKS)
+gemm_simt_pair_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                      float* __restrict__ out, float* __restrict__ residual, int M, int N, int K, int lda,
+                      int ldo, int act) {
+  constexpr int TX = BNT / 8, THREADS = BMT / 8 * TX, C4 = 2;              // C4: runs of 4 features a thread has
+  constexpr int NA = BMT * PK / 4 / THREADS, NB = BNT * PK / 4 / THREADS;  // 16-byte pieces a thread stages
+  constexpr int WX = TX < 8 ? TX : 8;                                      // a warp: WX x 32 / WX threads
+  static_assert(NA * THREADS * 4 == BMT * PK && NB * THREADS * 4 == BNT * PK, "");
+  __shared__ __align__(16) float As[2][PK][BMT + 4];
+  __shared__ __align__(16) float Ws[2][PK][BNT + 4];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx = warp % (TX / WX) * WX + lane % WX, ty = warp / (TX / WX) * (32 / WX) + lane / WX;
+  const int m0 = blockIdx.y * BMT, n0 = blockIdx.x * BNT;
+  const int lrow = tid / 4, lk = (tid % 4) * 4;      // rows lrow, lrow + THREADS / 4, ...; four k from lk
+  // (rows beyond the last are copies of it: their outputs are not stored)
+  const float* pa[NA];
+  const float* pw[NB];
+#pragma unroll
+  for (int r = 0; r < NA; r++) pa[r] = A + (size_t)min(m0 + lrow + THREADS / 4 * r, M - 1) * lda;
+#pragma unroll
+  for (int r = 0; r < NB; r++) pw[r] = W + (size_t)min(n0 + lrow + THREADS / 4 * r, N - 1) * K;
+  float4 ra[NA], rw[NB];
+  auto load_a = [&](int k) {
+    const bool on = k < K;                           // (K is a multiple of 4: a piece lies inside or outside)
+#pragma unroll
+    for (int r = 0; r < NA; r++) ra[r] = on ? load_early(pa[r] + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   };
-  for (int t = 0; t < ST - 1; t++) issue(t);
-  float acc[2] = {0.0f, 0.0f};
-  for (int tile = 0; tile < n_tiles; tile++) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
-    __syncthreads();                                 // tile `tile` has landed; the stage of tile-1 is free
-    issue(tile + ST - 1);
-    const int st = tile % ST;
+  auto load_w = [&](int k) {
+    const bool on = k < K;
 #pragma unroll
-    for (int k = 0; k < SK; k += 4) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[st][2 * ty][k]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[st][2 * ty + 1][k]);
-      const float4 w0 = *reinterpret_cast<const float4*>(&Ws[st][tx][k]);
-      acc[0] = fmaf(a0.x, w0.x, acc[0]); acc[1] = fmaf(a1.x, w0.x, acc[1]);
-      acc[0] = fmaf(a0.y, w0.y, acc[0]); acc[1] = fmaf(a1.y, w0.y, acc[1]);
-      acc[0] = fmaf(a0.z, w0.z, acc[0]); acc[1] = fmaf(a1.z, w0.z, acc[1]);
-      acc[0] = fmaf(a0.w, w0.w, acc[0]); acc[1] = fmaf(a1.w, w0.w, acc[1]);
+    for (int r = 0; r < NB; r++) rw[r] = on ? load_early(pw[r] + k) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  };
+  auto sstore = [&](int buf) {
+#pragma unroll
+    for (int r = 0; r < NA; r++) {
+      const int c = lrow + THREADS / 4 * r;
+      As[buf][lk + 0][c] = ra[r].x; As[buf][lk + 1][c] = ra[r].y;
+      As[buf][lk + 2][c] = ra[r].z; As[buf][lk + 3][c] = ra[r].w;
+    }
+#pragma unroll
+    for (int r = 0; r < NB; r++) {
+      const int c = lrow + THREADS / 4 * r;
+      Ws[buf][lk + 0][c] = rw[r].x; Ws[buf][lk + 1][c] = rw[r].y;
+      Ws[buf][lk + 2][c] = rw[r].z; Ws[buf][lk + 3][c] = rw[r].w;
+    }
+  };
+  unsigned long long acc[8][2 * C4];                 // [row][pair of features]
+#pragma unroll
+  for (int i = 0; i < 8; i++)
+#pragma unroll
+    for (int j = 0; j < 2 * C4; j++) acc[i][j] = 0ull;
+  load_w(lk);
+  load_a(lk);
+  sstore(0);
+  __syncthreads();
+  for (int k0 = 0, buf = 0; k0 < K; k0 += PK, buf ^= 1) {
+    const bool more = k0 + PK < K;
+    if (more) { load_a(k0 + PK + lk); load_w(k0 + PK + lk); }
+    float4 a0[2], a1[2];
+    ulonglong2 w4[2][C4];
+    auto take = [&](int to, int k) {
+      a0[to] = *reinterpret_cast<const float4*>(&As[buf][k][ty * 4]);
+      a1[to] = *reinterpret_cast<const float4*>(&As[buf][k][BMT / 2 + ty * 4]);
+#pragma unroll
+      for (int r = 0; r < C4; r++) w4[to][r] = *reinterpret_cast<const ulonglong2*>(&Ws[buf][k][BNT / C4 * r + tx * 4]);
+    };
+    take(0, 0);
+#pragma unroll
+    for (int k = 0; k < PK; k++) {
+      if (k + 1 < PK) take((k + 1) & 1, k + 1);
+      const float4 x = a0[k & 1], y = a1[k & 1];
+      const unsigned long long a[8] = {pack2(x.x, x.x), pack2(x.y, x.y), pack2(x.z, x.z), pack2(x.w, x.w),
+                                       pack2(y.x, y.x), pack2(y.y, y.y), pack2(y.z, y.z), pack2(y.w, y.w)};
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int r = 0; r < C4; r++) {
+          fma2(acc[i][2 * r], a[i], w4[k & 1][r].x);
+          fma2(acc[i][2 * r + 1], a[i], w4[k & 1][r].y);
+        }
+    }
+    if (more) sstore(buf ^ 1);                       // (its readers passed the barrier of the tile before)
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    const int m = m0 + (i < 4 ? ty * 4 + i : BMT / 2 + ty * 4 + i - 4);
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 2 * C4; j++) {
+      const float2 both = *reinterpret_cast<const float2*>(&acc[i][j]);
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int n = n0 + BNT / C4 * (j / 2) + tx * 4 + (j % 2) * 2 + e;
+        if (n >= N) continue;
+        float v = e ? both.y : both.x;
+        if (bias) v += bias[n];
+        v = apply_act(v, act);
+        const size_t o = (size_t)m * ldo + n;
+        if (residual) residual[o] = residual[o] + v;
+        else out[o] = v;
+      }
     }
   }
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const int m = m0 + 2 * ty + i;
-    const int n = n0 + tx;
-    if (m >= M || n >= N) continue;
-    float v = acc[i];
-    if (bias) v += bias[n];
-    v = apply_act(v, act);
-    const size_t o = (size_t)m * ldo + n;
-    if (residual) residual[o] = residual[o] + v;
-    else out[o] = v;
+}
+
+struct SimtArgs {
+  const float *A, *W, *bias;
+  float *out, *residual;
+  int M, N, K, lda, ldo, act;
+};
+
+// None of these kernels starts early behind the kernel ahead (programmatic dependent launch): blocks that wait
+// beside the running ones take up room unevenly, and a launch of about one block an SM then lasts twice as long (63
+// against 33 us for 672 x 768 x 768; 24 tokens for eight requests 25.6 against 23.1 ms).
+template <int MR, int NF, int ST>
+int launch_rows(const SimtArgs& p, cudaStream_t stream) {
+  constexpr int smem = ST * (4 * MR + 8 * NF) * PITCH * 4;
+  auto* kernel = gemm_simt_rows_kernel<MR, NF, ST>;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
   }
+  return sglc_launch(kernel, dim3((p.N + 8 * NF - 1) / (8 * NF), (p.M + 4 * MR - 1) / (4 * MR)), dim3(32), smem, stream, 1,
+                     false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K, p.lda, p.ldo, p.act);
+}
+
+int launch_tile(const SimtArgs& p, cudaStream_t stream) {
+  constexpr int smem = TILE_ST * (TILE_M + TILE_N) * LPITCH * 4;
+  const cudaError_t e = cudaFuncSetAttribute(gemm_simt_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  return sglc_launch(gemm_simt_tile_kernel, dim3((p.N + TILE_N - 1) / TILE_N, (p.M + TILE_M - 1) / TILE_M), dim3(128), smem,
+                     stream, 1, false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K, p.lda, p.ldo, p.act);
+}
+
+template <int BMT, int BNT, int BLOCKS>
+int launch_pair(const SimtArgs& p, cudaStream_t stream) {
+  return sglc_launch(gemm_simt_pair_kernel<BMT, BNT, BLOCKS>, dim3((p.N + BNT - 1) / BNT, (p.M + BMT - 1) / BMT),
+                     dim3(BMT / 8 * (BNT / 8)), 0, stream, 1, false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K,
+                     p.lda, p.ldo, p.act);
+}
+
+// Tuning hook: 0 (default) lets the launcher choose the kernel.
+int g_simt_form = 0;
+enum { FORM_ROWS = 1, FORM_ROWS_WIDE, FORM_TILE, FORM_PAIR, FORM_PAIR_WIDE };
+
+int choose_form(int M, int N) {
+  if (M <= 64) return FORM_ROWS;
+  // Else by time, in us at K = 768 (every form's grows with K alike), measured at 200 to 2,048 rows: so many
+  // full waves of resident blocks, and a rest that takes less the fewer blocks an SM has.
+  auto tiles = [&](int bm, int bn) { return (long long)((M + bm - 1) / bm) * ((N + bn - 1) / bn); };
+  auto waves = [](long long blocks, int resident, const double* us) {       // us[i]: i + 1 blocks an SM
+    const long long wave = 148LL * resident, rest = blocks % wave;
+    return (double)(blocks / wave) * us[resident - 1] + (rest ? us[(rest + 147) / 148 - 1] : 0.0);
+  };
+  static const double tile_us[] = {33.0, 58.0, 69.0}, pair_us[] = {64.0, 94.0, 126.0}, wide_us[] = {95.0, 154.0};
+  const double rows = 6.6 * (double)tiles(16, 32) / 148.0;
+  const double t[] = {rows < 17.0 ? 17.0 : rows, waves(tiles(64, 64), 3, tile_us), waves(tiles(128, 64), 3, pair_us),
+                      waves(tiles(128, 128), 2, wide_us)};
+  int best = 0;
+  for (int i = 1; i < 4; i++)
+    if (t[i] < t[best]) best = i;
+  return FORM_ROWS_WIDE + best;
+}
+
+int simt_f32(const SimtArgs& p, cudaStream_t stream) {
+  switch (g_simt_form ? g_simt_form : choose_form(p.M, p.N)) {
+    case FORM_ROWS_WIDE: return launch_rows<4, 4, 4>(p, stream);
+    case FORM_TILE: return launch_tile(p, stream);
+    case FORM_PAIR: return launch_pair<128, 64, 3>(p, stream);
+    case FORM_PAIR_WIDE: return launch_pair<128, 128, 2>(p, stream);
+  }
+  // Few rows, by the narrowest: the chain of K multiply-adds bounds a product, so a lane has one output; wider
+  // ones, where shared-memory reads do, more; the vocabulary's head, where enough weights have to be on their way,
+  // most, with a short ring so that more warps fit.  (us at 8 rows, one / two / four features a lane: 768 columns
+  // 4.8 (a row a lane) / 9.1 / 11.4, over K 3,072 12.6 / 29.9 / 37.9, 2,304 columns 7.5 / 9.5 / 11.9, 50,257
+  // columns 67.9 / 52.7 / 43.8.)
+  if (p.M <= 4) return p.N <= 8192 ? launch_rows<1, 1, 10>(p, stream) : launch_rows<1, 2, 4>(p, stream);
+  if (p.N > 8192) return p.M <= 8 ? launch_rows<2, 4, 3>(p, stream) : launch_rows<4, 4, 3>(p, stream);
+  if (p.M <= 16) {
+    if (p.N <= 1024) return launch_rows<1, 1, 10>(p, stream);
+    return p.N <= 2304 ? launch_rows<2, 1, 10>(p, stream) : launch_rows<2, 2, 8>(p, stream);
+  }
+  return p.N <= 1024 ? launch_rows<2, 1, 10>(p, stream) : launch_rows<2, 4, 5>(p, stream);
 }
 }  // namespace
 
 // A: [M,K] with row stride lda (elements); W: [N,K] contiguous; bias: float[N] or null.
 // If `residual` is given (float [M,N], row stride ldo) the result is added into it and
 // `out` is not written; else `out` ([M,N], row stride ldo, out_dtype) takes it.
+SGLC_API void sglc_gemm_simt_set_form(int form) { g_simt_form = form; }
+
 SGLC_API int sglc_gemm_simt(const void* A, const void* W, const float* bias, void* out,
                             float* residual, int M, int N, int K, int lda, int ldo, int in_dtype,
                             int out_dtype, int act, cudaStream_t stream) {
@@ -259,16 +527,8 @@ SGLC_API int sglc_gemm_simt(const void* A, const void* W, const float* bias, voi
   if (grid.y > 65535) return SGLC_ERR_UNSUPPORTED;
   const bool f32 = in_dtype == SGLC_F32 && (out_dtype == SGLC_F32 || residual);
   const bool wide_loads = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
-  const int m_blocks = (M + LM - 1) / LM;
-  if (f32 && wide_loads && M > BM && m_blocks <= 65535 && (long long)m_blocks * ((N + 127) / 128) >= 240) {
-    gemm_simt_large_kernel<2><<<dim3((N + 127) / 128, m_blocks), 256, 0, stream>>>(
-        (const float*)A, (const float*)W, bias, (float*)out, residual, M, N, K, lda, ldo, act);
-  } else if (f32 && wide_loads && M > BM && m_blocks <= 65535 && (long long)m_blocks * ((N + 63) / 64) >= 120) {
-    gemm_simt_large_kernel<1><<<dim3((N + 63) / 64, m_blocks), 256, 0, stream>>>(
-        (const float*)A, (const float*)W, bias, (float*)out, residual, M, N, K, lda, ldo, act);
-  } else if (f32 && wide_loads && M <= SM_) {
-    gemm_simt_small_kernel<<<dim3((N + SN - 1) / SN, (M + SM_ - 1) / SM_), 128, 0, stream>>>(
-        (const float*)A, (const float*)W, bias, (float*)out, residual, M, N, K, lda, ldo, act);
+  if (f32 && wide_loads) {
+    return simt_f32(SimtArgs{(const float*)A, (const float*)W, bias, (float*)out, residual, M, N, K, lda, ldo, act}, stream);
   } else if (in_dtype == SGLC_F32 && (out_dtype == SGLC_F32 || residual)) {
     gemm_simt_kernel<float, float, float><<<grid, 256, 0, stream>>>(
         (const float*)A, (const float*)W, bias, (float*)out, residual, M, N, K, lda, ldo, act);
