@@ -246,6 +246,309 @@ attention_simt_kernel(const TQ* __restrict__ q, int q_stride, const TC* __restri
   }
 }
 
+// ---- the 32-bit path's own two forms (head sizes that are multiples of 4, up to 128; no extensions) -----------
+// The same arithmetic in the same order as the kernel above, so the same bits; what differs is who does it and
+// how the tiles come.  The kernel above spends its time on shared-memory reads (of 128 multiply-adds a lane and
+// tile, 104 reads) and on waits for tiles that nothing covers.
+__device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool on) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+struct F32Args {
+  const float* q; int q_stride;
+  const float* cache;
+  const int* block_table; int bt_stride;
+  const int* token_req; const int* positions;
+  float* out; int o_stride;
+  int T, H, Hkv, D, page_size;
+  float scale;
+  int window, n_pages, kv_shared;
+  int* err;
+};
+// key p of request row bt: its key row (the value row lies v_off behind it); null where the page id is bad
+__device__ __forceinline__ const float* f32_row(const F32Args& a, const int* bt, int p, size_t page_elems, size_t head_off) {
+  const int page = bt[p / a.page_size];
+  if (!sglc_index_ok(page, a.n_pages, a.err)) return nullptr;
+  return a.cache + (size_t)page * page_elems + head_off + (size_t)(p % a.page_size) * a.D;
+}
+
+// Prompt portions: a warp has FP_Q consecutive tokens, so a key or a value leaves shared memory once for all of
+// them; eight warps a block share the tiles, which come by asynchronous copies one tile ahead.
+// 1,872 tokens of three prompts (up to 780 keys), 12 heads of 64: 280 -> 170 us.  Bound by shared-memory reads (224 passes
+// a warp and tile beside 128 cycles of multiply-adds); eight tokens a warp would halve them but leave one block
+// an SM: 194 us.  The last tokens of a prompt, which see the most keys, go first.
+constexpr int FP_Q = 4, FP_W = 8 * FP_Q;
+template <int NA>      // head sizes up to 32 NA
+__global__ void __launch_bounds__(256)
+attention_f32_portion_kernel(const F32Args a) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ int s_req[FP_W], s_lo[FP_W], s_pos[FP_W];
+  pdl_launch_dependents();
+  const int D = a.D, DP = D + 4, tile_floats = 32 * (DP + D);
+  float* qs = smem + 2 * tile_floats;                // [FP_W][D]
+  float* pw = qs + FP_W * D;                         // [FP_W][32]: a tile's weights
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.x, hk = h / (a.H / a.Hkv);
+  const int t0 = (gridDim.y - 1 - blockIdx.y) * FP_W;                    // (a prompt's last tokens see the most keys: first)
+  const size_t page_elems = (size_t)(a.kv_shared ? 1 : 2) * a.Hkv * a.page_size * D;
+  const size_t head_off = (size_t)hk * a.page_size * D, v_off = a.kv_shared ? 0 : (size_t)a.Hkv * a.page_size * D;
+  pdl_wait();
+  if (tid < FP_W) {
+    const int t = t0 + tid;
+    const bool on = t < a.T;
+    const int pos = on ? a.positions[t] : -1;
+    s_req[tid] = on ? a.token_req[t] : -1;
+    s_pos[tid] = pos;
+    s_lo[tid] = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
+  }
+  for (int x = tid; x < FP_W * D; x += 256) {
+    const int w = x / D, d = x - w * D;
+    qs[x] = t0 + w < a.T ? a.q[(size_t)(t0 + w) * a.q_stride + (size_t)h * D + d] : 0.0f;
+  }
+  __syncthreads();
+  int my_req[FP_Q], my_lo[FP_Q], my_pos[FP_Q];
+  float m[FP_Q], l[FP_Q], acc[FP_Q][NA];
+#pragma unroll
+  for (int i = 0; i < FP_Q; i++) {
+    my_req[i] = s_req[warp * FP_Q + i]; my_lo[i] = s_lo[warp * FP_Q + i]; my_pos[i] = s_pos[warp * FP_Q + i];
+    m[i] = -INFINITY; l[i] = 0.0f;
+#pragma unroll
+    for (int n = 0; n < NA; n++) acc[i][n] = 0.0f;
+  }
+  const float* qv = qs + warp * FP_Q * D;
+  float* pv = pw + warp * FP_Q * 32;
+  for (int lead = 0; lead < FP_W; lead++) {
+    const int rl = s_req[lead];
+    if (rl < 0 || (lead > 0 && s_req[lead - 1] == rl)) continue;         // not the start of a run
+    int lo_min = s_lo[lead], pos_max = s_pos[lead];
+    for (int w = lead + 1; w < FP_W && s_req[w] == rl; w++) {
+      lo_min = min(lo_min, s_lo[w]);
+      pos_max = max(pos_max, s_pos[w]);
+    }
+    const int* bt = a.block_table + (size_t)rl * a.bt_stride;
+    const int kt_first = lo_min / 32, kt_end = pos_max / 32 + 1;
+    auto ask = [&](int kt) {                          // eight threads bring one key and its value
+      if (kt < kt_end) {
+        float* ks = smem + (kt & 1) * tile_floats;
+        float* vs = ks + 32 * DP;
+        const int j = tid >> 3, part = tid & 7, p = kt * 32 + j;
+        const float* kp = (p >= lo_min && p <= pos_max) ? f32_row(a, bt, p, page_elems, head_off) : nullptr;
+        for (int d = part * 4; d < D; d += 32) {
+          copy16_or_zero(ks + j * DP + d, kp ? kp + d : a.cache, kp != nullptr);
+          copy16_or_zero(vs + j * D + d, kp ? kp + v_off + d : a.cache, kp != nullptr);
+        }
+      }
+      copies_commit();
+    };
+    __syncthreads();                                  // (the run before is done with the tiles)
+    ask(kt_first);
+    for (int kt = kt_first; kt < kt_end; kt++) {
+      ask(kt + 1);
+      copies_wait<1>();
+      __syncthreads();                                // tile kt has landed
+      const int key0 = kt * 32;
+      bool on[FP_Q];
+      bool any = false;
+#pragma unroll
+      for (int i = 0; i < FP_Q; i++) {
+        on[i] = my_req[i] == rl && key0 <= my_pos[i] && key0 + 31 >= my_lo[i];
+        any = any || on[i];
+      }
+      if (any) {
+        const float* ks = smem + (kt & 1) * tile_floats;
+        const float* vs = ks + 32 * DP;
+        const float* kr = ks + lane * DP;
+        float sc[FP_Q], corr[FP_Q];
+#pragma unroll
+        for (int i = 0; i < FP_Q; i++) sc[i] = 0.0f;
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+          const float4 k4 = *reinterpret_cast<const float4*>(kr + d);
+#pragma unroll
+          for (int i = 0; i < FP_Q; i++) {
+            const float4 q4 = *reinterpret_cast<const float4*>(qv + i * D + d);
+            sc[i] = fmaf(q4.x, k4.x, sc[i]);
+            sc[i] = fmaf(q4.y, k4.y, sc[i]);
+            sc[i] = fmaf(q4.z, k4.z, sc[i]);
+            sc[i] = fmaf(q4.w, k4.w, sc[i]);
+          }
+        }
+        const int key = key0 + lane;
+#pragma unroll
+        for (int i = 0; i < FP_Q; i++) {
+          corr[i] = 1.0f;
+          if (!on[i]) continue;
+          const bool valid = key >= my_lo[i] && key <= my_pos[i];
+          const float s = valid ? sc[i] * a.scale : -INFINITY;
+          const float m_new = fmaxf(m[i], warp_max(s));
+          corr[i] = expf(m[i] - m_new);                                 // (first tile: exp(-inf) = 0)
+          const float p = valid ? expf(s - m_new) : 0.0f;
+          l[i] = l[i] * corr[i] + warp_sum(p);
+          m[i] = m_new;
+          pv[i * 32 + lane] = p;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < FP_Q; i++)
+#pragma unroll
+          for (int n = 0; n < NA; n++)
+            if (on[i]) acc[i][n] *= corr[i];
+#pragma unroll 2
+        for (int j = 0; j < 32; j += 4) {
+          float4 p4[FP_Q];
+#pragma unroll
+          for (int i = 0; i < FP_Q; i++) p4[i] = *reinterpret_cast<const float4*>(pv + i * 32 + j);
+#pragma unroll
+          for (int n = 0; n < NA; n++) {
+            const int d = min(lane + 32 * n, D - 1);                    // (lanes beyond the head size: not stored)
+            const float v0 = vs[j * D + d], v1 = vs[(j + 1) * D + d], v2 = vs[(j + 2) * D + d], v3 = vs[(j + 3) * D + d];
+#pragma unroll
+            for (int i = 0; i < FP_Q; i++)
+              if (on[i]) {
+                float x = acc[i][n];
+                x = fmaf(p4[i].x, v0, x);
+                x = fmaf(p4[i].y, v1, x);
+                x = fmaf(p4[i].z, v2, x);
+                x = fmaf(p4[i].w, v3, x);
+                acc[i][n] = x;
+              }
+          }
+        }
+        __syncwarp();
+      }
+      __syncthreads();                                // everybody is done with tile kt: the next but one may come
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < FP_Q; i++) {
+    const int t = t0 + warp * FP_Q + i;
+    if (t >= a.T) continue;
+    const float inv = 1.0f / l[i];
+    float* op = a.out + (size_t)t * a.o_stride + (size_t)h * D;
+#pragma unroll
+    for (int n = 0; n < NA; n++)
+      if (lane + 32 * n < D) op[lane + 32 * n] = acc[i][n] * inv;
+  }
+}
+
+// Single tokens: a block has one (token, head).  Rounds of two tiles come through three stages of asynchronous copies;
+// while warps 0 and 1 walk the softmax and the sums over the values of one round (a half of the head's columns
+// each, the chain from tile to tile), warps 2 and 3 make the next round's scores, a tile each.
+// Eight requests of 60 to 140 keys, 12 heads: 12.3 -> 6.2 us in a decode step's chain.
+template <int NA>      // head sizes up to 64 NA
+__global__ void __launch_bounds__(128)
+attention_f32_single_kernel(const F32Args a) {
+  extern __shared__ __align__(16) float smem[];
+  __shared__ float scores[2][64], pw[2][32];
+  pdl_launch_dependents();
+  const int D = a.D, DP = D + 4, stage_floats = 64 * (DP + D);
+  float* qs = smem + 3 * stage_floats;               // [D]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = blockIdx.x, h = blockIdx.y, hk = h / (a.H / a.Hkv);
+  const size_t page_elems = (size_t)(a.kv_shared ? 1 : 2) * a.Hkv * a.page_size * D;
+  const size_t head_off = (size_t)hk * a.page_size * D, v_off = a.kv_shared ? 0 : (size_t)a.Hkv * a.page_size * D;
+  pdl_wait();
+  const int pos = a.positions[t];
+  const int lo = (a.window > 0 && pos - a.window + 1 > 0) ? pos - a.window + 1 : 0;
+  const int* bt = a.block_table + (size_t)a.token_req[t] * a.bt_stride;
+  const int kt_first = lo / 32, n_rounds = (pos / 32 + 1 - kt_first + 1) / 2;
+  auto ask = [&](int r) {                             // two threads bring one key and its value
+    if (r < n_rounds) {
+      float* ks = smem + (r % 3) * stage_floats;
+      float* vs = ks + 64 * DP;
+      const int j = tid >> 1, p = (kt_first + 2 * r) * 32 + j;
+      const float* kp = (p >= lo && p <= pos) ? f32_row(a, bt, p, page_elems, head_off) : nullptr;
+      for (int d = (tid & 1) * 4; d < D; d += 8) {
+        copy16_or_zero(ks + j * DP + d, kp ? kp + d : a.cache, kp != nullptr);
+        copy16_or_zero(vs + j * D + d, kp ? kp + v_off + d : a.cache, kp != nullptr);
+      }
+    }
+    copies_commit();
+  };
+  auto score = [&](int r) {                           // by warps 2 and 3
+    const int j = (warp - 2) * 32 + lane, key = (kt_first + 2 * r) * 32 + j;
+    const float* kr = smem + (r % 3) * stage_floats + j * DP;
+    float sc = 0.0f;
+#pragma unroll 8
+    for (int d = 0; d < D; d += 4) {
+      const float4 q4 = *reinterpret_cast<const float4*>(qs + d);
+      const float4 k4 = *reinterpret_cast<const float4*>(kr + d);
+      sc = fmaf(q4.x, k4.x, sc);
+      sc = fmaf(q4.y, k4.y, sc);
+      sc = fmaf(q4.z, k4.z, sc);
+      sc = fmaf(q4.w, k4.w, sc);
+    }
+    scores[r & 1][j] = (key >= lo && key <= pos) ? sc * a.scale : -INFINITY;
+  };
+  ask(0);
+  ask(1);
+  for (int d = tid; d < D; d += 128) qs[d] = a.q[(size_t)t * a.q_stride + (size_t)h * D + d];
+  copies_wait<1>();
+  __syncthreads();
+  if (warp >= 2) score(0);
+  float m = -INFINITY, l = 0.0f, acc[NA];
+#pragma unroll
+  for (int n = 0; n < NA; n++) acc[n] = 0.0f;
+  for (int r = 0; r < n_rounds; r++) {
+    copies_wait<0>();
+    __syncthreads();                                  // round r + 1 has landed, round r's scores are there, stage r - 1 is free
+    ask(r + 2);
+    if (warp >= 2) {
+      if (r + 1 < n_rounds) score(r + 1);
+    } else {
+      const float* vs = smem + (r % 3) * stage_floats + 64 * DP;
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        if ((kt_first + 2 * r + u) * 32 > pos) break;
+        const float s = scores[r & 1][u * 32 + lane];
+        const float m_new = fmaxf(m, warp_max(s));
+        const float corr = expf(m - m_new);                             // (first tile: exp(-inf) = 0)
+        const float p = s != -INFINITY ? expf(s - m_new) : 0.0f;
+        l = l * corr + warp_sum(p);
+        m = m_new;
+        pw[warp][lane] = p;
+        __syncwarp();
+        float pj[32];
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 p4 = *reinterpret_cast<const float4*>(&pw[warp][j]);
+          pj[j] = p4.x; pj[j + 1] = p4.y; pj[j + 2] = p4.z; pj[j + 3] = p4.w;
+        }
+#pragma unroll
+        for (int n = 0; n < NA; n++) {
+          const int d = min((warp + 2 * n) * 32 + lane, D - 1);
+          float x = acc[n] * corr;
+#pragma unroll
+          for (int j = 0; j < 32; j++) x = fmaf(pj[j], vs[(u * 32 + j) * D + d], x);
+          acc[n] = x;
+        }
+        __syncwarp();
+      }
+    }
+  }
+  if (warp < 2) {
+    const float inv = 1.0f / l;
+    float* op = a.out + (size_t)t * a.o_stride + (size_t)h * D;
+#pragma unroll
+    for (int n = 0; n < NA; n++) {
+      const int d = (warp + 2 * n) * 32 + lane;
+      if (d < D) op[d] = acc[n] * inv;
+    }
+  }
+}
+
+template <typename K>
+static int launch_f32(K* kernel, dim3 grid, int threads, size_t smem, const F32Args& a, cudaStream_t stream) {
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  return sglc_launch(kernel, grid, dim3(threads), smem, stream, 1, true, a);
+}
+
 // q: first query element of token 0 (rows q_stride apart, heads side by side); cache: one
 // layer's pages; block_table: [n_requests][bt_stride] page ids; token_req[t]: row of the
 // block table for token t; positions[t]: absolute position of token t (its own key is the
@@ -270,6 +573,23 @@ static int attention_simt_run(const void* q, int q_stride, const void* cache,
   if (H > 65535 || D > (ext ? 768 : 256)) return SGLC_ERR_UNSUPPORTED;
   // single tokens of many requests share nothing: a token a block; portions: eight tokens a block
   const bool single = max_q_len <= 1;
+  if (!ext && act_dtype == SGLC_F32 && cache_dtype == SGLC_F32 && D % 4 == 0 && D <= 128 && ((uintptr_t)cache & 15) == 0) {
+    F32Args a = {};
+    a.q = (const float*)q; a.q_stride = q_stride; a.cache = (const float*)cache; a.block_table = block_table;
+    a.bt_stride = bt_stride; a.token_req = token_req; a.positions = positions; a.out = (float*)out; a.o_stride = o_stride;
+    a.T = T; a.H = H; a.Hkv = Hkv; a.D = D; a.page_size = page_size; a.scale = scale; a.window = window;
+    a.n_pages = n_pages; a.kv_shared = kv_shared; a.err = err;
+    if (single) {
+      const size_t smem = ((size_t)3 * 64 * (2 * D + 4) + D) * sizeof(float);
+      return D <= 64 ? launch_f32(attention_f32_single_kernel<1>, dim3(T, H), 128, smem, a, stream)
+                     : launch_f32(attention_f32_single_kernel<2>, dim3(T, H), 128, smem, a, stream);
+    }
+    const size_t smem = ((size_t)2 * 32 * (2 * D + 4) + (size_t)FP_W * (D + 32)) * sizeof(float);
+    const dim3 grid(H, (T + FP_W - 1) / FP_W);
+    if (grid.y > 65535) return SGLC_ERR_UNSUPPORTED;
+    return D <= 64 ? launch_f32(attention_f32_portion_kernel<2>, grid, 256, smem, a, stream)
+                   : launch_f32(attention_f32_portion_kernel<4>, grid, 256, smem, a, stream);
+  }
   const int W = single ? 1 : 8;
   const size_t smem = ((size_t)32 * (D % 4 == 0 ? D + 4 : D + 1) + (size_t)32 * DV + (size_t)W * D + (size_t)W * 32) * sizeof(float);
   if (smem > 224 * 1024) return SGLC_ERR_UNSUPPORTED;

@@ -2,10 +2,11 @@
 wrong, and, in the 32-bit path, the same bits from each of them."""
 import math
 
+import numpy as np
 import pytest
 import torch
 
-from test_kernels_gpu import DEV, _ops, _rand
+from test_kernels_gpu import DEV, _attention_reference, _ops, _paged_case, _rand
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,24 @@ def test_gemm_simt_forms_give_the_same_bits(M, N, K):
     finally:
         lib.sglc_gemm_simt_set_form(0)
     assert float((first.double() - ref).abs().max()) < 1e-7 * K * math.sqrt(K) + 1e-6
+
+
+# -- 32-bit attention ------------------------------------------------------------------------------
+@pytest.mark.parametrize("H,Hkv,D,ps,window", [(2, 1, 64, 16, None), (3, 3, 128, 8, 40), (2, 2, 36, 16, 33), (1, 1, 4, 32, None)])
+def test_attention_f32_has_the_same_bits_in_every_cut(H, Hkv, D, ps, window):
+    """A token's result is the same, bit for bit, as part of a long portion, of a short one that begins inside a
+    tile, beside other requests, and as a single token: blocks of 32 tokens, tiles of 32 keys, rounds of two."""
+    ops = _ops()
+    lens = [130, 31, 64, 1, 97]
+    c = _paged_case(lens, lens, H, Hkv, D, ps, torch.float32, seed=D)
+    T, starts, scale = c["q"].shape[0], np.concatenate([[0], np.cumsum(lens)]), 1.3 / math.sqrt(D)
+    whole = torch.full((T, H * D), float("nan"), device=DEV)
+    ops.attention_simt(c["q"], c["cache"], c["bt"], c["token_req"], c["positions"], whole, H, scale, window, max(lens), max_q_len=130)
+    assert float((whole.double().cpu() - _attention_reference(c, H, Hkv, D, scale, window)).abs().max()) < 2e-5
+    some = torch.tensor(sorted({int(s + i) for s, n in zip(starts, lens) for i in (0, 1, 30, 31, 32, 63, 64, 65, 95, 96, 129) if i < n}),
+                        device=DEV)
+    for pick, longest in ((some, 1), (some, 2), (torch.arange(33, 130, device=DEV), 97), (torch.arange(T - 97, T, device=DEV), 97)):
+        out = torch.full((len(pick), H * D), float("nan"), device=DEV)
+        ops.attention_simt(c["q"][pick].contiguous(), c["cache"], c["bt"], c["token_req"][pick].contiguous(),
+                           c["positions"][pick].contiguous(), out, H, scale, window, max(lens), max_q_len=longest)
+        assert torch.equal(out, whole[pick]), longest
