@@ -60,3 +60,31 @@ def test_attention_f32_has_the_same_bits_in_every_cut(H, Hkv, D, ps, window):
         ops.attention_simt(c["q"][pick].contiguous(), c["cache"], c["bt"], c["token_req"][pick].contiguous(),
                            c["positions"][pick].contiguous(), out, H, scale, window, max(lens), max_q_len=longest)
         assert torch.equal(out, whole[pick]), longest
+
+
+# -- single tokens: items shared by clusters -------------------------------------------------------------
+@pytest.mark.parametrize("T,H,Hkv,D,window", [(9, 12, 12, 64, None), (13, 16, 4, 64, None), (18, 12, 12, 64, 200), (6, 16, 16, 128, None),
+                                              (3, 16, 2, 64, None)])
+def test_stream_decode_shares_items_between_blocks(T, H, Hkv, D, window):
+    """Contexts from one key to many tiles, so that ranks have full, short and empty runs of keys; the token's own
+    key and value fused in.  bfloat16 results of size below 1: 2^-8."""
+    ops = _ops()
+    ps = 16
+    lens = [int(n) for n in np.linspace(1, 700, T)]
+    c = _paged_case(lens, [1] * T, H, Hkv, D, ps, torch.bfloat16, seed=T)
+    scale = 0.9 / math.sqrt(D)
+    ref = _attention_reference(c, H, Hkv, D, scale, window)
+    k_new = torch.cat([K[-1:].reshape(1, Hkv * D) for K in c["Ks"]]).to(DEV)
+    v_new = torch.cat([V[-1:].reshape(1, Hkv * D) for V in c["Vs"]]).to(DEV)
+    both = torch.cat([k_new, v_new], 1).contiguous()
+    slots = torch.tensor([int(c["bt"][r, (n - 1) // ps]) * ps + (n - 1) % ps for r, n in enumerate(lens)], dtype=torch.int32, device=DEV)
+    for fused in (False, True):
+        cache = c["cache"].clone()
+        if fused:
+            for r, n in enumerate(lens):
+                cache[int(c["bt"][r, (n - 1) // ps]), :, :, (n - 1) % ps] = 0.0
+        kw = dict(k_new=both[:, :Hkv * D], v_new=both[:, Hkv * D:], slots=slots) if fused else {}
+        out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.attention_decode(c["q"], cache, c["bt"], None, c["positions"], out, H, scale, window, max(lens), variant="stream", n_tokens=T, **kw)
+        assert float((out.double().cpu() - ref).abs().max()) < 1.2e-2, fused
+        assert not fused or torch.equal(cache, c["cache"])
