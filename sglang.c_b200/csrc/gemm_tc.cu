@@ -1155,9 +1155,31 @@ int pairs_at_once() { return g_pairs_at_once; }
 // 128 x 128 partial sums, 64 KB a block, through distributed shared memory (measured at 96 and
 // 128 tokens: a decode step 15-17 % shorter; at 64 tokens and fewer the split wins or ties).
 constexpr int DIRECT_MIN_M = 65, DIRECT_MAX_KB = 32;
+// More tokens than that over a long K, with few features: the many-token kernel has few tiles, each a long walk
+// over K by one SM while the others idle.  The few-token orientation with tiles of 32 tokens deals K to a cluster as
+// long as all blocks find room at once (264 in clusters of three and more, 296 in pairs).  Measured, us before
+// and after: 768 columns over K 3,072 at 129 / 256 / 512 / 768 tokens 16.9 -> 7.1, 17.0 -> 9.1, 17.3 -> 13.8,
+// 17.4 -> 13.9; 1,024 over 4,096 at 129 / 512 tokens 21.4 -> 9.2, 21.9 -> 16.0; 1,600 over 6,400 at 129 / 256
+// tokens 32.2 -> 13.6, 32.2 -> 21.8.  Over a K of 2,048 and less the walk is short and both are even.
+// Returns the split, or 0 where the many-token kernel stays.
+static int long_k_split(int M, int N, int kb_total) {
+  if (M <= 128 || kb_total <= DIRECT_MAX_KB) return 0;
+  const long long tiles = (long long)((N + BM - 1) / BM) * ((M + 31) / 32);
+  if (tiles * 3 <= 264) return tiles * 8 <= 264 ? 8 : (int)(264 / tiles);
+  return tiles * 2 <= 296 ? 2 : 0;
+}
 static void plan(int M, int N, int K, int* swap, int* bn, int* splits, int* kb_per_split,
                  int* tiles_p, int* tiles_q) {
   int kb_total = (K + BK - 1) / BK;
+  if (const int want = long_k_split(M, N, kb_total)) {
+    *swap = 1;
+    *bn = 32;
+    *tiles_p = (N + BM - 1) / BM;
+    *tiles_q = (M + 31) / 32;
+    *kb_per_split = (kb_total + want - 1) / want;
+    *splits = (kb_total + *kb_per_split - 1) / *kb_per_split;
+    return;
+  }
   if (M <= 128 && !(M >= DIRECT_MIN_M && kb_total <= DIRECT_MAX_KB)) {
     *swap = 1;
     *tiles_p = (N + BM - 1) / BM;
