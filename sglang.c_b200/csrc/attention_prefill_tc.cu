@@ -34,10 +34,11 @@ constexpr int MMA_WARP = SOFTMAX_THREADS / 32;
 constexpr int THREADS = SOFTMAX_THREADS + 128;     // warps 0-7 softmax, warp 8 MMA + TMEM, warps 9-11 loaders
 constexpr int N_LOADERS = 96;
 constexpr int KV_STAGES = 2;
+constexpr int PIECE = 64;         // columns of a score tile a thread holds at a time
 
 
 struct Ctl {
-  uint64_t q_full, s_full, p_ready, o_full;
+  uint64_t q_full, s_full, s_free, p_ready, o_full;
   uint64_t land_free, land_full;       // the hand-over between the two blocks of a split tile
   uint64_t kv_full[KV_STAGES], kv_empty[KV_STAGES];
   uint32_t tmem_base;
@@ -59,6 +60,7 @@ struct Args {
   int window;
   int use_tma;            // keys, values and queries arrive by TMA (page_size divides 128)
   int skip_single;        // requests that bring one token are served by the decode kernel
+  int pick, R;            // pick: the launch covers only the requests that bring more (fewer than R)
   int split_min;          // key tiles from which a query tile is shared by the cluster's two blocks
   int* err;
   int kv_shared;          // pages [1][Hkv][page_size][D]: one block of rows serves as keys and as values
@@ -84,6 +86,25 @@ __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two products and sums at a time, each rounded as one alone.
+__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(reinterpret_cast<unsigned long long&>(x)), "l"(reinterpret_cast<unsigned long long&>(y)),
+      "l"(reinterpret_cast<unsigned long long&>(z)));
+  return reinterpret_cast<float2&>(r);
+}
+__device__ __forceinline__ float2 add2(float2 x, float2 y) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<unsigned long long&>(x)), "l"(reinterpret_cast<unsigned long long&>(y)));
+  return reinterpret_cast<float2&>(r);
+}
+// Four 8 x 8 matrices of 16-bit elements from the registers of the warp-level MMA's accumulator layout into
+// shared memory: lane i names the 16 bytes of row i % 8 of matrix i / 8.
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, const uint32_t (&w)[4]) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3])
+               : "memory");
 }
 
 // byte offset of 16-byte chunk `c` (0..7) of row `r` in a [rows][128 B] tile with the 128-byte swizzle
@@ -118,13 +139,27 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
   // the heaviest of them with the lightest (an idle partner would hold its place on the SM
   // until the cluster ends).  Without the split the launch lasts as long as its longest tile
   // (the last query tile of the longest request) while most SMs have long finished.
-  const int r = blockIdx.x / a.H, h = blockIdx.x % a.H, rank = blockIdx.z, cl = blockIdx.y;
+  const int h = blockIdx.x % a.H, rank = blockIdx.z, cl = blockIdx.y;
+  int r = blockIdx.x / a.H;
   pdl_launch_dependents();
   // What follows reads only the step's own arrays (request bounds, block tables), which no
   // kernel of the step writes: the block finds its work, sets up its barriers and tensor memory
   // and clears its stages while the kernel ahead still runs.  The loaders wait for that kernel
   // before they touch queries or cache pages; everything else in the block follows from what
   // they bring.
+  if (a.pick) {
+    // the r-th request of several tokens: a running server's step has many of one token and one or two of
+    // more, and blocks of this size that have nothing to do still take their turn on an SM
+    int left = r;
+    r = -1;
+    for (int r0 = 0; r0 < a.R && r < 0; r0 += 32) {
+      const int x = r0 + lane;
+      const unsigned many = __ballot_sync(0xffffffffu, x < a.R && a.q_start[x + 1] - a.q_start[x] > 1);
+      if (left < __popc(many)) r = r0 + (int)__fns(many, 0, left + 1);
+      left -= __popc(many);
+    }
+    if (r < 0) return;
+  }
   const int t0 = a.q_start[r];
   const int q_len = a.q_start[r + 1] - t0;
   if (a.skip_single && q_len == 1) return;
@@ -145,30 +180,27 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
     first_tile = fk / BKV;
     return lp / BKV - first_tile + 1;
   };
-  int n_split = 0;
-  for (int t = 0; t < nq; t++) {
+  // (a lane a query tile, 32 at a time: every warp of the block needs the answer before it can do anything)
+  auto splits = [&](int t) {
     int ft;
-    n_split += key_tiles(t, ft) >= a.split_min ? 1 : 0;
-  }
+    return t >= 0 && key_tiles(t, ft) >= a.split_min;
+  };
+  int n_split = 0;
+  for (int t0 = 0; t0 < nq; t0 += 32) n_split += __popc(__ballot_sync(0xffffffffu, splits(t0 + lane < nq ? t0 + lane : -1)));
   const bool split = cl < n_split;
   // this block's query tile: the cl-th split tile from the top, or among the others (from the
   // top) number cl - n_split for rank 0 and, from the bottom, the same number for rank 1
   int qt = -1;
   {
     const int n_rest = nq - n_split;
-    const int want = split ? cl : (rank == 0 ? cl - n_split : n_rest - 1 - (cl - n_split));
+    int want = split ? cl : (rank == 0 ? cl - n_split : n_rest - 1 - (cl - n_split));
     if (split || (cl - n_split < (n_rest + 1) / 2 && (rank == 0 || want > cl - n_split))) {
-      int seen = 0;
-      for (int t = nq - 1; t >= 0; t--) {
-        int ft;
-        const bool sp = key_tiles(t, ft) >= a.split_min;
-        if (sp == split) {
-          if (seen == want) {
-            qt = t;
-            break;
-          }
-          seen++;
-        }
+      for (int top = nq - 1; top >= 0 && qt < 0; top -= 32) {
+        const int t = top - lane;
+        const unsigned same = __ballot_sync(0xffffffffu, t >= 0 && splits(t) == split);
+        const int n = __popc(same);
+        if (want < n) qt = top - (int)__fns(same, 0, want + 1);
+        want -= n;
       }
     }
   }
@@ -191,6 +223,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
   if (threadIdx.x == 0) {
     mbar_init(&ctl.q_full, a.use_tma ? 1 : N_LOADERS);
     mbar_init(&ctl.s_full, 1);
+    mbar_init(&ctl.s_free, SOFTMAX_THREADS);
     mbar_init(&ctl.p_ready, SOFTMAX_THREADS);
     mbar_init(&ctl.o_full, 1);
     mbar_init(&ctl.land_free, SOFTMAX_THREADS);
@@ -222,31 +255,54 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
     const int lt = threadIdx.x - (MMA_WARP + 1) * 32;
     // rows of a tile that no page fills (beyond the last key, before the window) must hold
     // finite numbers: zero both stages once; later tiles leave finite data behind
-    for (int c = lt; c < (2 * KV_STAGES * TILE_BYTES) / 16; c += N_LOADERS)
-      reinterpret_cast<uint4*>(sK)[c] = make_uint4(0u, 0u, 0u, 0u);
-    fence_async_proxy();
-    asm volatile("bar.sync 2, 96;" ::: "memory");
-    if (lt == 0) {
+    const bool holes = (last_pos / a.page_size + 1) * a.page_size % BKV != 0 || first_key / a.page_size * a.page_size % BKV != 0;
+    if (holes) {
+      for (int c = lt; c < (2 * KV_STAGES * TILE_BYTES) / 16; c += N_LOADERS)
+        reinterpret_cast<uint4*>(sK)[c] = make_uint4(0u, 0u, 0u, 0u);
+      fence_async_proxy();
+      asm volatile("bar.sync 2, 96;" ::: "memory");
+    }
+    if (lt < 32) {
+      // A lane holds a page's id, asked for a tile ahead, and issues that page's copies: a thread that
+      // looks the pages of a tile up one behind the other waits for memory eight times a tile (pages of
+      // 16; 2 x 1,024 tokens of 25 heads 40.9 -> 38.5 us).
       const int ps = a.page_size;
       const int* bt = a.block_table + (size_t)r * a.bt_stride;
+      auto pages_of = [&](int j, int& pg0, int& npg) {
+        const int key0 = (kt0 + j) * BKV;
+        pg0 = key0 / ps;
+        const int pg1 = min(last_pos, key0 + BKV - 1) / ps;          // inclusive
+        if (pg0 * ps + ps - 1 < first_key) pg0 = first_key / ps;     // pages wholly before the window
+        npg = pg1 - pg0 + 1;
+      };
+      int pg0, npg;
+      pages_of(0, pg0, npg);
+      int id_next = lane < npg ? bt[pg0 + lane] : 0;
       pdl_wait();
-      mbar_expect_tx(&ctl.q_full, DB * BQ * 128);
-      for (int blk = 0; blk < DB; blk++)
-        tma_load_2d(sQ + blk * (BQ * 128), &map_q, &ctl.q_full, h * D + blk * 64, t0 + qt * BQ);
+      if (lane == 0) {
+        mbar_expect_tx(&ctl.q_full, DB * BQ * 128);
+        for (int blk = 0; blk < DB; blk++)
+          tma_load_2d(sQ + blk * (BQ * 128), &map_q, &ctl.q_full, h * D + blk * 64, t0 + qt * BQ);
+      }
       bool ok = true;
       for (int j = 0; j < n_tiles && ok; j++) {
         const int s = j % KV_STAGES;
-        if (j >= KV_STAGES) ok = mbar_wait(&ctl.kv_empty[s], ((j / KV_STAGES) - 1) & 1, abort_flag);
-        if (!ok) break;
-        const int key0 = (kt0 + j) * BKV;
-        int pg0 = key0 / ps;
-        int pg1 = min(last_pos, key0 + BKV - 1) / ps;          // inclusive
-        if (pg0 * ps + ps - 1 < first_key) pg0 = first_key / ps;   // pages wholly before the window
-        const int npg = pg1 - pg0 + 1;
-        mbar_expect_tx(&ctl.kv_full[s], (uint32_t)npg * 2u * DB * (uint32_t)ps * 128u);
-        for (int pi = pg0; pi <= pg1; pi++) {
-          const int page = bt[pi];
-          const uint32_t row_off = (uint32_t)(pi * ps - key0) * 128u;
+        const int first = pg0, n = npg, id = id_next;
+        if (j + 1 < n_tiles) {
+          pages_of(j + 1, pg0, npg);
+          id_next = lane < npg ? bt[pg0 + lane] : 0;
+        }
+        if (j >= KV_STAGES) {
+          int w = 1;
+          if (lane == 0) w = mbar_wait(&ctl.kv_empty[s], ((j / KV_STAGES) - 1) & 1, abort_flag) ? 1 : 0;
+          ok = __shfl_sync(0xffffffffu, w, 0) != 0;
+          if (!ok) break;
+        }
+        if (lane == 0) mbar_expect_tx(&ctl.kv_full[s], (uint32_t)n * 2u * DB * (uint32_t)ps * 128u);
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) {
+          const int page = i < 32 ? id : bt[first + i];
+          const uint32_t row_off = (uint32_t)((first + i) * ps - (kt0 + j) * BKV) * 128u;
           for (int blk = 0; blk < DB; blk++) {
             tma_load_5d(sK + s * TILE_BYTES + blk * (BKV * 128) + row_off, &map_kv, &ctl.kv_full[s],
                         blk * 64, 0, hk, 0, page);
@@ -346,24 +402,25 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
       }
       for (int j = 0; j < n_tiles && ok; j++) {
         const int s = j % KV_STAGES;
-        ok = mbar_wait(&ctl.p_ready, j & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after_sync();
-        // the next tile's scores go ahead of this tile's P.V: the softmax warps find them when
-        // they come back from sending P, and this P.V runs under their first pass
+        // the next tile's scores as soon as the softmax warps hold this tile's in registers: they run under
+        // the exponentials
         if (j + 1 < n_tiles) {
-          ok = mbar_wait(&ctl.kv_full[(j + 1) % KV_STAGES], ((j + 1) / KV_STAGES) & 1, abort_flag);
+          ok = mbar_wait(&ctl.kv_full[(j + 1) % KV_STAGES], ((j + 1) / KV_STAGES) & 1, abort_flag) &&
+               mbar_wait(&ctl.s_free, j & 1, abort_flag);
           if (!ok) break;
           tc_fence_after_sync();
           issue_s((j + 1) % KV_STAGES);
         }
+        ok = mbar_wait(&ctl.p_ready, j & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after_sync();
         const uint32_t p0 = smem_u32(sP), v0 = smem_u32(sV + s * TILE_BYTES);
 #pragma unroll
         for (int k = 0; k < BKV / 16; k++) {
           uint64_t dp = smem_desc_k_sw128(p0 + (k / 4) * (BQ * 128) + (k % 4) * 32);
           // V: 16 keys = 16 rows of 128 bytes further; blocks of 64 head elements BKV*128 bytes apart
           uint64_t dv = smem_desc_mn_sw128(v0 + k * 2048, BKV * 128, 1024);
-          mma_bf16(tO, dp, dv, idesc_o, k > 0 ? 1u : 0u);
+          mma_bf16(tO, dp, dv, idesc_o, (j > 0 || k > 0) ? 1u : 0u);      // (sums over the tiles)
         }
         mma_commit(&ctl.o_full);
         mma_commit(&ctl.kv_empty[s]);
@@ -389,23 +446,11 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
     const uint32_t tO = tS + 128;
     const int st = threadIdx.x;                                 // 0..SOFTMAX_THREADS-1
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};   // l: this thread's share of the row sums
-    // output: for every 32 columns 16 registers in the order they are loaded in (index & 2: row g + 8)
-    float o[D / 2];
+    // where this lane's matrix rows of the weights go: rows lane0 + lane % 8 (+ 8), chunk lane / 8 of the first (second)
+    // four chunks of a 64-key block
+    uint32_t p_addr[2];
 #pragma unroll
-    for (int d = 0; d < D / 2; d++) o[d] = 0.0f;
-    float alpha[2] = {0.0f, 0.0f};     // of the last tile seen: what its maximum made of the sums before it
-    // o = o * alpha + (the tile's P.V, from tensor memory)
-    auto fold = [&](const float (&al)[2]) {
-#pragma unroll
-      for (int c = 0; c < D; c += 32) {
-        uint32_t v[16];
-        tmem_ld_16x256b_x4(tO + c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 16; i++) o[c / 2 + i] = o[c / 2 + i] * al[(i >> 1) & 1] + __uint_as_float(v[i]);
-      }
-      tc_fence_before_sync();
-    };
+    for (int c = 0; c < 2; c++) p_addr[c] = smem_u32(sP) + sw128(lane0 + (lane & 7), 4 * c + (lane >> 3));
     bool ok = true;
     for (int j = 0; j < n_tiles && ok; j++) {
       ok = mbar_wait(&ctl.s_full, j & 1, abort_flag);
@@ -429,80 +474,122 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
         rel0[x] = any ? key0 + 2 * q4 - first : -(1 << 20);
         vis_span[x] = any ? (uint32_t)(last - first) : 0u;
       }
+      // the scores of PIECE columns (for every 32 of them 16 registers in the order they are loaded in, index & 2:
+      // row g + 8); a register per score for the whole tile would not leave room for two blocks on an SM
+      uint32_t v[PIECE / 32][16];
+      auto take = [&](int c0) {
+#pragma unroll
+        for (int c = 0; c < PIECE / 32; c++) tmem_ld_16x256b_x4(tS + c0 + 32 * c, v[c]);
+        tmem_ld_wait();
+        if (!full_tile) {
+#pragma unroll
+          for (int c = 0; c < PIECE / 32; c++)
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+              const int x = (i >> 1) & 1;
+              if ((uint32_t)(rel0[x] + c0 + 32 * c + 8 * (i >> 2) + (i & 1)) > vis_span[x]) v[c][i] = 0xff800000u;      // -inf
+            }
+        }
+      };
       // pass 1: the rows' maxima over the keys they may see
       float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll 1
-      for (int c = 0; c < BKV; c += 32) {
-        uint32_t v[16];
-        tmem_ld_16x256b_x4(tS + c, v);
-        tmem_ld_wait();
-        if (full_tile) {
+      for (int c0 = 0; c0 < BKV; c0 += PIECE) {
+        take(c0);
 #pragma unroll
-          for (int i = 0; i < 16; i++) mx[(i >> 1) & 1] = fmaxf(mx[(i >> 1) & 1], __uint_as_float(v[i]));
-        } else {
+        for (int c = 0; c < PIECE / 32; c++)
 #pragma unroll
-          for (int i = 0; i < 16; i++) {
-            const int x = (i >> 1) & 1;
-            const bool vis = (uint32_t)(rel0[x] + c + 8 * (i >> 2) + (i & 1)) <= vis_span[x];
-            mx[x] = fmaxf(mx[x], vis ? __uint_as_float(v[i]) : -INFINITY);
-          }
-        }
+          for (int i = 0; i < 16; i++) mx[(i >> 1) & 1] = fmaxf(mx[(i >> 1) & 1], __uint_as_float(v[c][i]));
       }
-      if (j > 0) {
-        // the tile before: its P.V ran under this pass; fold it in (its P may then be overwritten)
-        ok = mbar_wait(&ctl.o_full, (j - 1) & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after_sync();
-        fold(alpha);
-      }
-      float neg_m[2];
+      // The exponentials are taken against a reference m that follows the running maximum: it moves only when
+      // the maximum has grown by more than 2^8, and only then are the sums so far (in tensor memory and
+      // in l) scaled down.  Any reference gives the same quotient; weights of up to 2^8 lose no digits.
+      float alpha[2] = {1.0f, 1.0f};
+      bool moved = false;
 #pragma unroll
       for (int x = 0; x < 2; x++) {
         mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 1));
         mx[x] = fmaxf(mx[x], __shfl_xor_sync(0xffffffffu, mx[x], 2));
-        const float m_new = fmaxf(m[x], mx[x]);
-        const float m_use = m_new == -INFINITY ? 0.0f : m_new;     // a row with no key yet
-        alpha[x] = exp2f((m[x] - m_use) * a.scale_log2);           // m = -inf gives 0
-        neg_m[x] = -m_use * a.scale_log2;
-        m[x] = m_new;
-      }
-      // pass 2: p = exp(s - max) = 2^(s*c - max*c) as bfloat16 into shared memory, and the row sums
-      float sum[2] = {0.0f, 0.0f};
-#pragma unroll 1
-      for (int c = 0; c < BKV; c += 32) {
-        uint32_t v[16];
-        tmem_ld_16x256b_x4(tS + c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-#pragma unroll
-          for (int x = 0; x < 2; x++) {
-            float p0 = ex2_approx(fmaf(__uint_as_float(v[4 * b + 2 * x]), a.scale_log2, neg_m[x]));
-            float p1 = ex2_approx(fmaf(__uint_as_float(v[4 * b + 2 * x + 1]), a.scale_log2, neg_m[x]));
-            if (!full_tile) {
-              const uint32_t rel = (uint32_t)(rel0[x] + c + 8 * b);
-              if (rel > vis_span[x]) p0 = 0.0f;
-              if (rel + 1u > vis_span[x]) p1 = 0.0f;
-            }
-            sum[x] += p0 + p1;
-            __nv_bfloat162 hh = __floats2bfloat162_rn(p0, p1);
-            // keys c + 8b .. +7 are one 16-byte chunk of the row; this thread's pair is its q4-th word
-            *reinterpret_cast<uint32_t*>(sP + (c / 64) * (BQ * 128) + sw128(row_r[x], (c % 64) / 8 + b) + 4 * q4) =
-                *reinterpret_cast<uint32_t*>(&hh);
-          }
+        if (m[x] == -INFINITY) {
+          m[x] = mx[x];                                // (a row's first keys: its sums are zero)
+        } else if ((mx[x] - m[x]) * a.scale_log2 > 8.0f) {
+          alpha[x] = exp2f((m[x] - mx[x]) * a.scale_log2);
+          l[x] *= alpha[x];
+          m[x] = mx[x];
+          moved = true;
         }
       }
+      if (j > 0) {
+        // the tile before: its P.V is done, so its P may be overwritten and the sums may be scaled
+        ok = mbar_wait(&ctl.o_full, (j - 1) & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-      for (int x = 0; x < 2; x++) l[x] = l[x] * alpha[x] + sum[x];
-      tc_fence_before_sync();       // the loads of S are done before the next S may be written
+          for (int c = 0; c < D; c += 16) {
+            uint32_t t[8];
+            tmem_ld_16x256b_x2(tO + c, t);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 8; i++) t[i] = __float_as_uint(__uint_as_float(t[i]) * alpha[(i >> 1) & 1]);
+            tmem_st_16x256b_x2(tO + c, t);
+          }
+          tmem_st_wait();
+        }
+      }
+      float neg_m[2];
+#pragma unroll
+      for (int x = 0; x < 2; x++) neg_m[x] = m[x] == -INFINITY ? 0.0f : -m[x] * a.scale_log2;      // (a row with no key yet)
+      // pass 2: p = exp(s - m) = 2^(s*c - m*c) as bfloat16 into shared memory, and the row sums
+      float2 sum[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};      // (of a row's even keys and of its odd ones)
+#pragma unroll 1
+      for (int c0 = 0; c0 < BKV; c0 += PIECE) {
+        take(c0);
+        if (c0 + PIECE == BKV) {                         // (the next tile's scores may come)
+          tc_fence_before_sync();
+          mbar_arrive(&ctl.s_free);
+        }
+#pragma unroll
+        for (int x = 0; x < 2; x++)
+#pragma unroll
+          for (int c = 0; c < PIECE / 32; c++) {
+            uint32_t w[4];                               // 32 keys of row x: four 8 x 8 matrices of weights
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+              const float2 e = fma2(make_float2(__uint_as_float(v[c][4 * b + 2 * x]), __uint_as_float(v[c][4 * b + 2 * x + 1])),
+                                    make_float2(a.scale_log2, a.scale_log2), make_float2(neg_m[x], neg_m[x]));
+              const float2 pp = make_float2(ex2_approx(e.x), ex2_approx(e.y));
+              sum[x] = add2(sum[x], pp);
+              const __nv_bfloat162 hh = __floats2bfloat162_rn(pp.x, pp.y);
+              w[b] = *reinterpret_cast<const uint32_t*>(&hh);
+            }
+            // keys c0 + 32c + 8b .. +7 are one 16-byte chunk of a row; this lane names the row lane % 8 of matrix lane / 8
+            stmatrix_x4(p_addr[c & 1] + (uint32_t)((c0 + 32 * c) / 64) * (BQ * 128) + x * 8 * 128, w);
+          }
+      }
+      l[0] += sum[0].x + sum[0].y;
+      l[1] += sum[1].x + sum[1].y;
       fence_async_proxy();          // P is visible to the tensor core
+      tc_fence_before_sync();
       mbar_arrive(&ctl.p_ready);
     }
+    // output: for every 32 columns 16 registers in the order they are loaded in (index & 2: row g + 8)
+    float o[D / 2];
+#pragma unroll
+    for (int d = 0; d < D / 2; d++) o[d] = 0.0f;
     if (ok && n_tiles > 0) {
       ok = mbar_wait(&ctl.o_full, (n_tiles - 1) & 1, abort_flag);
       if (ok) {
         tc_fence_after_sync();
-        fold(alpha);
+#pragma unroll
+        for (int c = 0; c < D; c += 32) {
+          uint32_t t[16];
+          tmem_ld_16x256b_x4(tO + c, t);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 16; i++) o[c / 2 + i] = __uint_as_float(t[i]);
+        }
+        tc_fence_before_sync();
       }
     }
     // A shared tile is finished by both blocks, each for half of the head's columns: a block
@@ -680,15 +767,24 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const Args& a, int R, 
                          cudaSharedmemCarveoutMaxShared);
     configured = true;
   }
-  dim3 grid(a.H * R, (max_q_len + BQ - 1) / BQ, 2);      // two blocks (one cluster) per query tile
+  dim3 grid(a.H * (a.pick ? R - a.skip_single : R), (max_q_len + BQ - 1) / BQ, 2);      // two blocks (one cluster) per query tile
   return sglc_launch(attention_prefill_kernel<D, EXT>, grid, dim3(THREADS), smem, stream, 2, true, mq, mkv, a);
 }
 }  // namespace
 
 
-// Tuning hook: key tiles from which a query tile is split over two blocks (default 5).
-static int g_split_min = 5;
-SGLC_API void sglc_attention_prefill_set_split_min(int n) { g_split_min = n < 2 ? 2 : n; }
+// Tuning hook: key tiles from which a query tile is split over two blocks (0: the rule decides).
+static int g_split_min = 0;
+SGLC_API void sglc_attention_prefill_set_split_min(int n) { g_split_min = n <= 0 ? 0 : n < 2 ? 2 : n; }
+// A split tile ends sooner but costs a second start and the exchange: the fewer query tiles there are for the 296
+// blocks that run at once, the smaller the tiles worth splitting, and none are where all blocks have more than one.
+// (us at head size 64, splits from 2 / 4 / 5 / no splits: 48 tiles of up to 4 key tiles 11.4 / 11.7 / 13.2 / 13.2,
+// 96 such 12.4 / 11.7 / 13.3 / 13.2, 192 of up to 8 23.7 / 23.8 / 17.4 / 21.5, 400 38.9 / 38.3 / 39.3 / 36.7, 1,600
+// 142.6 / 134.4 / 125.9 / 113.8.)
+static int split_from(long long query_tiles) {
+  if (g_split_min) return g_split_min;
+  return query_tiles <= 74 ? 2 : query_tiles <= 148 ? 4 : query_tiles <= 296 ? 5 : 1 << 30;
+}
 
 // Head sizes this kernel takes.
 SGLC_API int sglc_attention_prefill_tc_supports(int D) { return D == 64 || D == 128; }
@@ -696,7 +792,8 @@ SGLC_API int sglc_attention_prefill_tc_supports(int D) { return D == 64 || D == 
 // q, out: bfloat16 [T][stride], heads side by side, tokens of request r at q_start[r]..q_start[r+1];
 // cache: one layer's pages [n_pages][2][Hkv][page_size][D]; kv_len[r]: the request's length after
 // this step (its last query sits at kv_len-1); max_q_len: the longest portion (sizes the grid).
-// T: rows of q; n_pages: pages of the cache tensor.
+// T: rows of q; n_pages: pages of the cache tensor.  skip_single: 0, or requests of one token are left out; their number
+// where it is known (1 also where it is not): the launch then covers the others only.
 static int attention_prefill_run(const void* q, int q_stride, const void* cache,
                                  const int* block_table, int bt_stride, const int* q_start,
                                  const int* kv_len, void* out, int o_stride, int R,
@@ -723,7 +820,9 @@ static int attention_prefill_run(const void* q, int q_stride, const void* cache,
   a.window = window;
   a.err = err;
   a.skip_single = skip_single;
-  a.split_min = g_split_min;
+  a.R = R;
+  a.pick = skip_single > 1 && skip_single < R ? 1 : 0;
+  a.split_min = split_from((long long)H * ((T + BQ - 1) / BQ));
   a.kv_shared = kv_shared;
   a.chunk = chunk;
   a.sinks = sinks;

@@ -666,7 +666,7 @@ def attention_prefill_tc(q, cache, block_table, q_start, kv_len, out, n_heads, s
             _ptr(q), q.stride(0), _ptr(cache), _ptr(block_table), block_table.stride(0), _ptr(q_start), _ptr(kv_len),
             _ptr(out), out.stride(0), int(n_requests), int(max_q_len), n_heads, Hkv, D, page_size,
             ctypes.c_float(scale), int(window or 0), int(chunk or 0), _ptr(sinks), q.shape[0], n_pages,
-            1 if skip_single else 0, _ptr(err), 1 if kv_shared else 0, gp, gs, per_head, _stream())
+            int(skip_single), _ptr(err), 1 if kv_shared else 0, gp, gs, per_head, _stream())
         _check(lib, code, f"attention_prefill_tc (head_dim {D}, chunk {chunk})")
         return
     fn = lib.sglc_attention_prefill_tc_shared if kv_shared else lib.sglc_attention_prefill_tc
@@ -674,7 +674,7 @@ def attention_prefill_tc(q, cache, block_table, q_start, kv_len, out, n_heads, s
               block_table.stride(0), _ptr(q_start), _ptr(kv_len), _ptr(out),
               out.stride(0), int(n_requests), int(max_q_len), n_heads, Hkv, D,
               page_size, ctypes.c_float(scale), int(window or 0), q.shape[0],
-              n_pages, 1 if skip_single else 0, _ptr(err), _stream())
+              n_pages, int(skip_single), _ptr(err), _stream())
     _check(lib, code, f"attention_prefill_tc (head_dim {D})")
 
 

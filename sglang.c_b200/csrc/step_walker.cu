@@ -228,7 +228,7 @@ struct Walk {
     if (bf16_ok && (D == 64 || D == 128) && L.scale > 0 && o_stride % 8 == 0 && ((uintptr_t)o & 15) == 0) {
       const bool split = s.n_decode > 0;
       if (!check(g.attention_prefill_tc(q, stride, c.cache, bt, s.bt_stride, s.q_start, s.kv_len, o, o_stride, s.R,
-                                        s.max_q_len, H, Hkv, D, ps, L.scale, L.window, s.T, c.n_pages, split ? 1 : 0,
+                                        s.max_q_len, H, Hkv, D, ps, L.scale, L.window, s.T, c.n_pages, s.n_decode,
                                         s.tc_err, s.stream),
                  "attention_prefill_tc"))
         return;

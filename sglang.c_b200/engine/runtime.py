@@ -93,7 +93,7 @@ class Runtime:
             # them go to the split-key kernel (a tile of one query would waste the other 127 rows)
             split = ctx.n_decode > 0
             ops.attention_prefill_tc(q, cache, grp.block_table, ctx.q_start, ctx.kv_len, out, n_heads,
-                                     scale, window, ctx.R, ctx.max_q_len, skip_single=split)
+                                     scale, window, ctx.R, ctx.max_q_len, skip_single=ctx.n_decode)
             if split:
                 ops.attention_decode(q, cache, grp.block_table, ctx.token_req, ctx.positions, out, n_heads,
                                      scale, window, ctx.max_keys, token_list=ctx.decode_tokens,
@@ -125,7 +125,7 @@ class Runtime:
                 and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
             split = ctx.n_decode > 0
             ops.attention_prefill_tc(q, cache, grp.block_table, ctx.q_start, ctx.kv_len, out, n_heads, scale, window,
-                                     ctx.R, ctx.max_q_len, skip_single=split, kv_shared=True, **more)
+                                     ctx.R, ctx.max_q_len, skip_single=ctx.n_decode, kv_shared=True, **more)
             if split:
                 single(q, cache, grp.block_table, ctx.token_req, ctx.positions, out, n_heads, scale, window,
                        ctx.max_keys, token_list=ctx.decode_tokens, n_tokens=ctx.n_decode, **more)

@@ -62,6 +62,33 @@ def test_attention_f32_has_the_same_bits_in_every_cut(H, Hkv, D, ps, window):
         assert torch.equal(out, whole[pick]), longest
 
 
+# -- tensor-core prompt attention ---------------------------------------------------------------------
+@pytest.mark.parametrize("D,window,grow", [(64, None, 3.0), (64, 150, 3.0), (128, None, 3.0), (64, None, 0.0), (64, None, -3.0)])
+def test_prompt_attention_follows_a_growing_maximum(D, window, grow):
+    """Scores whose maximum grows (or shrinks) by far more than 2^8 from key tile to key tile, so that the sums in
+    tensor memory are scaled down again and again; ragged prompts, one behind a cached context.  bfloat16
+    weights and results: 2^-8 of values of size about 3."""
+    ops = _ops()
+    H, Hkv, ps = 2, 1, 16
+    lens, q_lens = [600, 129, 40], [470, 129, 40]
+    c = _paged_case(lens, q_lens, H, Hkv, D, ps, torch.bfloat16, seed=D)
+    one = torch.zeros(D)
+    one[0] = 1.0
+    for r, n in enumerate(lens):                      # the first entry of key p: grow * p / 16; of every query: 8
+        c["Ks"][r][:, :, 0] = (grow * torch.arange(n)[:, None] / 16.0).to(torch.bfloat16)
+        c["Qs"][r][:, :, 0] = 8.0
+        for p in range(n):
+            c["cache"][int(c["bt"][r, p // ps]), 0, :, p % ps] = c["Ks"][r][p].to(DEV)
+    q = torch.cat([x.reshape(x.shape[0], H * D) for x in c["Qs"]]).to(DEV)
+    T, scale = q.shape[0], 0.25
+    q_start = torch.tensor(np.concatenate([[0], np.cumsum(q_lens)]), dtype=torch.int32, device=DEV)
+    kv_len = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.attention_prefill_tc(q, c["cache"], c["bt"], q_start, kv_len, out, H, scale, window, len(lens), max(q_lens))
+    ref = _attention_reference(c, H, Hkv, D, scale, window)
+    assert float((out.double().cpu() - ref).abs().max()) < 2.5e-2
+
+
 # -- single tokens: items shared by clusters -------------------------------------------------------------
 @pytest.mark.parametrize("T,H,Hkv,D,window", [(9, 12, 12, 64, None), (13, 16, 4, 64, None), (18, 12, 12, 64, 200), (6, 16, 16, 128, None),
                                               (3, 16, 2, 64, None)])
