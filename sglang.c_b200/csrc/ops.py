@@ -1122,6 +1122,71 @@ def state_chunks(q, k, v, weights, A_log, out, state, q_start, state_slots, n_re
     _check(lib, code, f"state_chunks ({dim} x {v_dim})", n_kernels=3)
 
 
+DELTA_CHUNKS_MAX_DIM = 64        # key sizes of the chunks of the delta rule and the fixed decay (state_chunks.cu)
+
+
+def delta_chunks_pay(mode, n_tokens, n_requests, max_q_len, n_heads, dim):
+    """Whether a step's delta rule (or recurrence of fixed decay) is worked on in chunks.  A walk takes the time of
+    its longest portion, chunks that of all of them on the whole chip.  Measured, heads of 64, walk against chunks:
+    delta rule, 12 heads, 1 x 128 tokens 30 and 36 us, 8 x 128 51 and 53, 12 x 160 70 and 78, 2 x 192 46 and 39,
+    1 x 256 56 and 37, 2 x 1,024 232 and 80; fixed decay, 3 heads, 1 x 64 tokens 14 and 19, 8 x 100 22 and 20,
+    1 x 128 25 and 19, 2 x 1,024 174 and 21."""
+    if dim > DELTA_CHUNKS_MAX_DIM or n_requests > n_tokens // STATE_CHUNK:
+        return False
+    work = (n_tokens // STATE_CHUNK + n_requests // 2) * n_heads         # about the (chunk, head) pairs
+    return max_q_len >= (150 + work // 2 if mode == "delta" else 96 + work // 6)
+
+
+def delta_chunks_workspace(mode, n_tokens, n_requests, n_heads, v_dim):
+    """Floats of workspace that delta_chunks takes for such a step."""
+    tiles = (v_dim + 63) // 64
+    units = 3 + 2 * tiles if mode == "delta" else 1 + tiles
+    return (n_tokens // STATE_CHUNK + n_requests) * n_heads * (units * STATE_CHUNK ** 2 + 1)
+
+
+def delta_chunks(mode, q, k, v, out, state, q_start, state_slots, n_requests, n_heads, n_qk_heads, dim, v_dim, workspace,
+                 gates=None, head_decay=None, silu_in=False):
+    """matrix_state's modes "delta" and "decay" in chunks that run side by side (state_chunks.cu), for portions
+    of many tokens and key sizes up to 64; the arguments are matrix_state's; workspace: float32,
+    delta_chunks_workspace entries."""
+    _need_cuda(q, k, v, out, state, q_start, state_slots, gates, head_decay, workspace)
+    T = out.shape[0]
+    _f32_rows(q, "delta_chunks: q", n_qk_heads * dim)
+    _f32_rows(k, "delta_chunks: k", n_qk_heads * dim)
+    _f32_rows(v, "delta_chunks: v", n_heads * v_dim)
+    _f32_rows(out, "delta_chunks: out", n_heads * v_dim)
+    if mode not in ("delta", "decay"):
+        raise KernelError(f"delta_chunks: no mode '{mode}'")
+    if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (n_heads, dim, v_dim):
+        raise KernelError(f"delta_chunks: the state is float32 [n_slots, {n_heads}, {dim}, {v_dim}]")
+    if min(t.shape[0] for t in (q, k, v)) < T:
+        raise KernelError("delta_chunks: a row of q, k and v for every token")
+    if mode == "delta":
+        if gates is None or head_decay is not None:
+            raise KernelError("delta_chunks: the delta rule takes its gates")
+        _f32_rows(gates, "delta_chunks: gates", 2 * n_heads)
+        if gates.shape[0] < T:
+            raise KernelError("delta_chunks: gates for every token")
+    elif gates is not None or head_decay is None or head_decay.dtype != torch.float32 or head_decay.numel() != n_heads \
+            or not head_decay.is_contiguous():
+        raise KernelError("delta_chunks: the decay form takes one float32 decay per head")
+    _i32(q_start, "q_start")
+    _i32(state_slots, "state_slots")
+    R = int(n_requests)
+    if workspace.dtype != torch.float32 or not workspace.is_contiguous() \
+            or workspace.numel() < delta_chunks_workspace(mode, T, R, n_heads, v_dim):
+        raise KernelError("delta_chunks: the workspace is too small")
+    lib = build.load("state_chunks")
+    code = lib.sglc_delta_chunks(_ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(k), ctypes.c_longlong(k.stride(0)), _ptr(v),
+                                 ctypes.c_longlong(v.stride(0)), _ptr(gates),
+                                 ctypes.c_longlong(gates.stride(0) if gates is not None else 0), _ptr(head_decay), _ptr(out),
+                                 ctypes.c_longlong(out.stride(0)), _ptr(state), state.shape[0], _ptr(q_start),
+                                 _ptr(state_slots), R, int(n_heads), int(n_qk_heads), int(dim), int(v_dim),
+                                 1 if silu_in else 0, _ptr(workspace), T // STATE_CHUNK + R, _ptr(tc_error_flag(q.device)),
+                                 _stream())
+    _check(lib, code, f"delta_chunks ({mode}, {dim} x {v_dim})", n_kernels=3)
+
+
 def state_step(q, k, v, gates, out, state, state_slots, n_heads, n_groups, dim, v_dim, skip=None):
     """matrix_state's gated form (with its skip) for a step in which every request brings one token: row r
     is request r's.  gates: float32 [R, 2H] (input weights, decays)."""

@@ -409,6 +409,501 @@ SGLC_API int sglc_state_chunks(const float* q, long long q_stride, const float* 
   return sglc_launch(chunk_read_kernel, dim3(n_chunks, H, col_tiles), dim3(SC_THREADS), smem3, stream, 1, true, p);
 }
 
+// ---- the gated delta rule, and the recurrence of fixed decay, in chunks -------------------------------------------
+// With r_ij = g_(j+1) .. g_i (products taken token by token: a decay of zero stays one), c_i = g_1 .. g_i, S_in the
+// state ahead of a chunk and C its last token:
+//   delta rule   u_i = b_i (v_i - (g_i S_(i-1))^T k_i), that is  (I + L) U = diag(b) V - diag(b c) K S_in,
+//                L_ij = b_i r_ij (k_i . k_j) for j < i;  so  U = U0 - W S_in  with  (I + L) [W | U0] = diag(b) [diag(c) K | V]
+//   decay form   u_i = v_i
+//   o_i   = c_i S_in^T q_i + sum_{j <= i} r_ij (q_i . k_j) u_j
+//   S_out = c_C S_in + sum_j r_Cj k_j u_j^T = A S_in + B,  A = c_C I - sum_j r_Cj k_j w_j^T,  B = sum_j r_Cj k_j u0_j^T
+// in three launches: a chunk's products, its triangular system (forward substitution, a column a thread, in
+// registers), A and B; a pass over the chunks of each request, S <- A S + B, eight columns a block; the read-outs.
+// All 32-bit multiply-adds, in the order of the tokens where one depends on another.  The walk token by token
+// (matrix_state.cu) is a chain of T dependent steps of 215 ns with most of the GPU idle; this does about twice
+// the multiply-adds with every SM at work.  2 x 1,024 tokens: delta rule, 12 heads of 64, 232 -> 80 us (38, 24 and 21:
+// the first bound by shared memory reads and the chain of the triangular system, the second a chain of 16 chunks, 1.4
+// us each); fixed decay, 3 heads, 174 -> 21.  Key sizes up to 64 (three blocks' tiles then fit into an SM's shared
+// memory); value columns in tiles of 64.
+constexpr int DC_LD = 64 + SC_PAD, DC_TILE = 64 * DC_LD;
+constexpr int DC_PASS_COLS = 8, DC_PASS_RING = 4;
+constexpr int DC_TERM_THREADS = 128;      // (three blocks an SM: 34 chunks of 12 heads then take one round)
+
+struct DcArgs {
+  const float* q; long long q_stride;       // [T][..], group g at columns g*D
+  const float* k; long long k_stride;
+  const float* v; long long v_stride;       // head h at columns h*V
+  const float* gates; long long gates_stride;   // delta rule: [T][2H]: b, then the decays
+  const float* head_decay;                  // decay form: [H]
+  float* out; long long out_stride;         // [T][H*V]
+  float* state;                             // [n_slots][H][D][V]
+  float* qk;                                // [n_chunks][H][64][64]: r_ij (q_i . k_j), zero above the diagonal
+  float* W;                                 // [n_chunks][H][64][64]
+  float* A;                                 // [n_chunks][H][64][64]
+  float* U;                                 // [n_chunks][H][tiles][64][64]: U0
+  float* S;                                 // [n_chunks][H][tiles][64][64]: B, then the states ahead of the chunks
+  float* total;                             // [n_chunks][H]: c_C
+  const int* q_start; const int* state_slots;
+  int R, H, G, D, V, tiles, n_slots, n_chunks;
+  int vec, silu_in;
+  int* err;
+};
+
+__device__ __forceinline__ float dc_silu(float v) { return v / (1.0f + expf(-v)); }
+
+// 64 rows of src, columns c0 .. c0 + 63 of rows that end at column n, into dst; zeros outside.
+template <int NT>      // NT: the block's threads
+__device__ __forceinline__ void dc_stage(const float* src, long long stride, int len, int c0, int n, bool vec, float* dst) {
+  if (vec) {
+    for (int x = threadIdx.x; x < 64 * 16; x += NT) {
+      const int i = x >> 4, c = (x & 15) * 4;
+      const bool on = i < len && c0 + c < n;
+      copy16(dst + i * DC_LD + c, on ? src + (size_t)i * stride + c0 + c : src, on);
+    }
+  } else {
+    for (int x = threadIdx.x; x < 64 * 64; x += NT) {
+      const int i = x >> 6, c = x & 63;
+      dst[i * DC_LD + c] = (i < len && c0 + c < n) ? src[(size_t)i * stride + c0 + c] : 0.0f;
+    }
+  }
+}
+__device__ __forceinline__ void dc_stage64(const float* src, float* dst) {        // a whole tile of the workspace
+  for (int x = threadIdx.x; x < 64 * 16; x += blockDim.x) copy16(dst + (x >> 4) * DC_LD + (x & 15) * 4, src + x * 4, true);
+}
+template <int NT>
+__device__ __forceinline__ void dc_silu_tile(float* t) {
+  for (int x = threadIdx.x; x < 64 * 64; x += NT) t[(x >> 6) * DC_LD + (x & 63)] = dc_silu(t[(x >> 6) * DC_LD + (x & 63)]);
+}
+// A sum of short sums rounds less than one long one, as the walk's partial sums do: 64 entries go eight at a time, in
+// pairs; and what a sum is added to, it is added to once.  (Against 64 bits, six draws of gates, keys and
+// values as a layer makes them, 256 to 2,048 tokens: 1.60e-7, the walk 1.62e-7; sums of sixteen that start from their
+// addend 1.85e-7.)
+// acc[half][i][j] += a row (32 half + ty*4 + i) . b row (tx + 16 j), by 128 threads
+__device__ __forceinline__ void dc_rows_product(float (&acc)[2][4][4], const float* a, const float* b, int ty, int tx) {
+#pragma unroll 1
+  for (int e0 = 0; e0 < 64; e0 += 16) {
+    float sum[2][2][4][4] = {};
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+#pragma unroll
+      for (int e = e0 + 8 * n; e < e0 + 8 * n + 8; e += 4) {
+        float4 y[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) y[j] = ld4(b + (tx + 16 * j) * DC_LD + e);
+#pragma unroll
+        for (int f = 0; f < 2; f++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const float4 x = ld4(a + (32 * f + ty * 4 + i) * DC_LD + e);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              float& s = sum[n][f][i][j];
+              s = fmaf(x.x, y[j].x, s); s = fmaf(x.y, y[j].y, s); s = fmaf(x.z, y[j].z, s); s = fmaf(x.w, y[j].w, s);
+            }
+          }
+      }
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[f][i][j] += sum[0][f][i][j] + sum[1][f][i][j];
+  }
+}
+// acc[half][i][j] += sum over rows e of a(e, 32 half + ty*4 + i) b(e, tx*4 + j), by 128 threads
+__device__ __forceinline__ void dc_columns_product(float (&acc)[2][4][4], const float* a, const float* b, int ty, int tx) {
+#pragma unroll 1
+  for (int e0 = 0; e0 < 64; e0 += 16) {
+    float sum[2][4][4] = {};
+#pragma unroll 8
+    for (int e = e0; e < e0 + 16; e++) {
+      const float4 y = ld4(b + e * DC_LD + tx * 4);
+      fma16(sum[0], ld4(a + e * DC_LD + ty * 4), y);
+      fma16(sum[1], ld4(a + e * DC_LD + 32 + ty * 4), y);
+    }
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[f][i][j] += sum[f][i][j];
+  }
+}
+// acc += a rows ty*4 .. +3 (n entries of each, a multiple of 8) times b's rows, columns tx*4 .. +3, by 256 threads
+__device__ __forceinline__ void dc_product(float (&acc)[4][4], const float* a, const float* b, int n, int ty, int tx) {
+#pragma unroll 1
+  for (int e0 = 0; e0 < n; e0 += 8) {
+    float sum[4][4] = {};
+#pragma unroll
+    for (int e = e0; e < e0 + 8; e += 4) {
+      float4 x[4], y[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) x[i] = ld4(a + (ty * 4 + i) * DC_LD + e);
+#pragma unroll
+      for (int i = 0; i < 4; i++) y[i] = ld4(b + (e + i) * DC_LD + tx * 4);
+      fma64(sum, x, y);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[i][j] += sum[i][j];
+  }
+}
+__device__ __forceinline__ void dc_write64(float* o, const float (&a)[2][4][4], int ty, int tx) {
+#pragma unroll
+  for (int f = 0; f < 2; f++)
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *reinterpret_cast<float4*>(o + (32 * f + ty * 4 + i) * 64 + tx * 4) = make_float4(a[f][i][0], a[f][i][1], a[f][i][2], a[f][i][3]);
+}
+
+// Grid (chunks, H, column tiles).
+template <bool DELTA>
+__global__ void __launch_bounds__(DC_TERM_THREADS, 3)
+delta_terms_kernel(const DcArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float bs[64], gs[64], cs[64], rl[64];      // b, g, c_i, r_Cj
+  float* ks = sm;                               // K
+  float* qs = sm + DC_TILE;                     // Q, then W
+  float* vs = sm + 2 * DC_TILE;                 // V, then U0
+  float* ls = sm + 3 * DC_TILE;                 // r, then L / b
+  const int c = blockIdx.x, h = blockIdx.y, z = blockIdx.z, tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  pdl_wait();
+  ScArgs f = {};
+  f.q_start = p.q_start;
+  f.R = p.R;
+  const Chunk ck = find_chunk(f, c);
+  if (ck.r < 0) return;
+  const int g = h / (p.H / p.G);
+  dc_stage<DC_TERM_THREADS>(p.k + (size_t)ck.t0 * p.k_stride + (size_t)g * p.D, p.k_stride, ck.len, 0, p.D, p.vec, ks);
+  if (z == 0) dc_stage<DC_TERM_THREADS>(p.q + (size_t)ck.t0 * p.q_stride + (size_t)g * p.D, p.q_stride, ck.len, 0, p.D, p.vec, qs);
+  dc_stage<DC_TERM_THREADS>(p.v + (size_t)ck.t0 * p.v_stride + (size_t)h * p.V, p.v_stride, ck.len, z * 64, p.V, p.vec, vs);
+  copies_end_group();
+  if (tid < 64) {                               // (behind the end: weight zero, no decay)
+    const bool on = tid < ck.len;
+    bs[tid] = !on ? 0.0f : DELTA ? p.gates[(size_t)(ck.t0 + tid) * p.gates_stride + h] : 1.0f;
+    gs[tid] = !on ? 1.0f : DELTA ? p.gates[(size_t)(ck.t0 + tid) * p.gates_stride + p.H + h] : p.head_decay[h];
+  }
+  __syncthreads();
+  if (tid < 64) {                               // r_ij of column j, downwards
+    float r = 1.0f;
+    for (int i = 0; i < 64; i++) {
+      r = i <= tid ? 1.0f : r * gs[i];
+      ls[i * DC_LD + tid] = i < tid ? 0.0f : r;
+    }
+    rl[tid] = r;
+  } else if (tid == 64) {
+    float r = 1.0f;
+    for (int i = 0; i < 64; i++) { r *= gs[i]; cs[i] = r; }
+    if (z == 0) p.total[(size_t)c * p.H + h] = r;
+  }
+  copies_wait<0>();
+  __syncthreads();
+  if (p.silu_in) {
+    dc_silu_tile<DC_TERM_THREADS>(ks);
+    if (z == 0) dc_silu_tile<DC_TERM_THREADS>(qs);
+    dc_silu_tile<DC_TERM_THREADS>(vs);
+    __syncthreads();
+  }
+  const size_t at = ((size_t)c * p.H + h) * 4096, atz = (((size_t)c * p.H + h) * p.tiles + z) * 4096;
+  if (z == 0) {
+    float acc[2][4][4] = {};
+    dc_rows_product(acc, qs, ks, ty, tx);
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int row = 32 * f + ty * 4 + i, col = tx + 16 * j;
+          p.qk[at + row * 64 + col] = col <= row ? acc[f][i][j] * ls[row * DC_LD + col] : 0.0f;
+        }
+  }
+  if (DELTA) {
+    float acc[2][4][4] = {};
+    dc_rows_product(acc, ks, ks, ty, tx);
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {           // (each entry of r is read and replaced by one thread)
+          const int row = 32 * f + ty * 4 + i;
+          float* e = ls + row * DC_LD + tx + 16 * j;
+          *e *= acc[f][i][j];
+        }
+    __syncthreads();                            // (and Q has been read)
+    {
+      // forward substitution: thread c < 64 the column c of W, the others a column of U0
+      const bool w = tid < 64;
+      const int col = tid & 63;
+      if (!w || z == 0) {
+        float x[64];
+#pragma unroll
+        for (int i = 0; i < 64; i++) {
+          // (four sums side by side: a row's chain is a quarter as long)
+          float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+#pragma unroll
+          for (int j4 = 0; j4 < i; j4 += 4) {
+            const float4 l = ld4(ls + i * DC_LD + j4);
+            s1 = fmaf(-l.x, x[j4], s1);
+            if (j4 + 1 < i) s2 = fmaf(-l.y, x[j4 + 1], s2);
+            if (j4 + 2 < i) s3 = fmaf(-l.z, x[j4 + 2], s3);
+            if (j4 + 3 < i) s0 = fmaf(-l.w, x[j4 + 3], s0);
+          }
+          const float s = (s0 + s1) + (s2 + s3);
+          x[i] = bs[i] * (w ? fmaf(cs[i], ks[i * DC_LD + col], s) : vs[i * DC_LD + col] + s);
+        }
+        float* to = w ? qs : vs;
+#pragma unroll
+        for (int i = 0; i < 64; i++) to[i * DC_LD + col] = x[i];
+      }
+    }
+  }
+  __syncthreads();
+  for (int x = tid; x < 64 * 16; x += DC_TERM_THREADS) {      // (all that is read of K from here on carries r_Cj)
+    float4* e = reinterpret_cast<float4*>(ks + (x >> 4) * DC_LD + (x & 15) * 4);
+    const float r = rl[x >> 4];
+    *e = make_float4(e->x * r, e->y * r, e->z * r, e->w * r);
+    if (DELTA) {
+      if (z == 0) *reinterpret_cast<float4*>(p.W + at + x * 4) = ld4(qs + (x >> 4) * DC_LD + (x & 15) * 4);
+      *reinterpret_cast<float4*>(p.U + atz + x * 4) = ld4(vs + (x >> 4) * DC_LD + (x & 15) * 4);
+    }
+  }
+  __syncthreads();
+  float b[2][4][4] = {};
+  dc_columns_product(b, ks, vs, ty, tx);
+  dc_write64(p.S + atz, b, ty, tx);
+  if (DELTA && z == 0) {
+    float a[2][4][4] = {};
+    dc_columns_product(a, ks, qs, ty, tx);
+#pragma unroll
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) a[f][i][j] = (32 * f + ty * 4 + i == tx * 4 + j ? cs[63] : 0.0f) - a[f][i][j];
+    dc_write64(p.A + at, a, ty, tx);
+  }
+}
+
+// Grid (requests, H, pieces of 8 columns): S <- A S + B from chunk to chunk.  A thread keeps two entries of the state; in
+// the product it has two rows and an eighth of their terms (the eighths are added behind a barrier).  All that a chunk
+// brings comes through a ring of asynchronous copies.  Bound by what shared memory hands to registers.
+template <bool DELTA>
+__global__ void __launch_bounds__(SC_THREADS)
+delta_pass_kernel(const DcArgs p) {
+  constexpr int C = DC_PASS_COLS, RING = DC_PASS_RING;
+  extern __shared__ __align__(16) float sm[];        // delta rule: RING tiles of A
+  constexpr int PARTS = 8;
+  __shared__ __align__(16) float bring[RING][64 * C], ss[DELTA ? 64 * C : 4], part[DELTA ? PARTS : 1][DELTA ? 64 * C : 4];
+  __shared__ float tring[RING];
+  __shared__ int first_s;
+  const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, d = tid / 4, c2 = tid % 4 * 2, v0 = blockIdx.z * C;
+  const int slot = p.state_slots[r];
+  if (tid < 32) {
+    int n = 0;
+    for (int x = tid; x < r; x += 32) n += (p.q_start[x + 1] - p.q_start[x] + SC_Q - 1) / SC_Q;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (tid == 0) first_s = n;
+  }
+  __syncthreads();
+  const int first = first_s, count = (p.q_start[r + 1] - p.q_start[r] + SC_Q - 1) / SC_Q;
+  if (count <= 0 || !sglc_index_ok(slot, p.n_slots, p.err)) return;
+  float* st = p.state + (((size_t)slot * p.H + h) * p.D + d) * p.V + v0 + c2;
+  const bool on0 = d < p.D && v0 + c2 < p.V, on1 = d < p.D && v0 + c2 + 1 < p.V;
+  float s0 = on0 ? st[0] : 0.0f, s1 = on1 ? st[1] : 0.0f;
+  float* tile = p.S + (((size_t)first * p.H + h) * p.tiles + v0 / 64) * 4096 + v0 % 64;
+  const size_t step = (size_t)p.H * p.tiles * 4096;
+  auto ask = [&](int c) {
+    if (c < count) {
+      if (DELTA) dc_stage64(p.A + ((size_t)(first + c) * p.H + h) * 4096, sm + c % RING * DC_TILE);
+      if (tid < 128) copy16(bring[c % RING] + tid * 4, tile + c * step + (tid >> 1) * 64 + (tid & 1) * 4, true);
+      else if (!DELTA && tid == 128) {
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(&tring[c % RING]);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(p.total + (size_t)(first + c) * p.H + h) : "memory");
+      }
+    }
+    copies_end_group();
+  };
+  for (int c = 0; c < RING - 1; c++) ask(c);
+  for (int c = 0; c < count; c++) {
+    ask(c + RING - 1);
+    if (DELTA) *reinterpret_cast<float2*>(ss + d * C + c2) = make_float2(s0, s1);
+    copies_wait<RING - 1>();
+    __syncthreads();                                 // chunk c is there (its contribution has left its place) and S is
+    *reinterpret_cast<float2*>(tile + c * step + d * 64 + c2) = make_float2(s0, s1);
+    const float2 own = *reinterpret_cast<const float2*>(bring[c % RING] + d * C + c2);
+    if (DELTA) {
+      const int row = tid & 31, q = tid >> 5;          // (rows `row` and `row` + 32, an eighth of their terms)
+      const float* a = sm + c % RING * DC_TILE + row * DC_LD + q * 8;
+      float acc[2][C] = {};
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        const float4 a0 = ld4(a + e), a1 = ld4(a + 32 * DC_LD + e);
+        const float av[2][4] = {{a0.x, a0.y, a0.z, a0.w}, {a1.x, a1.y, a1.z, a1.w}};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float4 x = ld4(ss + (q * 8 + e + i) * C), y = ld4(ss + (q * 8 + e + i) * C + 4);
+#pragma unroll
+          for (int w = 0; w < 2; w++) {
+            acc[w][0] = fmaf(av[w][i], x.x, acc[w][0]); acc[w][1] = fmaf(av[w][i], x.y, acc[w][1]);
+            acc[w][2] = fmaf(av[w][i], x.z, acc[w][2]); acc[w][3] = fmaf(av[w][i], x.w, acc[w][3]);
+            acc[w][4] = fmaf(av[w][i], y.x, acc[w][4]); acc[w][5] = fmaf(av[w][i], y.y, acc[w][5]);
+            acc[w][6] = fmaf(av[w][i], y.z, acc[w][6]); acc[w][7] = fmaf(av[w][i], y.w, acc[w][7]);
+          }
+        }
+      }
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        float* to = &part[q][(row + 32 * w) * C];
+        *reinterpret_cast<float4*>(to) = make_float4(acc[w][0], acc[w][1], acc[w][2], acc[w][3]);
+        *reinterpret_cast<float4*>(to + 4) = make_float4(acc[w][4], acc[w][5], acc[w][6], acc[w][7]);
+      }
+      __syncthreads();
+      float2 sum[PARTS];
+#pragma unroll
+      for (int x = 0; x < PARTS; x++) sum[x] = *reinterpret_cast<const float2*>(&part[x][d * C + c2]);
+      s0 = own.x + (((sum[0].x + sum[1].x) + (sum[2].x + sum[3].x)) + ((sum[4].x + sum[5].x) + (sum[6].x + sum[7].x)));
+      s1 = own.y + (((sum[0].y + sum[1].y) + (sum[2].y + sum[3].y)) + ((sum[4].y + sum[5].y) + (sum[6].y + sum[7].y)));
+    } else {
+      const float t = tring[c % RING];
+      s0 = fmaf(t, s0, own.x);
+      s1 = fmaf(t, s1, own.y);
+      __syncthreads();                               // (the slot may be filled again)
+    }
+  }
+  if (on0) st[0] = s0;
+  if (on1) st[1] = s1;
+}
+
+// Grid (chunks, H, column tiles): the read-outs.
+template <bool DELTA>
+__global__ void __launch_bounds__(SC_THREADS, 3)
+delta_read_kernel(const DcArgs p) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float gs[64], cs[64];
+  float* ss = sm;                               // S_in
+  float* qs = sm + DC_TILE;
+  float* us = sm + 2 * DC_TILE;                 // delta rule: W, then U; decay form: V
+  float* ms = sm + 3 * DC_TILE;
+  const int c = blockIdx.x, h = blockIdx.y, z = blockIdx.z, tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  ScArgs f = {};
+  f.q_start = p.q_start;
+  f.R = p.R;
+  const Chunk ck = find_chunk(f, c);
+  if (ck.r < 0) return;
+  const int g = h / (p.H / p.G);
+  const size_t at = ((size_t)c * p.H + h) * 4096, atz = (((size_t)c * p.H + h) * p.tiles + z) * 4096;
+  dc_stage64(p.S + atz, ss);
+  dc_stage<SC_THREADS>(p.q + (size_t)ck.t0 * p.q_stride + (size_t)g * p.D, p.q_stride, ck.len, 0, p.D, p.vec, qs);
+  if (DELTA) dc_stage64(p.W + at, us);
+  else dc_stage<SC_THREADS>(p.v + (size_t)ck.t0 * p.v_stride + (size_t)h * p.V, p.v_stride, ck.len, z * 64, p.V, p.vec, us);
+  copies_end_group();
+  dc_stage64(p.qk + at, ms);
+  copies_end_group();
+  if (tid < 64) gs[tid] = tid >= ck.len ? 1.0f : DELTA ? p.gates[(size_t)(ck.t0 + tid) * p.gates_stride + p.H + h] : p.head_decay[h];
+  float4 u0[4];
+  if (DELTA) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) u0[i] = ld4(p.U + atz + (ty * 4 + i) * 64 + tx * 4);
+  }
+  copies_wait<1>();
+  __syncthreads();
+  if (tid == 0) {
+    float r = 1.0f;
+    for (int i = 0; i < 64; i++) { r *= gs[i]; cs[i] = r; }
+  }
+  if (p.silu_in) {
+    dc_silu_tile<SC_THREADS>(qs);
+    if (!DELTA) dc_silu_tile<SC_THREADS>(us);
+    __syncthreads();
+  }
+  if (DELTA) {                                           // U0 - W S
+    float w[4][4] = {};
+    dc_product(w, us, ss, 64, ty, tx);
+#pragma unroll
+    for (int i = 0; i < 4; i++) u0[i] = make_float4(u0[i].x - w[i][0], u0[i].y - w[i][1], u0[i].z - w[i][2], u0[i].w - w[i][3]);
+  }
+  float acc[4][4] = {};
+  dc_product(acc, qs, ss, 64, ty, tx);
+  copies_wait<0>();
+  __syncthreads();                                       // (W has been read, c_i are there)
+  if (DELTA) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *reinterpret_cast<float4*>(us + (ty * 4 + i) * DC_LD + tx * 4) = u0[i];
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[i][e] *= cs[ty * 4 + i];
+  __syncthreads();
+  dc_product(acc, ms, us, (tid / 32 + 1) * 8, ty, tx);   // (no row of this warp sees a later token)
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int t = ty * 4 + i, v = z * 64 + tx * 4;
+    if (t >= ck.len) continue;
+    float* o = p.out + (size_t)(ck.t0 + t) * p.out_stride + (size_t)h * p.V + v;
+    if (p.vec) {
+      if (v < p.V) *reinterpret_cast<float4*>(o) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        if (v + e < p.V) o[e] = acc[i][e];
+    }
+  }
+}
+
+// gates: the delta rule's [T][2H] (b, then the decays), or null with head_decay [H]: the decay form.  silu_in:
+// silu of q, k and v first.  ws: float, n_chunks * H * (1 + 4096 * (delta rule: 3 + 2 tiles; decay form: 1 + tiles))
+// entries, tiles = ceil(V / 64), n_chunks being at least the chunks of the step.
+SGLC_API int sglc_delta_chunks(const float* q, long long q_stride, const float* k, long long k_stride, const float* v,
+                               long long v_stride, const float* gates, long long gates_stride, const float* head_decay,
+                               float* out, long long out_stride, float* state, int n_slots, const int* q_start,
+                               const int* state_slots, int R, int H, int G, int D, int V, int silu_in, float* ws,
+                               int n_chunks, int* err, cudaStream_t stream) {
+  if (R <= 0 || n_chunks <= 0) return SGLC_OK;
+  if (H <= 0 || G <= 0 || H % G != 0 || D <= 0 || V <= 0 || !ws || (!gates) == (!head_decay)) return SGLC_ERR_ARGUMENT;
+  const int tiles = (V + 63) / 64, pieces = (V + DC_PASS_COLS - 1) / DC_PASS_COLS;
+  if (D > 64 || H > 65535 || pieces > 65535) return SGLC_ERR_UNSUPPORTED;
+  DcArgs p = {};
+  p.q = q; p.q_stride = q_stride; p.k = k; p.k_stride = k_stride; p.v = v; p.v_stride = v_stride;
+  p.gates = gates; p.gates_stride = gates_stride; p.head_decay = head_decay; p.out = out; p.out_stride = out_stride;
+  p.state = state; p.n_slots = n_slots; p.q_start = q_start; p.state_slots = state_slots;
+  p.R = R; p.H = H; p.G = G; p.D = D; p.V = V; p.tiles = tiles; p.n_chunks = n_chunks; p.silu_in = silu_in; p.err = err;
+  const size_t unit = (size_t)n_chunks * H * 4096;
+  p.qk = ws;
+  p.S = p.qk + unit;
+  float* end = p.S + unit * tiles;
+  if (gates) {
+    p.W = end;
+    p.A = p.W + unit;
+    p.U = p.A + unit;
+    end = p.U + unit * tiles;
+  }
+  p.total = end;
+  auto al = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
+  if (!al(ws)) return SGLC_ERR_ARGUMENT;
+  p.vec = D % 4 == 0 && V % 4 == 0 && (q_stride | k_stride | v_stride | out_stride) % 4 == 0 && al(q) && al(k) && al(v) && al(out);
+  constexpr int smem = 4 * DC_TILE * 4;
+  const dim3 grid(n_chunks, H, tiles), pass(R, H, pieces);
+  auto go = [&](auto* terms, auto* over, auto* read) {
+    cudaFuncSetAttribute(terms, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(read, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    // (no early start behind one another: blocks that wait take up the room of running ones unevenly)
+    const int pass_smem = gates ? DC_PASS_RING * DC_TILE * 4 : 0;
+    cudaFuncSetAttribute(over, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_PASS_RING * DC_TILE * 4);
+    int rc = sglc_launch(terms, grid, dim3(DC_TERM_THREADS), smem, stream, 1, true, p);
+    if (rc == SGLC_OK) rc = sglc_launch(over, pass, dim3(SC_THREADS), pass_smem, stream, 1, false, p);
+    if (rc == SGLC_OK) rc = sglc_launch(read, grid, dim3(SC_THREADS), smem, stream, 1, false, p);
+    return rc;
+  };
+  return gates ? go(delta_terms_kernel<true>, delta_pass_kernel<true>, delta_read_kernel<true>)
+               : go(delta_terms_kernel<false>, delta_pass_kernel<false>, delta_read_kernel<false>);
+}
+
 // Every request brings one token (token r is request r's).  Grid (requests, H, column tiles of SS_COLS); a
 // thread keeps W columns of every SS_ROWS-th row.
 constexpr int SS_COLS = 64, SS_DEEP = 8;

@@ -64,6 +64,24 @@ def _stacked(store, refs):
     return store.computed("+".join(r.name for r in refs), lambda: torch.cat([r.tensor.float() for r in refs], 0))
 
 
+def _chunk_bytes(mode, H, D, V):
+    """Bytes of workspace a token needs where a recurrence goes in chunks."""
+    if D > ops.DELTA_CHUNKS_MAX_DIM:
+        return 0
+    return 4 * ops.delta_chunks_workspace(mode, ops.STATE_CHUNK, 1, H, V) // ops.STATE_CHUNK
+
+
+def _matrix_state(ctx, mode, q, k, v, out, state, H, G, D, V, **kw):
+    """The recurrence over the step's tokens: in chunks side by side where portions are long, else token by token."""
+    if ops.delta_chunks_pay(mode, out.shape[0], ctx.R, ctx.max_q_len, H, D):
+        mark = ctx.mark()
+        ws = ctx.alloc((ops.delta_chunks_workspace(mode, out.shape[0], ctx.R, H, V),), torch.float32)
+        ops.delta_chunks(mode, q, k, v, out, state, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, ws, **kw)
+        ctx.release(mark)
+    else:
+        ops.matrix_state(mode, q, k, v, out, state, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, **kw)
+
+
 @register_part("mixer", "gated_delta")
 class GatedDeltaRule(Part):
     """The gated delta rule: per head a matrix state S [dim x v_dim] that decays, is corrected
@@ -119,7 +137,8 @@ class GatedDeltaRule(Part):
         p = self.params
         H, G, D, V = p["n_heads"], p["n_qk_heads"], p["dim"], p["v_dim"]
         act = 4 if self.rt.dtype == "float32" else 2
-        return 4 * (2 * G * D + 2 * H * V + 2 * H + 8) + 4 * (2 * G * D + H * V) + 8 * H + 4 * H * V + act * H * V + 2048
+        return 4 * (2 * G * D + 2 * H * V + 2 * H + 8) + 4 * (2 * G * D + H * V) + 8 * H + 4 * H * V + act * H * V + 2048 \
+            + _chunk_bytes("delta", H, D, V)
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params
@@ -135,8 +154,8 @@ class GatedDeltaRule(Part):
                        self.segments, unit_eps=self.UNIT_EPS,
                        gates=(H, gate_col, gate_col + H, self.A_log, self.dt_bias, gates))
         o = ctx.alloc((T, H * V), torch.float32)
-        ops.matrix_state("delta", ctx.columns(y, 0, G * D), ctx.columns(y, G * D, 2 * G * D), ctx.columns(y, 2 * G * D, C),
-                         o, state.tensor, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, gates=gates)
+        _matrix_state(ctx, "delta", ctx.columns(y, 0, G * D), ctx.columns(y, G * D, 2 * G * D),
+                      ctx.columns(y, 2 * G * D, C), o, state.tensor, H, G, D, V, gates=gates)
         z = ctx.alloc((T, H * V), self.rt.act_dtype)
         ops.gated_norm(o, ctx.columns(pre, C, C + H * V), self.norm, z, H, V, float(p["eps"]), "silu")
         return self.out.forward(ctx, z, out=out, residual=residual)
@@ -176,7 +195,7 @@ class LinearDecayAttention(Part):
         p = self.params
         H, D, V = p["n_heads"], p["dim"], p["v_dim"]
         act = 4 if self.rt.dtype == "float32" else 2
-        return 4 * (2 * H * D + 2 * H * V) + 4 * H * V + act * H * V + 1024
+        return 4 * (2 * H * D + 2 * H * V) + 4 * H * V + act * H * V + 1024 + _chunk_bytes("decay", H, D, V)
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params
@@ -185,9 +204,9 @@ class LinearDecayAttention(Part):
         pre = ctx.alloc((T, 2 * H * D + 2 * H * V), torch.float32)
         self.inp.forward(ctx, h, out=pre)
         o = ctx.alloc((T, H * V), torch.float32)
-        ops.matrix_state("decay", ctx.columns(pre, 0, H * D), ctx.columns(pre, H * D, 2 * H * D),
-                         ctx.columns(pre, 2 * H * D, 2 * H * D + H * V), o, cache.tensor, ctx.q_start, ctx.state_slots,
-                         ctx.R, H, H, D, V, head_decay=self.decay, silu_in=True)
+        _matrix_state(ctx, "decay", ctx.columns(pre, 0, H * D), ctx.columns(pre, H * D, 2 * H * D),
+                      ctx.columns(pre, 2 * H * D, 2 * H * D + H * V), o, cache.tensor, H, H, D, V, head_decay=self.decay,
+                      silu_in=True)
         z = ctx.alloc((T, H * V), self.rt.act_dtype)
         ops.gated_norm(o, ctx.columns(pre, 2 * H * D + H * V, 2 * H * D + 2 * H * V), self.norm, z, 1, H * V,
                        float(p["eps"]), "sigmoid")

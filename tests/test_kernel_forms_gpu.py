@@ -115,3 +115,55 @@ def test_stream_decode_shares_items_between_blocks(T, H, Hkv, D, window):
         ops.attention_decode(c["q"], cache, c["bt"], None, c["positions"], out, H, scale, window, max(lens), variant="stream", n_tokens=T, **kw)
         assert float((out.double().cpu() - ref).abs().max()) < 1.2e-2, fused
         assert not fused or torch.equal(cache, c["cache"])
+
+
+# -- recurrences in chunks ----------------------------------------------------------------------------
+def _walk(mode, q, k, v, gates, decay, H, G, D, V, S):
+    n = q.shape[0]
+    q, k, v = (t.double().reshape(n, -1, w) for t, w in ((q, D), (k, D), (v, V)))
+    q, k = q.repeat_interleave(H // G, 1), k.repeat_interleave(H // G, 1)
+    out = torch.zeros(n, H, V, dtype=torch.float64, device=DEV)
+    for t in range(n):
+        S = S * (gates[t, H:] if mode == "delta" else decay).double()[:, None, None]
+        u = gates[t, :H].double()[:, None] * (v[t] - torch.einsum("hdv,hd->hv", S, k[t])) if mode == "delta" else v[t]
+        S = S + k[t][:, :, None] * u[:, None, :]
+        out[t] = torch.einsum("hdv,hd->hv", S, q[t])
+    return out.reshape(n, H * V), S
+
+
+@pytest.mark.parametrize("mode,H,G,D,V,rate", [("delta", 4, 2, 64, 64, 0.1), ("delta", 3, 3, 40, 100, 0.002), ("delta", 2, 1, 7, 9, 3.0),
+                                               ("decay", 2, 2, 64, 64, 0.05), ("decay", 2, 2, 33, 70, 0.5)])
+def test_recurrences_in_chunks(mode, H, G, D, V, rate):
+    """Portions of 1 to 200 tokens over shuffled slots: chunk edges, states carried in, decays near one, far from it
+    and zero, sizes no vector load fits.  The chunks may not be further off than 2 x the walk token by token."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(D)
+    lens = [200, 1, 64, 65, 127]
+    T, R = sum(lens), len(lens)
+    q, k, v = (torch.randn(T, n, generator=g).to(DEV) for n in (G * D, G * D, H * V))
+    k = torch.nn.functional.normalize(k.reshape(T, G, D), dim=-1).reshape(T, G * D).contiguous()
+    gates = torch.cat([torch.rand(T, H, generator=g), torch.exp(-rate * 2 * torch.rand(T, H, generator=g))], 1).to(DEV)
+    if rate > 1:
+        gates[::19, H:] = 0.0
+    decay = torch.exp(-rate * torch.arange(1, H + 1)).to(DEV)
+    S0 = torch.randn(R + 2, H, D, V, generator=g).to(DEV)
+    starts, slots = np.concatenate([[0], np.cumsum(lens)]), [3, 0, 6, 1, 4]
+    i32 = lambda x: torch.tensor(np.asarray(x), dtype=torch.int32, device=DEV)      # noqa: E731
+    kw = dict(gates=gates) if mode == "delta" else dict(head_decay=decay)
+    got = {}
+    for way in ("walk", "chunks"):
+        S, o = S0.clone(), torch.full((T, H * V), float("nan"), device=DEV)
+        if way == "walk":
+            ops.matrix_state(mode, q, k, v, o, S, i32(starts), i32(slots), R, H, G, D, V, **kw)
+        else:
+            ws = torch.full((ops.delta_chunks_workspace(mode, T, R, H, V),), float("nan"), device=DEV)
+            ops.delta_chunks(mode, q, k, v, o, S, i32(starts), i32(slots), R, H, G, D, V, ws, **kw)
+        got[way] = (o, S)
+    for r, slot in enumerate(slots):
+        at = slice(starts[r], starts[r + 1])
+        want, state = _walk(mode, q[at], k[at], v[at], gates[at], decay, H, G, D, V, S0[slot].double())
+        for i, (ref, pick) in enumerate(((want, lambda t: t[0][at]), (state, lambda t: t[1][slot]))):
+            err = {w: float((pick(got[w]).double() - ref).norm() / ref.norm()) for w in got}
+            assert err["chunks"] < max(2.0 * err["walk"], 5e-7), (r, i, err)
+    for slot in set(range(R + 2)) - set(slots):
+        assert torch.equal(got["chunks"][1][slot], S0[slot])
