@@ -1187,6 +1187,45 @@ def delta_chunks(mode, q, k, v, out, state, q_start, state_slots, n_requests, n_
     _check(lib, code, f"delta_chunks ({mode}, {dim} x {v_dim})", n_kernels=3)
 
 
+def delta_step_fits(state, dim, v_dim):
+    """Whether delta_step takes such states."""
+    return dim <= MATRIX_STATE_MAX_DIM and v_dim % 4 == 0 and state.data_ptr() % 16 == 0
+
+
+def delta_step(mode, q, k, v, out, state, state_slots, n_heads, n_qk_heads, dim, v_dim, gates=None, head_decay=None,
+               silu_in=False):
+    """matrix_state's modes "delta" and "decay" for a step in which every request brings one token: row r is
+    request r's."""
+    _need_cuda(q, k, v, out, state, state_slots, gates, head_decay)
+    R = out.shape[0]
+    _f32_rows(q, "delta_step: q", n_qk_heads * dim)
+    _f32_rows(k, "delta_step: k", n_qk_heads * dim)
+    _f32_rows(v, "delta_step: v", n_heads * v_dim)
+    _f32_rows(out, "delta_step: out", n_heads * v_dim)
+    if mode not in ("delta", "decay"):
+        raise KernelError(f"delta_step: no mode '{mode}'")
+    if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (n_heads, dim, v_dim):
+        raise KernelError(f"delta_step: the state is float32 [n_slots, {n_heads}, {dim}, {v_dim}]")
+    if mode == "delta":
+        if gates is None:
+            raise KernelError("delta_step: the delta rule takes its gates")
+        _f32_rows(gates, "delta_step: gates", 2 * n_heads)
+    elif gates is not None or head_decay is None or head_decay.dtype != torch.float32 or head_decay.numel() != n_heads \
+            or not head_decay.is_contiguous():
+        raise KernelError("delta_step: the decay form takes one float32 decay per head")
+    _i32(state_slots, "state_slots")
+    if state_slots.numel() < R or min(t.shape[0] for t in (q, k, v)) < R or (gates is not None and gates.shape[0] < R):
+        raise KernelError("delta_step: a slot and a row of q, k, v and gates for every request")
+    lib = build.load("state_chunks")
+    code = lib.sglc_delta_step(_ptr(q), ctypes.c_longlong(q.stride(0)), _ptr(k), ctypes.c_longlong(k.stride(0)), _ptr(v),
+                               ctypes.c_longlong(v.stride(0)), _ptr(gates),
+                               ctypes.c_longlong(gates.stride(0) if gates is not None else 0), _ptr(head_decay), _ptr(out),
+                               ctypes.c_longlong(out.stride(0)), _ptr(state), state.shape[0], _ptr(state_slots), R,
+                               int(n_heads), int(n_qk_heads), int(dim), int(v_dim), 1 if silu_in else 0,
+                               _ptr(tc_error_flag(q.device)), _stream())
+    _check(lib, code, f"delta_step ({mode}, {dim} x {v_dim})")
+
+
 def state_step(q, k, v, gates, out, state, state_slots, n_heads, n_groups, dim, v_dim, skip=None):
     """matrix_state's gated form (with its skip) for a step in which every request brings one token: row r
     is request r's.  gates: float32 [R, 2H] (input weights, decays)."""

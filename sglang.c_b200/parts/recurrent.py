@@ -72,8 +72,11 @@ def _chunk_bytes(mode, H, D, V):
 
 
 def _matrix_state(ctx, mode, q, k, v, out, state, H, G, D, V, **kw):
-    """The recurrence over the step's tokens: in chunks side by side where portions are long, else token by token."""
-    if ops.delta_chunks_pay(mode, out.shape[0], ctx.R, ctx.max_q_len, H, D):
+    """The recurrence over the step's tokens: one token a request in a pass over the states, long portions in chunks
+    side by side, else token by token."""
+    if ctx.max_q_len == 1 and ops.delta_step_fits(state, D, V):
+        ops.delta_step(mode, q, k, v, out, state, ctx.state_slots, H, G, D, V, **kw)
+    elif ops.delta_chunks_pay(mode, out.shape[0], ctx.R, ctx.max_q_len, H, D):
         mark = ctx.mark()
         ws = ctx.alloc((ops.delta_chunks_workspace(mode, out.shape[0], ctx.R, H, V),), torch.float32)
         ops.delta_chunks(mode, q, k, v, out, state, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, ws, **kw)

@@ -167,3 +167,40 @@ def test_recurrences_in_chunks(mode, H, G, D, V, rate):
             assert err["chunks"] < max(2.0 * err["walk"], 5e-7), (r, i, err)
     for slot in set(range(R + 2)) - set(slots):
         assert torch.equal(got["chunks"][1][slot], S0[slot])
+
+
+# -- steps of one token a request ------------------------------------------------------------------------
+@pytest.mark.parametrize("mode,H,G,D,V", [("delta", 4, 2, 64, 64), ("delta", 3, 3, 40, 100), ("delta", 2, 1, 129, 68), ("delta", 2, 2, 256, 4),
+                                          ("decay", 3, 3, 64, 64), ("decay", 2, 2, 7, 12), ("decay", 2, 2, 128, 132)])
+def test_recurrences_of_single_tokens(mode, H, G, D, V):
+    """Key sizes at the edges of the rows a thread keeps, value sizes of one tile, a part of one and several; no further
+    off than 2 x the walk, or a handful of roundings."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(D + V)
+    R = 5
+    q, k, v = (torch.randn(R, n, generator=g).to(DEV) for n in (G * D, G * D, H * V))
+    k = torch.nn.functional.normalize(k.reshape(R, G, D), dim=-1).reshape(R, G * D).contiguous()
+    gates = torch.rand(R, 2 * H, generator=g).to(DEV)
+    decay = torch.rand(H, generator=g).to(DEV)
+    S0 = torch.randn(R + 2, H, D, V, generator=g).to(DEV)
+    slots = [3, 0, 6, 1, 4]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)      # noqa: E731
+    kw = dict(gates=gates) if mode == "delta" else dict(head_decay=decay)
+    for silu in (False, True):
+        got = {}
+        for way in ("walk", "step"):
+            S, o = S0.clone(), torch.full((R, H * V), float("nan"), device=DEV)
+            if way == "walk":
+                ops.matrix_state(mode, q, k, v, o, S, i32(list(range(R + 1))), i32(slots), R, H, G, D, V, silu_in=silu, **kw)
+            else:
+                ops.delta_step(mode, q, k, v, o, S, i32(slots), H, G, D, V, silu_in=silu, **kw)
+            got[way] = (o, S)
+        act = (lambda t: torch.nn.functional.silu(t.double())) if silu else (lambda t: t)
+        for r, slot in enumerate(slots):
+            at = slice(r, r + 1)
+            want, state = _walk(mode, act(q[at]), act(k[at]), act(v[at]), gates[at], decay, H, G, D, V, S0[slot].double())
+            for ref, pick in ((want, lambda t: t[0][at]), (state, lambda t: t[1][slot])):
+                err = {w: float((pick(got[w]).double() - ref).norm() / ref.norm()) for w in got}
+                assert err["step"] < max(2.0 * err["walk"], 5e-7), (silu, r, err)
+        for slot in set(range(R + 2)) - set(slots):
+            assert torch.equal(got["step"][1][slot], S0[slot])
