@@ -204,3 +204,32 @@ def test_recurrences_of_single_tokens(mode, H, G, D, V):
                 assert err["step"] < max(2.0 * err["walk"], 5e-7), (silu, r, err)
         for slot in set(range(R + 2)) - set(slots):
             assert torch.equal(got["step"][1][slot], S0[slot])
+
+
+@pytest.mark.parametrize("taps,D,V", [(2, 12, 7), (3, 33, 64), (4, 64, 32)])
+def test_short_convolution_of_single_tokens(taps, D, V):
+    """Token by token or as one portion: the same bits, and the same inputs left for the next step."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(taps)
+    R, n, G, H = 3, 6, 2, 3
+    C = 2 * G * D + H * V
+    x = torch.randn(n, R, C + 2 * H, generator=g).to(DEV)
+    w, a_log, dt = torch.randn(C, taps, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    segs = [(0, G, D, 1, D ** -0.5), (G * D, G, D, 1, 1.0), (2 * G * D, H, V, 0, 1.0)]
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)      # noqa: E731
+    tail0 = torch.randn(5, taps - 1, C, generator=g).to(DEV)
+
+    def run(rows, lens, tail):
+        T = sum(lens)
+        y, gates = torch.empty(T, C, device=DEV), torch.empty(T, 2 * H, device=DEV)
+        starts = np.concatenate([[0], np.cumsum(lens)]).tolist()
+        ops.short_conv(rows.contiguous(), w, tail, y, i32([r for r, m in enumerate(lens) for _ in range(m)]), i32(starts), i32([3, 1, 4]),
+                       R, segs, gates=(H, C, C + H, a_log, dt, gates))
+        return y, gates
+
+    whole, stepped = tail0.clone(), tail0.clone()
+    y, gates = run(x.transpose(0, 1).reshape(R * n, -1), [n] * R, whole)
+    steps = [run(x[t], [1] * R, stepped) for t in range(n)]
+    assert torch.equal(y.view(R, n, C).transpose(0, 1), torch.stack([s[0] for s in steps]))
+    assert torch.equal(gates.view(R, n, -1).transpose(0, 1), torch.stack([s[1] for s in steps]))
+    assert torch.equal(whole, stepped)
