@@ -109,6 +109,35 @@ __device__ __forceinline__ void route(const RouterArgs& a, int t, const float* z
       if (e < E && !((kept >> (e / per)) & 1ull)) c[i] = -INFINITY;
     }
   }
+  if (E <= 32) {
+    // An expert a lane: its place in the order of choice is the number of better ones, which no lane waits for
+    // (`top` rounds of a maximum over the warp are a chain of 250 cycles each).  8 of 8
+    // experts, 8 / 2,048 tokens 4.0 / 9.9 -> 2.2 / 3.3 us; with the product 4.7 -> 3.0 (the prefetch below its part).
+    const unsigned bits = __float_as_uint(c[0]), mine = bits & 0x80000000u ? ~bits : bits | 0x80000000u;   // (ordered as c is)
+    int place = 0;
+#pragma unroll 8
+    for (int e = 0; e < E; e++) {
+      const unsigned other = __shfl_sync(0xffffffffu, mine, e);
+      place += other > mine || (other == mine && e < lane);
+    }
+    const bool on = lane < E && place < a.top;
+    __syncwarp();                              // (the group scores have been read)
+    if (on) {
+      cs[place] = s[0];
+      a.ids[(size_t)t * a.top + place] = lane;
+    }
+    __syncwarp();
+    float sum = 0.0f;
+    for (int n = 0; n < a.top; n++) sum += cs[n];
+    const float f = (a.renorm ? 1.0f / (sum + a.renorm_eps) : 1.0f) * a.weight_scale, w = on ? s[0] * f : 0.0f;
+    if (on) a.wts[(size_t)t * a.top + place] = w;
+    if (lane < E) a.dense[(size_t)t * a.dense_stride + lane] = w;
+    if (a.pass) {
+      const float handed_on = warp_sum(lane < E && lane >= E - a.n_pass ? w : 0.0f);
+      if (lane == 0) a.pass[t] = handed_on;
+    }
+    return;
+  }
   unsigned chosen = 0u;                        // bit i: expert lane + 32 i is taken
   float sum = 0.0f;
   for (int n = 0; n < a.top; n++) {
@@ -188,6 +217,10 @@ router_product_kernel(const RouterArgs a) {
   __shared__ float zs[ROUTER_MAX_EXPERTS], cs[ROUTER_MAX_EXPERTS];
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x;
+  for (int e = warp; e < a.E; e += ROUTER_WARPS) {             // the matrix into L2 ahead of the wait
+    const char* row = reinterpret_cast<const char*>(static_cast<const TA*>(a.w) + (size_t)e * a.K);
+    for (size_t at = lane * 128; at < a.K * sizeof(TA); at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + at));
+  }
   pdl_wait();
   const TA* h = static_cast<const TA*>(a.h) + (size_t)t * a.h_stride;
   for (int e = warp; e < a.E; e += ROUTER_WARPS) {

@@ -233,3 +233,20 @@ def test_short_convolution_of_single_tokens(taps, D, V):
     assert torch.equal(y.view(R, n, C).transpose(0, 1), torch.stack([s[0] for s in steps]))
     assert torch.equal(gates.view(R, n, -1).transpose(0, 1), torch.stack([s[1] for s in steps]))
     assert torch.equal(whole, stepped)
+
+
+@pytest.mark.parametrize("E,top", [(1, 1), (8, 8), (8, 3), (31, 5), (32, 32), (33, 4), (96, 8)])
+def test_router_order_of_choice(E, top):
+    """Logits with many ties on both sides of 32 experts: the larger first, the lower index first among equals."""
+    ops = _ops()
+    T = 37
+    z = torch.randint(-3, 4, (T, E), generator=torch.Generator().manual_seed(E), dtype=torch.int64).float().to(DEV)
+    dense, ids, wts = torch.empty(T, E, device=DEV), torch.empty(T, top, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    ops.router(z, None, dense, ids, wts, top, renorm=True, weight_scale=1.5)
+    want = torch.sort(z, dim=1, descending=True, stable=True).indices[:, :top]
+    assert torch.equal(ids.long(), want)
+    s = torch.sigmoid(z.double())
+    w = torch.gather(s, 1, want)
+    w = w / w.sum(1, keepdim=True) * 1.5
+    assert float((wts.double() - w).abs().max()) < 1e-6
+    assert float((dense.double() - torch.zeros_like(s).scatter(1, want, w)).abs().max()) < 1e-6
