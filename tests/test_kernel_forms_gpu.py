@@ -250,3 +250,20 @@ def test_router_order_of_choice(E, top):
     w = w / w.sum(1, keepdim=True) * 1.5
     assert float((wts.double() - w).abs().max()) < 1e-6
     assert float((dense.double() - torch.zeros_like(s).scatter(1, want, w)).abs().max()) < 1e-6
+
+
+@pytest.mark.parametrize("width", [64, 65, 256, 257])
+def test_gated_norm_at_the_edges_of_what_a_lane_keeps(width):
+    ops = _ops()
+    g = torch.Generator().manual_seed(width)
+    T, groups = 5, 3
+    o, z = (torch.randn(T, groups * width, generator=g).to(DEV) for _ in range(2))
+    gain = torch.randn(width, generator=g).to(DEV)
+    x = o.double().view(T, groups, width)
+    x = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * gain.double()
+    for act, gate in (("silu", torch.nn.functional.silu(z.double())), ("sigmoid", torch.sigmoid(z.double())), ("none", None)):
+        y = torch.empty_like(o)
+        ops.gated_norm(o, None if gate is None else z, gain, y, groups, width, 1e-5, act)
+        want = x.reshape(T, -1) * (1.0 if gate is None else gate)
+        # about ten 32-bit roundings a value (2^-24 each) and a sum of `width` squares
+        assert float(((y.double() - want).abs() / (want.abs() + 1e-3)).max()) < 1e-5
