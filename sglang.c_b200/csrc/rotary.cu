@@ -26,15 +26,27 @@ __device__ __forceinline__ float turn_v(float u, float v, float cs, float sn) { 
 
 template <typename TA>
 __global__ void __launch_bounds__(ROT_WARPS * 32)
-rotary_kv_kernel(const float* __restrict__ x, long long x_stride, const int* __restrict__ positions,
+rotary_kv_kernel(const float* x, long long x_stride, const int* __restrict__ positions,
                  const double* __restrict__ freq, float mult, int dims, int norm, float eps,
                  TA* __restrict__ q_out, long long q_stride, TA* __restrict__ cache, const int* __restrict__ slots,
                  int T, int H, int G, int D, int V, int page_size, int n_pages, int* err) {
   __shared__ float buf[ROT_WARPS][ROT_MAX_DIM];
+  __shared__ float2 turn[ROT_MAX_DIM / 2];
   pdl_launch_dependents();
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pos = positions[t];                // (the step's own array: no kernel of the step writes it)
+  // (cosine, sine) of the token's pairs, once for all of its rows and ahead of the wait (x is not __restrict__: its loads
+  // might move ahead of it).  8 tokens
+  // of 15 turned heads in a decode step's chain: 6.6 -> 5.7 us.
+  for (int i = threadIdx.x; i < dims / 2; i += ROT_WARPS * 32) {
+    double a = (double)pos * freq[i];
+    a -= floor(a * 0.15915494309189535) * 6.283185307179586;
+    float sn, cs;
+    sincosf((float)a, &sn, &cs);
+    turn[i] = make_float2(cs * mult, sn * mult);
+  }
   pdl_wait();
-  const int pos = positions[t];
+  __syncthreads();
   const int slot = slots[t];
   const int page = slot / page_size, off = slot % page_size;
   const bool page_ok = slot >= 0 && sglc_index_ok(page, n_pages, err);
@@ -55,11 +67,7 @@ rotary_kv_kernel(const float* __restrict__ x, long long x_stride, const int* __r
     const float* src = xr + (size_t)row * D;
     float ss = 0.0f;
     for (int i = lane; i < half; i += 32) {
-      double a = (double)pos * freq[i];
-      a -= floor(a * 0.15915494309189535) * 6.283185307179586;
-      float sn, cs;
-      sincosf((float)a, &sn, &cs);
-      sn *= mult; cs *= mult;
+      const float cs = turn[i].x, sn = turn[i].y;
       const float u = src[i], v = src[i + half];
       const float ru = u * cs - v * sn, rv = v * cs + u * sn;
       b[i] = ru; b[i + half] = rv;
