@@ -1168,10 +1168,11 @@ static int long_k_split(int M, int N, int kb_total) {
   if (tiles * 3 <= 264) return tiles * 8 <= 264 ? 8 : (int)(264 / tiles);
   return tiles * 2 <= 296 ? 2 : 0;
 }
-static void plan(int M, int N, int K, int* swap, int* bn, int* splits, int* kb_per_split,
+// deal_k: false for the projections that write the cache, which only the many-token kernels do.
+static void plan(int M, int N, int K, bool deal_k, int* swap, int* bn, int* splits, int* kb_per_split,
                  int* tiles_p, int* tiles_q) {
   int kb_total = (K + BK - 1) / BK;
-  if (const int want = long_k_split(M, N, kb_total)) {
+  if (const int want = deal_k ? long_k_split(M, N, kb_total) : 0) {
     *swap = 1;
     *bn = 32;
     *tiles_p = (N + BM - 1) / BM;
@@ -1249,7 +1250,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   if (K % 8 != 0 || lda % 8 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15))
     return SGLC_ERR_UNSUPPORTED;
   int swap, bn, splits, per, tp, tq;
-  plan(M, N, K, &swap, &bn, &splits, &per, &tp, &tq);
+  plan(M, N, K, kv == nullptr, &swap, &bn, &splits, &per, &tp, &tq);
   const bool xi = act_is_xielu(act);          // the epilogue's other instantiation
   GemmArgs a;
   a.M = M; a.N = N; a.K = K;
@@ -1358,7 +1359,7 @@ SGLC_API int sglc_gemm_tc_kv(const void* A, const void* W, const float* bias, vo
 // choose for a kernel do reach it.)
 SGLC_API int sglc_gemm_tc_form(int M, int N, int K, int act) {
   int swap, bn, splits, per, tp, tq;
-  plan(M, N, K, &swap, &bn, &splits, &per, &tp, &tq);
+  plan(M, N, K, true, &swap, &bn, &splits, &per, &tp, &tq);
   if (swap) return 0;
   return (bn == 128 && pair_pays(M, N, K, act, tp, tq)) ? 2 : 1;
 }

@@ -267,3 +267,21 @@ def test_gated_norm_at_the_edges_of_what_a_lane_keeps(width):
         want = x.reshape(T, -1) * (1.0 if gate is None else gate)
         # about ten 32-bit roundings a value (2^-24 each) and a sum of `width` squares
         assert float(((y.double() - want).abs() / (want.abs() + 1e-3)).max()) < 1e-5
+
+
+def test_cache_writing_projection_over_a_long_k():
+    """Sizes whose plain product is dealt over K: the projection that writes the cache is still taken, and right."""
+    ops = _ops()
+    M, H, Hkv, D, K, ps = 200, 6, 1, 64, 2304, 16
+    N, n_pages = (H + 2 * Hkv) * D, 13
+    assert ops.gemm_tc_form(M, N, K) == "few"
+    g = torch.Generator().manual_seed(K)
+    a, w = (torch.randn(n, K, generator=g).mul_(s).to(DEV, torch.bfloat16) for n, s in ((M, 1.0), (N, 0.02)))
+    slots = torch.randperm(n_pages * ps, generator=g)[:M].to(DEV, torch.int32)
+    out = torch.zeros(M, N, dtype=torch.bfloat16, device=DEV)
+    cache = torch.zeros(n_pages, 2, Hkv, ps, D, dtype=torch.bfloat16, device=DEV)
+    assert ops.gemm_tc_kv(a, w, None, out, cache, slots, H, Hkv, D)
+    want = a.double() @ w.double().T
+    got = torch.cat([out[:, :H * D].double()] + [cache[slots.long() // ps, i, 0, slots.long() % ps].double() for i in range(2)], 1)
+    # half a unit of bfloat16 a value and the 32-bit sums before it
+    assert float((got - want).abs().max()) < float(want.abs().max()) * 2.0 ** -8
