@@ -4,8 +4,8 @@
 // (16 query rows a warp, a row spread over a quad of threads as in the accumulator of the
 // warp-level MMA) read S, apply the scale, the causal bound and the window, keep the running
 // maximum and sum of an online softmax in 32-bit, write P = exp(S - max) as bfloat16 to shared
-// memory, O_tile = P·V (second MMA, V taken as it lies in the cache: keys by rows), and the
-// threads fold O_tile into their rows' output with the usual rescaling.  Keys and values come
+// memory, O += P·V (second MMA, into sums that stay in tensor memory; V taken as it lies in the cache: keys
+// by rows), the sums scaled down only when a row's maximum has grown by 2^8.  Keys and values come
 // page by page through the block table (one TMA box per page, or 16-byte cp.async where the
 // page size does not divide 128, into the 128-byte swizzle the MMA expects).  Lengths,
 // positions and block tables are read on the device.
@@ -81,7 +81,7 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// 2^x by the special-function unit (inputs here are <= 0 up to rounding; -inf gives 0)
+// 2^x by the special-function unit (inputs here are at most 8; -inf gives 0)
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

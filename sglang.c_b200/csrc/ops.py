@@ -643,7 +643,9 @@ def attention_prefill_tc(q, cache, block_table, q_start, kv_len, out, n_heads, s
     kv_shared: cache is [n_pages, 1, n_kv_heads, page_size, head_dim], rows that are keys and
     values at once.  chunk: a query sees only the keys of its own chunk of so many positions;
     sinks: float32 [n_heads], a score per head that joins the softmax's denominator; gate: float32
-    pre-activations [T, n_heads] or [T, n_heads * head_dim] whose sigmoid multiplies the heads' results."""
+    pre-activations [T, n_heads] or [T, n_heads * head_dim] whose sigmoid multiplies the heads' results.
+    skip_single: requests of one token are left out; their number, where it is known, keeps them out of the launch (True
+    or 1: some, or a number not known)."""
     _need_cuda(q, cache, block_table, q_start, kv_len, out, sinks)
     for t, nm in ((block_table, "block_table"), (q_start, "q_start"), (kv_len, "kv_len")):
         _i32(t, nm)
