@@ -1040,6 +1040,7 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, const CUtensorMap& mo, 
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, XI>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
+    cudaFuncSetAttribute(gemm_tc_kernel<BN, XI>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);    // (clusters of 16)
     // ask for the largest shared-memory split of the SM, so that two blocks fit side by side
     // (one block's epilogue then overlaps the other's main loop)
     cudaFuncSetAttribute(gemm_tc_kernel<BN, XI>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1169,6 +1170,11 @@ static int long_k_split(int M, int N, int kb_total) {
   return tiles * 2 <= 296 ? 2 : 0;
 }
 // deal_k: false for the projections that write the cache, which only the many-token kernels do.
+// Few tokens and features over a long K: clusters of 16 blocks where 8 leave every other SM without one; the weights
+// of a block's share then all find room in its ring, ahead of the wait for the kernel before.  Measured, us with 8
+// and with 16, up to 16 tokens: 768 columns over K 2,048 / 3,072 / 8,192 4.4 / 5.0 / 7.9 and 4.8 / 4.9 / 6.5, 1,024 over
+// 4,096 5.8 and 5.2, 1,152 over 4,608 6.2 and 5.7; 32 tokens, 1,024 over 4,096 6.3 and 9.8 (not all clusters fit at once).
+static bool wide_split(int M, int tiles_p, int kb_total) { return M <= 16 && tiles_p <= 9 && kb_total >= 48; }
 static void plan(int M, int N, int K, bool deal_k, int* swap, int* bn, int* splits, int* kb_per_split,
                  int* tiles_p, int* tiles_q) {
   int kb_total = (K + BK - 1) / BK;
@@ -1187,7 +1193,7 @@ static void plan(int M, int N, int K, bool deal_k, int* swap, int* bn, int* spli
     // enough blocks to put most SMs on the weights, but few enough partial sums that the
     // last block's reduction stays short
     int want = (2 * 148) / (*tiles_p);
-    if (want > 8) want = 8;
+    if (want > 8) want = wide_split(M, *tiles_p, kb_total) ? 16 : 8;
     if (want < 1) want = 1;
     if (want > kb_total) want = kb_total;
     int per = (kb_total + want - 1) / want;

@@ -285,3 +285,17 @@ def test_cache_writing_projection_over_a_long_k():
     got = torch.cat([out[:, :H * D].double()] + [cache[slots.long() // ps, i, 0, slots.long() % ps].double() for i in range(2)], 1)
     # half a unit of bfloat16 a value and the 32-bit sums before it
     assert float((got - want).abs().max()) < float(want.abs().max()) * 2.0 ** -8
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 3072), (16, 1152, 4608), (5, 100, 3080), (16, 768, 8200), (17, 768, 3072), (16, 1160, 3072)])
+def test_few_tokens_over_a_long_k(M, N, K):
+    """K dealt to more than eight blocks, evenly and not, and the sizes just beyond."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(K + M)
+    a, w = (torch.randn(n, K, generator=g).mul_(s).to(DEV, torch.bfloat16) for n, s in ((M, 1.0), (N, 0.02)))
+    bias, x = torch.randn(N, generator=g).to(DEV), torch.randn(M, N, generator=g).to(DEV)
+    want = x.double() + a.double() @ w.double().T + bias.double()
+    ops.gemm_tc(a, w, bias, residual=x)
+    # 32-bit sums of K products: K roundings of 2^-24 of sums that stay below sum |a w|, a random walk of them
+    bound = float((a.double().abs() @ w.double().abs().T).max()) * 2.0 ** -24 * K ** 0.5
+    assert float((x.double() - want).abs().max()) < bound
