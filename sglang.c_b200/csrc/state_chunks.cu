@@ -549,6 +549,26 @@ __device__ __forceinline__ void dc_product(float (&acc)[4][4], const float* a, c
       for (int j = 0; j < 4; j++) acc[i][j] += sum[i][j];
   }
 }
+// The eight terms at the diagonal of a lower triangular a (e0: their first; a warp has the rows e0 .. e0 + 7), each row's
+// up to its own: a zero times a later token's infinity or NaN is not zero, and would reach the tokens before it.
+__device__ __forceinline__ void dc_product_diagonal(float (&acc)[4][4], const float* a, const float* b, int e0, int ty, int tx) {
+  float sum[4][4] = {};
+#pragma unroll
+  for (int e = e0; e < e0 + 8; e++) {
+    const float4 y = ld4(b + e * DC_LD + tx * 4);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (e > ty * 4 + i) continue;
+      const float x = a[(ty * 4 + i) * DC_LD + e];
+      sum[i][0] = fmaf(x, y.x, sum[i][0]); sum[i][1] = fmaf(x, y.y, sum[i][1]);
+      sum[i][2] = fmaf(x, y.z, sum[i][2]); sum[i][3] = fmaf(x, y.w, sum[i][3]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] += sum[i][j];
+}
 __device__ __forceinline__ void dc_write64(float* o, const float (&a)[2][4][4], int ty, int tx) {
 #pragma unroll
   for (int f = 0; f < 2; f++)
@@ -840,7 +860,8 @@ delta_read_kernel(const DcArgs p) {
 #pragma unroll
     for (int e = 0; e < 4; e++) acc[i][e] *= cs[ty * 4 + i];
   __syncthreads();
-  dc_product(acc, ms, us, (tid / 32 + 1) * 8, ty, tx);   // (no row of this warp sees a later token)
+  dc_product(acc, ms, us, tid / 32 * 8, ty, tx);         // (no row of this warp sees a later token)
+  dc_product_diagonal(acc, ms, us, tid / 32 * 8, ty, tx);
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int t = ty * 4 + i, v = z * 64 + tx * 4;

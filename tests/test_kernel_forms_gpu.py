@@ -169,6 +169,32 @@ def test_recurrences_in_chunks(mode, H, G, D, V, rate):
         assert torch.equal(got["chunks"][1][slot], S0[slot])
 
 
+@pytest.mark.parametrize("mode", ["delta", "decay"])
+@pytest.mark.parametrize("at,what", [(5, "v"), (13, "k"), (62, "v"), (71, "q"), (90, "gates")])
+def test_chunks_keep_a_bad_number_from_the_tokens_before_it(mode, at, what):
+    """An infinity or NaN of one token: the tokens before it and the other requests keep their bits, as they do where
+    the recurrence goes token by token."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(at)
+    H, G, D, V, lens = 2, 1, 64, 70, [100, 130]
+    T, R = sum(lens), len(lens)
+    x = {n: torch.randn(T, w, generator=g).to(DEV) for n, w in (("q", G * D), ("k", G * D), ("v", H * V))}
+    x["k"] = torch.nn.functional.normalize(x["k"], dim=-1)
+    x["gates"] = torch.rand(T, 2 * H, generator=g).to(DEV)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)      # noqa: E731
+    kw = dict(gates=x["gates"]) if mode == "delta" else dict(head_decay=torch.rand(H, generator=g).to(DEV))
+    outs = []
+    for bad in (None, float("inf"), float("nan")):
+        if bad is not None:
+            x[what][lens[0] + at] = bad
+        o, S = torch.zeros(T, H * V, device=DEV), torch.zeros(R, H, D, V, device=DEV)
+        ws = torch.empty(ops.delta_chunks_workspace(mode, T, R, H, V), device=DEV)
+        ops.delta_chunks(mode, x["q"], x["k"], x["v"], o, S, i32([0, lens[0], T]), i32([1, 0]), R, H, G, D, V, ws, **kw)
+        outs.append((o, S))
+    for o, S in outs[1:]:
+        assert torch.equal(o[:lens[0] + at], outs[0][0][:lens[0] + at]) and torch.equal(S[1], outs[0][1][1])
+
+
 # -- steps of one token a request ------------------------------------------------------------------------
 @pytest.mark.parametrize("mode,H,G,D,V", [("delta", 4, 2, 64, 64), ("delta", 3, 3, 40, 100), ("delta", 2, 1, 129, 68), ("delta", 2, 2, 256, 4),
                                           ("decay", 3, 3, 64, 64), ("decay", 2, 2, 7, 12), ("decay", 2, 2, 128, 132)])
