@@ -788,7 +788,7 @@ attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const
       l_run = warp_sum(l_run);
       for (int x = 0; x < sa.n_split - 1; x++) {
         const float* rec = recs + x * (D + 2);
-        if (!(rec[1] > 0.0f)) continue;                  // (an empty run of keys)
+        if (rec[1] == 0.0f) continue;                    // (an empty run of keys; a sum that is no number goes into the result)
         const float m_new = fmaxf(m_run, rec[0]), c0 = ex2(m_run - m_new), c1 = ex2(rec[0] - m_new);
         m_run = m_new;
         l_run = l_run * c0 + rec[1] * c1;

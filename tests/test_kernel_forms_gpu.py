@@ -117,6 +117,29 @@ def test_stream_decode_shares_items_between_blocks(T, H, Hkv, D, window):
         assert not fused or torch.equal(cache, c["cache"])
 
 
+@pytest.mark.parametrize("T", [9, 18, 40])
+def test_decode_attention_keeps_a_bad_key_in_every_share(T):
+    """A key that is no number, near the front of a request's keys, in the middle or near their end: the request's result
+    is none either, whichever block has that key; the other requests' results keep their bits."""
+    ops = _ops()
+    H, D, ps = 12, 64, 16
+    lens = [650 + r for r in range(T)]
+    c = _paged_case(lens, [1] * T, H, H, D, ps, torch.bfloat16, seed=T)
+
+    def run(cache):
+        out = torch.zeros(T, H * D, dtype=torch.bfloat16, device=DEV)
+        ops.attention_decode(c["q"], cache, c["bt"], None, c["positions"], out, H, 0.1, None, max(lens), variant="stream", n_tokens=T)
+        return out
+
+    clean = run(c["cache"])
+    for key in (3, 200, 340, 500, 640):
+        cache = c["cache"].clone()
+        cache[int(c["bt"][1, key // ps]), 0, :, key % ps] = float("nan")
+        out = run(cache)
+        assert bool(torch.isnan(out[1]).all()), key
+        assert torch.equal(torch.cat([out[:1], out[2:]]), torch.cat([clean[:1], clean[2:]])), key
+
+
 # -- recurrences in chunks ----------------------------------------------------------------------------
 def _walk(mode, q, k, v, gates, decay, H, G, D, V, S):
     n = q.shape[0]
