@@ -13,6 +13,8 @@
 // memory (a block of eight consecutive tokens of a prompt portion reads them once instead of
 // eight times: the reference's kernel, one block per token, reads them per token).  This is the
 // kernel of the 32-bit path and the general fallback of the bfloat16 path.
+#include <type_traits>
+
 #include "common.cuh"
 
 SGLC_DEFINE_ERROR_STRING()
@@ -397,27 +399,38 @@ attention_f32_portion_kernel(const F32Args a) {
 #pragma unroll
           for (int n = 0; n < NA; n++)
             if (on[i]) acc[i][n] *= corr[i];
+        // (A tile that some of the warp's tokens see in part: their sums leave the other keys out, for the weight zero times an
+        // infinite value is not zero.)
+        auto add_values = [&](auto whole) {
 #pragma unroll 2
-        for (int j = 0; j < 32; j += 4) {
-          float4 p4[FP_Q];
+          for (int j = 0; j < 32; j += 4) {
+            float4 p4[FP_Q];
 #pragma unroll
-          for (int i = 0; i < FP_Q; i++) p4[i] = *reinterpret_cast<const float4*>(pv + i * 32 + j);
+            for (int i = 0; i < FP_Q; i++) p4[i] = *reinterpret_cast<const float4*>(pv + i * 32 + j);
 #pragma unroll
-          for (int n = 0; n < NA; n++) {
-            const int d = min(lane + 32 * n, D - 1);                    // (lanes beyond the head size: not stored)
-            const float v0 = vs[j * D + d], v1 = vs[(j + 1) * D + d], v2 = vs[(j + 2) * D + d], v3 = vs[(j + 3) * D + d];
+            for (int n = 0; n < NA; n++) {
+              const int d = min(lane + 32 * n, D - 1);                  // (lanes beyond the head size: not stored)
+              const float v0 = vs[j * D + d], v1 = vs[(j + 1) * D + d], v2 = vs[(j + 2) * D + d], v3 = vs[(j + 3) * D + d];
 #pragma unroll
-            for (int i = 0; i < FP_Q; i++)
-              if (on[i]) {
-                float x = acc[i][n];
-                x = fmaf(p4[i].x, v0, x);
-                x = fmaf(p4[i].y, v1, x);
-                x = fmaf(p4[i].z, v2, x);
-                x = fmaf(p4[i].w, v3, x);
-                acc[i][n] = x;
-              }
+              for (int i = 0; i < FP_Q; i++)
+                if (on[i]) {
+                  const int key4 = key0 + j;
+                  auto sees = [&](int e) { return decltype(whole)::value || (key4 + e >= my_lo[i] && key4 + e <= my_pos[i]); };
+                  float x = acc[i][n];
+                  if (sees(0)) x = fmaf(p4[i].x, v0, x);
+                  if (sees(1)) x = fmaf(p4[i].y, v1, x);
+                  if (sees(2)) x = fmaf(p4[i].z, v2, x);
+                  if (sees(3)) x = fmaf(p4[i].w, v3, x);
+                  acc[i][n] = x;
+                }
+            }
           }
-        }
+        };
+        bool whole = true;
+#pragma unroll
+        for (int i = 0; i < FP_Q; i++) whole = whole && (!on[i] || (key0 >= my_lo[i] && key0 + 31 <= my_pos[i]));
+        if (whole) add_values(std::true_type{});
+        else add_values(std::false_type{});
         __syncwarp();
       }
       __syncthreads();                                // everybody is done with tile kt: the next but one may come

@@ -62,6 +62,28 @@ def test_attention_f32_has_the_same_bits_in_every_cut(H, Hkv, D, ps, window):
         assert torch.equal(out, whole[pick]), longest
 
 
+@pytest.mark.parametrize("D,at", [(64, 9), (64, 61), (128, 40)])
+def test_attention_f32_keeps_a_bad_value_from_the_tokens_before_it(D, at):
+    """A value that is infinite or no number reaches the tokens that see it, and no other token of its tile or block."""
+    ops = _ops()
+    H, ps, lens, q_lens = 8, 16, [70, 640], [70, 600]
+    c = _paged_case(lens, q_lens, H, H, D, ps, torch.float32, seed=at)
+    T = sum(q_lens)
+
+    def run():
+        out = torch.zeros(T, H * D, device=DEV)
+        ops.attention_simt(c["q"], c["cache"], c["bt"], c["token_req"], c["positions"], out, H, 0.1, None, 640, max_q_len=600)
+        return out
+
+    clean = run()
+    for bad in (float("inf"), float("nan")):
+        key = 40 + at                                   # (the second request's token `at`: its first token is at position 40)
+        c["cache"][int(c["bt"][1, key // ps]), 1, :, key % ps] = bad
+        out = run()
+        assert torch.equal(out[:70 + at], clean[:70 + at])
+        assert not bool(torch.isfinite(out[70 + at:]).any())
+
+
 # -- tensor-core prompt attention ---------------------------------------------------------------------
 @pytest.mark.parametrize("D,window,grow", [(64, None, 3.0), (64, 150, 3.0), (128, None, 3.0), (64, None, 0.0), (64, None, -3.0)])
 def test_prompt_attention_follows_a_growing_maximum(D, window, grow):
