@@ -64,17 +64,20 @@ def _stacked(store, refs):
     return store.computed("+".join(r.name for r in refs), lambda: torch.cat([r.tensor.float() for r in refs], 0))
 
 
-def _chunk_bytes(mode, H, D, V):
+def _chunk_bytes(rt, mode, H, D, V):
     """Bytes of workspace a token needs where a recurrence goes in chunks."""
-    if D > ops.DELTA_CHUNKS_MAX_DIM:
+    if D > ops.DELTA_CHUNKS_MAX_DIM or rt.dtype == "float32":
         return 0
     return 4 * ops.delta_chunks_workspace(mode, ops.STATE_CHUNK, 1, H, V) // ops.STATE_CHUNK
 
 
 def _matrix_state(ctx, mode, q, k, v, out, state, H, G, D, V, **kw):
     """The recurrence over the step's tokens: one token a request in a pass over the states, long portions in chunks
-    side by side, else token by token."""
-    if ctx.max_q_len == 1 and ops.delta_step_fits(state, D, V):
+    side by side, else token by token.  In the 32-bit path always token by token: each form has an order of additions of
+    its own, and there a request's bits must not depend on what else is in its step."""
+    if ctx.rt.dtype == "float32":
+        ops.matrix_state(mode, q, k, v, out, state, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, **kw)
+    elif ctx.max_q_len == 1 and ops.delta_step_fits(state, D, V):
         ops.delta_step(mode, q, k, v, out, state, ctx.state_slots, H, G, D, V, **kw)
     elif ops.delta_chunks_pay(mode, out.shape[0], ctx.R, ctx.max_q_len, H, D):
         mark = ctx.mark()
@@ -141,7 +144,7 @@ class GatedDeltaRule(Part):
         H, G, D, V = p["n_heads"], p["n_qk_heads"], p["dim"], p["v_dim"]
         act = 4 if self.rt.dtype == "float32" else 2
         return 4 * (2 * G * D + 2 * H * V + 2 * H + 8) + 4 * (2 * G * D + H * V) + 8 * H + 4 * H * V + act * H * V + 2048 \
-            + _chunk_bytes("delta", H, D, V)
+            + _chunk_bytes(self.rt, "delta", H, D, V)
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params
@@ -198,7 +201,7 @@ class LinearDecayAttention(Part):
         p = self.params
         H, D, V = p["n_heads"], p["dim"], p["v_dim"]
         act = 4 if self.rt.dtype == "float32" else 2
-        return 4 * (2 * H * D + 2 * H * V) + 4 * H * V + act * H * V + 1024 + _chunk_bytes("decay", H, D, V)
+        return 4 * (2 * H * D + 2 * H * V) + 4 * H * V + act * H * V + 1024 + _chunk_bytes(self.rt, "decay", H, D, V)
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params

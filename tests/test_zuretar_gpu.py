@@ -432,7 +432,35 @@ def test_mixed_results_do_not_depend_on_the_batch_in_32_bit(dirs, tmp_path):
     alone, _ = run_trace(d, "float32", "A", traces.whole(reqs), tmp_path)
     for rid in reqs:
         for p in alone[rid]:
-            assert np.abs(mixed[rid][p] - alone[rid][p]).max() < 2e-5
+            assert np.array_equal(mixed[rid][p], alone[rid][p])
+
+
+RECURRENT = {"architecture": "Zuretar", "vocab": 300, "width": 64, "norm": {"eps": 1e-6}, "layers": [
+    {"type": "delta", "mixer": {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 64, "conv": 4}, "mlp": {"kind": "dense", "ff": 96}},
+    {"type": "delta", "mixer": {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 32, "conv": 3}, "mlp": {"kind": "dense", "ff": 96}}]}
+
+
+@pytest.mark.parametrize("name", ["C", "R"])
+def test_32_bit_recurrences_have_one_order_of_additions(dirs, tmp_path, name):
+    """Long prompts whole, in portions, beside others and token by token: the same bits, in a model of every kind of layer
+    and in one of delta layers with heads of 64."""
+    import zuretar_models
+    if name == "R":
+        zuretar_models.ZUR[name], zuretar_models.PAGE[name] = RECURRENT, 16
+    try:
+        d = dirs(name)
+        V = zuretar_models.ZUR[name]["vocab"]
+        reqs = {f"q{i}": traces.random_tokens(500 + i, n, V) for i, n in enumerate([300, 33, 200])}
+        prompt_len = {rid: len(t) - 5 for rid, t in reqs.items()}
+        alone, _ = run_trace(d, "float32", name, traces.whole(reqs), tmp_path)
+        for steps in (traces.mixed(reqs, prompt_len, seed=9, sizes=(160, 3, 64, 90)), traces.tail_decoded(reqs, 12), traces.portions(reqs)):
+            got, _ = run_trace(d, "float32", name, steps, tmp_path)
+            for rid in reqs:
+                for p in alone[rid]:
+                    assert np.array_equal(got[rid][p], alone[rid][p]), (rid, p)
+    finally:
+        if name == "R":
+            del zuretar_models.ZUR[name], zuretar_models.PAGE[name]
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
