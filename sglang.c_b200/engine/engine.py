@@ -442,7 +442,7 @@ class Engine:
     def _graph_key(self, ctx):
         bound = self.model.graph_bound(ctx)
         return (ctx.T, ctx.R, ctx.n_want, (ctx.max_q_len + 127) // 128 if ctx.max_q_len > 1 else 0,
-                bound, ctx.n_decode, ctx.decode_ordered), bound
+                bound, ctx.n_decode, ctx.decode_ordered, self.model.launch_forms(ctx)), bound
 
     def _graph_lookup(self, ctx):
         """Replay the graph of this step's shape if there is one (and its output buffer still
@@ -462,7 +462,8 @@ class Engine:
     def _forward_graphed(self, ctx):
         """Replay a CUDA graph when this step's launch shapes have been seen before.  The
         shapes depend on the number of tokens, requests and wanted rows, on the longest
-        portion (in 128-query tiles) and on an upper bound of the context length (see _graph_key).  Everything else a step
+        portion (in 128-query tiles; finer where a mixer says so) and on an upper bound of the context length (see
+        _graph_key).  Everything else a step
         varies in lies in device arrays at fixed addresses.  A shape runs eagerly the first
         time it is seen, is captured the second time, and replayed afterwards; the least
         recently used graphs are dropped beyond `max_graphs`.  (A step of steady decoding, which

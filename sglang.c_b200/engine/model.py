@@ -3,6 +3,7 @@ given their params, and bound to the tensors the plan names.  The forward pass
 walks the plan's running order; nothing here knows an architecture."""
 import torch
 
+from ..parts.base import Part
 from ..parts.registry import get_part
 from ..weights.loader import DeviceStore, load_checked
 
@@ -88,6 +89,8 @@ class Model:
         for layer in self.layers:
             parts += [layer.block] + list(layer.parts.values())
         self.graph_safe = all(getattr(p, "graph_safe", True) for p in parts)
+        self._formed = [m for m in (layer.the_mixer for layer in self.layers)
+                        if isinstance(m, Part) and type(m).launch_form is not Part.launch_form]
         self.largest_layer_matrix = 0     # elements of the largest matrix a layer holds (set by load)
 
     def load(self, model_dir):
@@ -132,6 +135,11 @@ class Model:
         if asked:
             bound = max(asked)
         return min(bound, self.plan.max_positions)
+
+    def launch_forms(self, ctx):
+        """What the mixers' launches follow beyond the rest of a step graph's key (see Part.launch_form); steps of single
+        tokens have one form each."""
+        return tuple(m.launch_form(ctx) for m in self._formed) if ctx.max_q_len > 1 else ()
 
     def forward(self, ctx, cache, logits_out):
         """Run the step's tokens through every call of the running order; write

@@ -617,6 +617,9 @@ class SideBySideMixers(Part):
     def workspace_per_token(self):
         return 4 * self.params["size"] + max(m.workspace_per_token() for m in self.sides)
 
+    def launch_form(self, ctx):
+        return tuple(m.launch_form(ctx) for m in self.sides)
+
     def graph_bound(self, ctx):
         asked = [b for b in (m.graph_bound(ctx) for m in self.sides) if b is not None]
         return max(asked) if asked else None

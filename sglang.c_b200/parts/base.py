@@ -78,3 +78,9 @@ class Part:
         """Mixers only: an upper bound of the context length for this step's launches, if the
         mixer's kernels want another than the next power of two (None: no wish)."""
         return None
+
+    def launch_form(self, ctx):
+        """Mixers only: what this step's launches follow besides its numbers of tokens, requests and single tokens, its
+        longest portion in runs of 128 tokens and its context bound: a form chosen, or a grid sized, by something finer.  Any
+        value that compares (None: nothing).  A captured graph serves the steps that agree in it."""
+        return None

@@ -71,17 +71,26 @@ def _chunk_bytes(rt, mode, H, D, V):
     return 4 * ops.delta_chunks_workspace(mode, ops.STATE_CHUNK, 1, H, V) // ops.STATE_CHUNK
 
 
-def _matrix_state(ctx, mode, q, k, v, out, state, H, G, D, V, **kw):
-    """The recurrence over the step's tokens: one token a request in a pass over the states, long portions in chunks
-    side by side, else token by token.  In the 32-bit path always token by token: each form has an order of additions of
-    its own, and there a request's bits must not depend on what else is in its step."""
+def _form(ctx, T, mode, H, D):
+    """How a step's recurrence is worked on: "step" (one token a request, in a pass over the states), "chunks" (long
+    portions, side by side) or "walk" (token by token).  In the 32-bit path always the walk: each form has an order
+    of additions of its own, and there a request's bits must not depend on what else is in its step."""
     if ctx.rt.dtype == "float32":
-        ops.matrix_state(mode, q, k, v, out, state, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, **kw)
-    elif ctx.max_q_len == 1 and ops.delta_step_fits(state, D, V):
+        return "walk"
+    if ctx.max_q_len == 1:
+        return "step"
+    return "chunks" if ops.delta_chunks_pay(mode, T, ctx.R, ctx.max_q_len, H, D) else "walk"
+
+
+def _matrix_state(ctx, mode, q, k, v, out, state, H, G, D, V, **kw):
+    """The recurrence over the step's tokens."""
+    T = out.shape[0]
+    form = _form(ctx, T, mode, H, D)
+    if form == "step" and ops.delta_step_fits(state, D, V):
         ops.delta_step(mode, q, k, v, out, state, ctx.state_slots, H, G, D, V, **kw)
-    elif ops.delta_chunks_pay(mode, out.shape[0], ctx.R, ctx.max_q_len, H, D):
+    elif form == "chunks":
         mark = ctx.mark()
-        ws = ctx.alloc((ops.delta_chunks_workspace(mode, out.shape[0], ctx.R, H, V),), torch.float32)
+        ws = ctx.alloc((ops.delta_chunks_workspace(mode, T, ctx.R, H, V),), torch.float32)
         ops.delta_chunks(mode, q, k, v, out, state, ctx.q_start, ctx.state_slots, ctx.R, H, G, D, V, ws, **kw)
         ctx.release(mark)
     else:
@@ -146,6 +155,9 @@ class GatedDeltaRule(Part):
         return 4 * (2 * G * D + 2 * H * V + 2 * H + 8) + 4 * (2 * G * D + H * V) + 8 * H + 4 * H * V + act * H * V + 2048 \
             + _chunk_bytes(self.rt, "delta", H, D, V)
 
+    def launch_form(self, ctx):
+        return _form(ctx, ctx.T, "delta", self.params["n_heads"], self.params["dim"])
+
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params
         H, G, D, V = p["n_heads"], p["n_qk_heads"], p["dim"], p["v_dim"]
@@ -202,6 +214,9 @@ class LinearDecayAttention(Part):
         H, D, V = p["n_heads"], p["dim"], p["v_dim"]
         act = 4 if self.rt.dtype == "float32" else 2
         return 4 * (2 * H * D + 2 * H * V) + 4 * H * V + act * H * V + 1024 + _chunk_bytes(self.rt, "decay", H, D, V)
+
+    def launch_form(self, ctx):
+        return _form(ctx, ctx.T, "decay", self.params["n_heads"], self.params["dim"])
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params

@@ -485,6 +485,43 @@ def test_long_decoding_replays_graphs(dirs, tmp_path, dtype):
     assert eng.graph_replays > 150, "steady decoding did not replay captured graphs"
 
 
+@pytest.mark.parametrize("first,second", [((134, 133, 133), (192, 104, 104)), ((204, 100, 98, 98), (129, 129, 129, 113)),
+                                          ((90, 71, 70), (127, 40, 64))])
+def test_replayed_prompts_have_the_eager_pass_bits(dirs, tmp_path, first, second):
+    """Two layouts of prompts, as many tokens and requests and longest portions in one run of 128 tokens, one of them
+    better off in chunks than the other: a step that replays has the bits of the same step run eagerly, whatever was
+    captured before it."""
+    import zuretar_models
+    from sglang_c_b200.engine import Engine, StepEntry
+    assert sum(first) == sum(second)
+    zuretar_models.ZUR["G"] = zuretar_models.ZUR_G
+    try:
+        d = dirs("G", "bfloat16")
+    finally:
+        del zuretar_models.ZUR["G"]
+
+    def run(graphs, layouts):
+        eng = Engine.from_dir(d, dtype="bfloat16", page_size=16, n_pages=64, max_requests=8, max_step_tokens=1024)
+        eng.use_graphs = graphs
+        outs = []
+        for n, lens in enumerate(layouts):
+            for i in range(len(lens)):
+                eng.add_request(f"{n}.{i}")
+            outs.append(eng.step([StepEntry(f"{n}.{i}", traces.random_tokens(31 + i, k, 300), [k - 1])
+                                  for i, k in enumerate(lens)]).clone())
+            for i in range(len(lens)):
+                eng.end_request(f"{n}.{i}")
+        return outs, eng.graph_replays
+
+    eager, _ = run(False, (first, second))
+    for order in ((first, second), (second, first)):
+        want = eager if order[0] == first else eager[::-1]
+        (a, b, c, again, e), replays = run(True, (order[0], order[0], order[0], order[1], order[1]))
+        assert replays >= 2
+        for got, ref in ((a, want[0]), (b, want[0]), (c, want[0]), (again, want[1]), (e, want[1])):
+            assert torch.equal(got, ref)
+
+
 def check_greedy(model_dir, prompt, got, tie):
     cfg, w = P.read_model_dir(model_dir)
     seq = list(prompt)

@@ -67,6 +67,13 @@ ZUR_C = {"architecture": "Zuretar", "vocab": 101, "width": 50, "norm": {"eps": 1
     _delta(3, 1, 7, 5, 1, _moe(5, 5, 11)),
     _parallel(_left(3, 3, 10, 6, 0.4, 5, 6, 100.0, (2.0, 16, 3.0, 0.5)), _right(1, 9, 3, (0.8,)), _moe(6, 2, 9, (3, 3))),
     _delta(6, 3, 33, 35, 5, _dense(70))]}
+# heads of 64, whose recurrences have a form in chunks
+ZUR_G = {"architecture": "Zuretar", "vocab": 300, "width": 128, "norm": {"eps": 1e-6}, "layers": [
+    {"type": "delta", "mixer": {"heads": 12, "kv_heads": 6, "dim": 64, "vdim": 64, "conv": 4}, "mlp": {"kind": "dense", "ff": 96}},
+    {"type": "parallel", "mixer": {"left": {"heads": 4, "kv_heads": 1, "dim": 64, "vdim": 64, "scale": 0.125, "mask": {"size": 256},
+                                            "rot": {"base": 10000.0, "dims": 64}},
+                                   "right": {"heads": 4, "dim": 64, "vdim": 64, "decay": [0.9, 0.99, 0.95, 0.999]}},
+     "mlp": {"kind": "dense", "ff": 96}}]}
 ZUR = {"A": ZUR_A, "B": ZUR_B, "C": ZUR_C}
 PAGE = {"A": 16, "B": 16, "C": 8}
 
