@@ -1747,6 +1747,7 @@ def talk_attention(q, cache, block_table, token_req, positions, slopes, talk, ga
 
 
 TALK_TILES_MAX_HEADS = 16
+TALK_TILE_ROWS = 16         # queries of a tile (attention_talk.cu: TT_ROWS)
 _TALK_UNSUPPORTED = -2
 
 

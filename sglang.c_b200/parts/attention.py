@@ -348,6 +348,12 @@ class TalkingHeadsAttention(Part):
         act = 4 if self.rt.dtype == "float32" else 2
         return 4 * ((2 * H + G) * D + 8) + 4 * H * D + act * H * D + 1024
 
+    def launch_form(self, ctx):
+        # tiles of queries (bfloat16): the grid has as many as the longest portion, their buffers the rows one can have
+        from ..csrc import ops
+        rows = ops.TALK_TILE_ROWS
+        return None if self.rt.dtype != "bfloat16" else ctx.max_q_len if ctx.max_q_len < rows else -(-ctx.max_q_len // rows) * rows
+
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         from ..csrc import ops
         p = self.params

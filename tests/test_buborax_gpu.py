@@ -387,6 +387,32 @@ def test_mixed_results_do_not_depend_on_the_batch_in_32_bit(dirs, tmp_path):
             assert np.abs(mixed[rid][p] - alone[rid][p]).max() < 2e-5
 
 
+def test_replayed_prompts_of_other_lengths(dirs):
+    """Two prompts as long as each other, captured and replayed, then as many tokens in one long prompt and a short one:
+    every query of the long one has the eager pass's bits."""
+    from sglang_c_b200.engine import Engine, StepEntry
+
+    def run(*layouts):
+        eng = Engine.from_dir(dirs("B", "bfloat16"), dtype="bfloat16", page_size=PAGE["B"], n_pages=64, max_requests=4, max_step_tokens=256)
+        outs = []
+        for n, lens in enumerate(layouts):
+            ids = [f"{n}.{i}" for i in range(len(lens))]
+            for q in ids:
+                eng.add_request(q)
+            outs.append(eng.step([StepEntry(q, traces.random_tokens(7 + i, k, BUB["B"]["vocab"]), list(range(k)))
+                                  for i, (q, k) in enumerate(zip(ids, lens))]).clone())
+            for q in ids:
+                eng.end_request(q)
+        return outs, eng.graph_replays
+
+    even, uneven = (55, 55), (100, 10)
+    first = [run(lens)[0][0] for lens in (even, uneven)]          # (a shape's first step runs eagerly)
+    got, replays = run(even, even, even, uneven, uneven, uneven)
+    assert replays >= 3
+    for out, ref in zip(got, [first[0]] * 3 + [first[1]] * 3):
+        assert torch.equal(out, ref)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_long_decoding_replays_graphs(dirs, tmp_path, dtype):
     """Two requests decoded for 240 steps: windows pass over decoded tokens, pages behind them return."""

@@ -3,6 +3,7 @@ from types import SimpleNamespace
 
 import pytest
 
+from buborax_models import BUB_B
 from sglang_c_b200.config import resolve_architecture
 from sglang_c_b200.engine.engine import Engine
 from sglang_c_b200.engine.model import Model
@@ -25,3 +26,12 @@ def test_a_recurrence_in_chunks_has_a_graph_of_its_own(walk, chunks):
     assert _key(ZUR_G, walk) != _key(ZUR_G, chunks)
     assert _key(ZUR_G, walk, "float32") == _key(ZUR_G, chunks, "float32")          # (always token by token there)
     assert _key(ZUR_G, walk) == _key(ZUR_G, walk[::-1])
+
+
+@pytest.mark.parametrize("few,many", [((55, 55), (100, 10)), ((5, 5), (8, 2)), ((16, 16), (17, 15)), ((130, 130), (145, 115))])
+def test_tiles_of_queries_are_part_of_the_key(few, many):
+    """Talking-heads attention sizes its grid (and a tile's buffers) by the longest portion: a graph captured for fewer
+    tiles would leave the last queries of a longer portion undone."""
+    assert _key(BUB_B, few) != _key(BUB_B, many)
+    assert _key(BUB_B, few, "float32") == _key(BUB_B, many, "float32")             # (a block a token there)
+    assert _key(BUB_B, (100, 100)) == _key(BUB_B, (104, 96))                       # (seven tiles each)
