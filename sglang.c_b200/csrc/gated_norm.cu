@@ -19,16 +19,55 @@ SGLC_DEFINE_ERROR_STRING()
 
 enum { GN_SILU = 0, GN_SIGMOID = 1, GN_NONE = 2 };   // GN_NONE: no gate at all (gate may be null)
 
-// KEEP: rows of up to 32 KEEP columns, all of whose values, gates and gains are asked for together and kept in
-// registers (the gains ahead of the wait for the kernel before); 0: any width, in two passes.  The same
-// arithmetic in the same order.  Rows of 64, in a step's chain of launches: 96 rows 3.6 -> 1.5 us, 24,576 rows
-// 11.7 -> 7.8.  (o, gate and m_run are not __restrict__: loads of what the kernel before writes might move ahead of the wait.)
+// Rows of any width, in two passes over them.
+template <typename TO>
+__global__ void __launch_bounds__(128)
+gated_norm_kernel(const float* __restrict__ o, long long o_stride, const float* __restrict__ gate,
+                  long long gate_stride, const float* __restrict__ gain, TO* __restrict__ y, long long y_stride,
+                  long long n_rows, int groups, int width, float eps, int act, int o_pitch, int gain_rows,
+                  const float* __restrict__ m_run, long long m_stride) {
+  pdl_launch_dependents();
+  const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  pdl_wait();
+  if (row >= n_rows) return;
+  const long long t = row / groups;
+  const int c0 = (int)(row % groups) * width;
+  const float* op = o + t * o_stride + (row % groups) * o_pitch;
+  const float* gp = act == GN_NONE ? nullptr : gate + t * gate_stride + c0;
+  if (gain_rows) gain += c0;
+  float pre = 1.0f;
+  if (m_run) pre = 1.0f / (fmaxf(fabsf(op[width]), expf(-m_run[t * m_stride + row % groups])) + 1e-6f);
+  float ss = 0.0f;
+  for (int d = lane; d < width; d += 32) {
+    const float v = op[d] * pre;
+    ss = fmaf(v, v, ss);
+  }
+  ss = warp_sum(ss);
+  const float inv = pre / sqrtf(ss / (float)width + eps);
+  TO* yp = y + t * y_stride + c0;
+  for (int d = lane; d < width; d += 32) {
+    if (act == GN_NONE) {
+      yp[d] = from_f32<TO>(op[d] * inv * gain[d]);
+      continue;
+    }
+    const float g = gp[d];
+    const float s = 1.0f / (1.0f + expf(-g));
+    yp[d] = from_f32<TO>(op[d] * inv * gain[d] * (act == GN_SILU ? g * s : s));
+  }
+}
+
+// Rows of up to 32 KEEP columns: all of a row's values, gates and gains are asked for together and kept in registers
+// (the gains ahead of the wait for the kernel before).  The same arithmetic in the same order.  Rows of 64, in a step's chain
+// of launches: 96 rows 3.6 -> 1.5 us, 24,576 rows 11.7 -> 7.8.  (o, gate and m_run are not __restrict__: loads of
+// what the kernel before writes might move ahead of the wait.  In the kernel above they are: without it its loads go one
+// behind the other, one row of 2,048 columns 26.2 us instead of 18.8.)
 template <typename TO, int KEEP>
 __global__ void __launch_bounds__(128)
-gated_norm_kernel(const float* o, long long o_stride, const float* gate, long long gate_stride,
-                  const float* __restrict__ gain, TO* __restrict__ y, long long y_stride, long long n_rows,
-                  int groups, int width, float eps, int act, int o_pitch, int gain_rows,
-                  const float* m_run, long long m_stride) {
+gated_norm_kept_kernel(const float* o, long long o_stride, const float* gate, long long gate_stride,
+                       const float* __restrict__ gain, TO* __restrict__ y, long long y_stride, long long n_rows,
+                       int groups, int width, float eps, int act, int o_pitch, int gain_rows,
+                       const float* m_run, long long m_stride) {
   pdl_launch_dependents();
   const long long row = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -39,7 +78,7 @@ gated_norm_kernel(const float* o, long long o_stride, const float* gate, long lo
   const float* gp = act == GN_NONE ? nullptr : gate + t * gate_stride + c0;
   if (gain_rows) gain += c0;
   TO* yp = y + t * y_stride + c0;
-  float kept[KEEP > 0 ? KEEP : 1], gated[KEEP > 0 ? KEEP : 1], gains[KEEP > 0 ? KEEP : 1];
+  float kept[KEEP], gated[KEEP], gains[KEEP];
 #pragma unroll
   for (int n = 0; n < KEEP; n++) gains[n] = lane + 32 * n < width ? gain[lane + 32 * n] : 0.0f;
   pdl_wait();
@@ -51,39 +90,20 @@ gated_norm_kernel(const float* o, long long o_stride, const float* gate, long lo
   float pre = 1.0f;
   if (m_run) pre = 1.0f / (fmaxf(fabsf(op[width]), expf(-m_run[t * m_stride + row % groups])) + 1e-6f);
   float ss = 0.0f;
-  if constexpr (KEEP > 0) {
 #pragma unroll
-    for (int n = 0; n < KEEP; n++)
-      if (lane + 32 * n < width) {
-        const float v = kept[n] * pre;
-        ss = fmaf(v, v, ss);
-      }
-  } else {
-    for (int d = lane; d < width; d += 32) {
-      const float v = op[d] * pre;
+  for (int n = 0; n < KEEP; n++)
+    if (lane + 32 * n < width) {
+      const float v = kept[n] * pre;
       ss = fmaf(v, v, ss);
     }
-  }
   ss = warp_sum(ss);
   const float inv = pre / sqrtf(ss / (float)width + eps);
-  if constexpr (KEEP > 0) {
 #pragma unroll
-    for (int n = 0; n < KEEP; n++) {
-      if (lane + 32 * n >= width) continue;
-      const float x = kept[n] * inv * gains[n], g = gated[n];
-      const float s = 1.0f / (1.0f + expf(-g));
-      yp[lane + 32 * n] = from_f32<TO>(act == GN_NONE ? x : x * (act == GN_SILU ? g * s : s));
-    }
-    return;
-  }
-  for (int d = lane; d < width; d += 32) {
-    if (act == GN_NONE) {
-      yp[d] = from_f32<TO>(op[d] * inv * gain[d]);
-      continue;
-    }
-    const float g = gp[d];
+  for (int n = 0; n < KEEP; n++) {
+    if (lane + 32 * n >= width) continue;
+    const float x = kept[n] * inv * gains[n], g = gated[n];
     const float s = 1.0f / (1.0f + expf(-g));
-    yp[d] = from_f32<TO>(op[d] * inv * gain[d] * (act == GN_SILU ? g * s : s));
+    yp[lane + 32 * n] = from_f32<TO>(act == GN_NONE ? x : x * (act == GN_SILU ? g * s : s));
   }
 }
 
@@ -99,20 +119,18 @@ SGLC_API int sglc_gated_norm_ext(const float* o, long long o_stride, const float
   if (o_pitch < width + (m_run ? 1 : 0)) return SGLC_ERR_ARGUMENT;
   const long long n_rows = (long long)T * groups;
   const dim3 grid((unsigned)((n_rows + 3) / 4));
-#define GO(TO, KEEP)                                                                                             \
-  return sglc_launch(gated_norm_kernel<TO, KEEP>, grid, dim3(128), 0, stream, 1, true, o, o_stride, gate, gate_stride, \
-                     gain, (TO*)y, y_stride, n_rows, groups, width, eps, act, o_pitch, gain_rows, m_run, m_stride)
-  if (y_dtype == SGLC_F32) {
-    if (width <= 64) GO(float, 2);
-    if (width <= 256) GO(float, 8);
-    GO(float, 0);
-  }
-  if (y_dtype == SGLC_BF16) {
-    if (width <= 64) GO(__nv_bfloat16, 2);
-    if (width <= 256) GO(__nv_bfloat16, 8);
-    GO(__nv_bfloat16, 0);
-  }
-#undef GO
+  auto go = [&](auto* kernel, auto* to) {
+    return sglc_launch(kernel, grid, dim3(128), 0, stream, 1, true, o, o_stride, gate, gate_stride, gain, to, y_stride, n_rows,
+                       groups, width, eps, act, o_pitch, gain_rows, m_run, m_stride);
+  };
+  if (y_dtype == SGLC_F32)
+    return go(width <= 64 ? gated_norm_kept_kernel<float, 2> : width <= 256 ? gated_norm_kept_kernel<float, 8> : gated_norm_kernel<float>,
+              (float*)y);
+  if (y_dtype == SGLC_BF16)
+    return go(width <= 64    ? gated_norm_kept_kernel<__nv_bfloat16, 2>
+              : width <= 256 ? gated_norm_kept_kernel<__nv_bfloat16, 8>
+                             : gated_norm_kernel<__nv_bfloat16>,
+              (__nv_bfloat16*)y);
   return SGLC_ERR_ARGUMENT;
 }
 
