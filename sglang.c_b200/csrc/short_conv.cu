@@ -180,7 +180,7 @@ short_conv_run_kernel(ConvArgs p) {
             acc = fmaf(taps[e][j], v, acc);
           }
         }
-        a[e] = silu_f32(acc);
+        a[e] = silu_f32(lane + 32 * e < sg.width ? acc : 1.0f);      // (a division of zero would be a slow one)
         if (lane + 32 * e < sg.width) ss = fmaf(a[e], a[e], ss);
       }
       float f = 1.0f;
@@ -241,7 +241,7 @@ short_conv_step_kernel(ConvArgs p) {
       float acc = 0.0f;
 #pragma unroll
       for (int j = 0; j < K; j++) acc = fmaf(taps[e][j], v[e][j], acc);
-      a[e] = silu_f32(acc);
+      a[e] = silu_f32(lane + 32 * e < sg.width ? acc : 1.0f);
       if (lane + 32 * e < sg.width) ss = fmaf(a[e], a[e], ss);
     }
     float f = 1.0f;
@@ -286,6 +286,17 @@ short_conv_tail_kernel(ConvArgs p) {
   }
 }
 
+// Whether a step with portions goes by runs of CONV_RUN tokens.  There a warp walks its tokens one behind the other, and
+// one near its portion's start looks its tail up: where the general kernel has few blocks, or portions are short, its
+// spread is worth more.  By its blocks times taps, general kernel and runs: one portion of 200 tokens of 1,536 channels
+// (5,600) 7.2 and 8.5 us, of 512 (14,336) 11.6 and 9.3; 384 of 1,024 channels in rows of 32, three taps (10,368) 8.2 and
+// 7.3; 1,024 of 160 in rows of 16 (12,288) 6.5 and 7.5, 1,536 (18,432) 8.5 and 8.2; 100 portions of 5 of 1,024 (13,500)
+// 9.6 and 11.6, 31 single tokens beside 481 (14,336) 12.1 and 14.3, 100 beside 1,000 (17,600; 30,800) 12.8 and 13.4, 20.7
+// and 16.5.
+static bool conv_runs_pay(int T, int R, int groups, int K) {
+  return (long long)T * groups * K >= (T >= 64LL * R ? 12800 : 18432);
+}
+
 // segs: n_seg x {col0, rows, width, unit} as ints, scales: n_seg floats.
 SGLC_API int sglc_short_conv(const float* x, long long x_stride, const float* taps, float* tail, float* y,
                              long long y_stride, const int* token_req, const int* q_start, const int* state_slots,
@@ -319,7 +330,7 @@ SGLC_API int sglc_short_conv(const float* x, long long x_stride, const float* ta
     rc = K == 4   ? sglc_launch(short_conv_step_kernel<4>, grid, block, 0, stream, 1, true, p)
          : K == 3 ? sglc_launch(short_conv_step_kernel<3>, grid, block, 0, stream, 1, true, p)
                   : sglc_launch(short_conv_step_kernel<2>, grid, block, 0, stream, 1, true, p);
-  } else if (runs) {
+  } else if (runs && conv_runs_pay(T, R, groups, K)) {
     const dim3 grid((T + CONV_RUN - 1) / CONV_RUN, groups), block(CONV_WARPS * 32);
     rc = K == 4   ? sglc_launch(short_conv_run_kernel<4>, grid, block, 0, stream, 1, true, p)
          : K == 3 ? sglc_launch(short_conv_run_kernel<3>, grid, block, 0, stream, 1, true, p)

@@ -306,6 +306,32 @@ def test_short_convolution_of_single_tokens(taps, D, V):
     assert torch.equal(whole, stepped)
 
 
+@pytest.mark.parametrize("taps,D,V", [(2, 12, 7), (3, 33, 64), (4, 64, 32)])
+def test_short_convolution_of_long_portions(taps, D, V):
+    """Portions long enough to go by runs of tokens, and the same in pieces that do not: the same bits, and the same inputs
+    left for the next step; a portion that starts inside a run, one of three tokens, tails of an earlier step."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(10 + taps)
+    lens, G, H, slots = [700, 3, 598], 4, 9, [3, 1, 4]
+    T, R, C = sum(lens), len(lens), 2 * G * D + H * V
+    x = torch.randn(T, C + 2 * H, generator=g).to(DEV)
+    w, a_log, dt = torch.randn(C, taps, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV), torch.randn(H, generator=g).to(DEV)
+    segs = [(0, G, D, 1, D ** -0.5), (G * D, G, D, 1, 1.0), (2 * G * D, H, V, 0, 1.0)]
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device=DEV)      # noqa: E731
+    tail0, starts = torch.randn(5, taps - 1, C, generator=g).to(DEV), np.concatenate([[0], np.cumsum(lens)]).tolist()
+
+    def run(rows, tail, lens, slots):
+        y, gates = torch.empty(sum(lens), C, device=DEV), torch.empty(sum(lens), 2 * H, device=DEV)
+        ops.short_conv(rows.contiguous(), w, tail, y, i32([r for r, m in enumerate(lens) for _ in range(m)]),
+                       i32(np.concatenate([[0], np.cumsum(lens)]).tolist()), i32(slots), len(lens), segs, gates=(H, C, C + H, a_log, dt, gates))
+        return torch.cat([y, gates], 1)
+
+    whole, pieces = tail0.clone(), tail0.clone()
+    got = run(x, whole, lens, slots)
+    cut = [run(x[s + p:s + min(p + 61, n)], pieces, [min(61, n - p)], [slot]) for s, n, slot in zip(starts, lens, slots) for p in range(0, n, 61)]
+    assert torch.equal(got, torch.cat(cut)) and torch.equal(whole, pieces)
+
+
 @pytest.mark.parametrize("E,top", [(1, 1), (8, 8), (8, 3), (31, 5), (32, 32), (33, 4), (96, 8)])
 def test_router_order_of_choice(E, top):
     """Logits with many ties on both sides of 32 experts: the larger first, the lower index first among equals."""
