@@ -431,6 +431,7 @@ constexpr int S_THREADS = (S_WARPS + 1) * 32;
 constexpr int S_MAX_STAGES = 8;
 constexpr int S_PMAX = 8;                   // page ids held per producer lane: 256 pages per item
 constexpr int S_TILE = 64;                  // keys per stage
+constexpr int S_WHOLE_TILES = 4;            // tiles of an item that a cluster does not share
 
 struct ItemGeom {
   int lo, first_page, k_base, n_rows, n_tiles, n_pages;
@@ -488,8 +489,8 @@ attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const
   if (SPLIT) cluster_arrive();                         // (its other half stands ahead of the first remote store)
   volatile int* af = &s_abort;
   // this block's tiles of an item: all of them, or its rank's run of them
-  // (an item of one or two tiles: the first rank's alone)
-  auto shared_item = [&](const ItemGeom& g) { return SPLIT && g.n_tiles > 2; };
+  // (an item of few tiles: the first rank's alone)
+  auto shared_item = [&](const ItemGeom& g) { return SPLIT && g.n_tiles > S_WHOLE_TILES; };
   auto first_tile = [&](const ItemGeom& g) {
     if (!shared_item(g)) return SPLIT && rank != 0 ? g.n_tiles : 0;
     return min(g.n_tiles, rank * ((g.n_tiles + sa.n_split - 1) / sa.n_split));
@@ -966,12 +967,15 @@ SGLC_API int sglc_attention_decode_stream(const void* q, int q_stride, void* cac
   if (per_sm > 3) per_sm = 3;
   if (per_sm < 1) per_sm = 1;
   int grid = n_sm * per_sm;
-  // Items that leave half of the resident blocks without work are shared by clusters of 2 (or 4) blocks: 208 items
-  // of 350 to 700 keys 14.3 -> 9.7 us a launch (28 MB of keys and values, 4.3 us at the copy rate).  (By the number
-  // of items alone, so that a token's bits do not depend on max_keys; an item of few keys stays with its cluster's
-  // first block, see the kernel.)
+  // Items that leave half of the resident blocks without work are shared by clusters of two blocks: 208 items of 350 to 700
+  // keys 14.3 -> 9.7 us a launch (28 MB of keys and values, 4.3 us at the copy rate).  An item of up to S_WHOLE_TILES tiles
+  // stays with its cluster's first block, and where no item can have more the launch is the plain one (its items
+  // have the same bits; a cluster costs it 0.2 to 1.2 us: 192 items of 32 / 100 / 200 keys 4.3 / 5.1 / 7.3 us plain, 5.0 /
+  // 6.1 / 7.7 in pairs; from 272 on the pairs win, 8.4 -> 7.6).  So a token's bits follow its own keys and the number of
+  // items, and not max_keys.
   sa.n_split = 1;
-  while (sa.n_split < S_MAX_SPLIT && sa.n_items * sa.n_split * 2 <= grid) sa.n_split *= 2;
+  const int most_rows = (window > 0 && window < max_keys ? window + page_size - 1 : max_keys) - 1;
+  if (sa.n_items * 2 <= grid && most_rows > S_WHOLE_TILES * S_TILE) sa.n_split = 2;
   if (sa.n_split > 1 || grid > sa.n_items) grid = sa.n_items;
   const bool split = sa.n_split > 1;
   auto kern = D == 64 ? (split ? attention_decode_stream_kernel<64, true> : attention_decode_stream_kernel<64, false>)
