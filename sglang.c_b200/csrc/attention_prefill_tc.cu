@@ -780,18 +780,14 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const Args& a, int R, 
 }  // namespace
 
 
-// Tuning hook: key tiles from which a query tile is split over two blocks (0: the rule decides).
-static int g_split_min = 0;
-SGLC_API void sglc_attention_prefill_set_split_min(int n) { g_split_min = n <= 0 ? 0 : n < 2 ? 2 : n; }
-// A split tile ends sooner but costs a second start and the exchange: the fewer query tiles there are for the 296
-// blocks that run at once, the smaller the tiles worth splitting, and none are where all blocks have more than one.
-// (us at head size 64, splits from 2 / 4 / 5 / no splits: 48 tiles of up to 4 key tiles 11.4 / 11.7 / 13.2 / 13.2,
-// 96 such 12.4 / 11.7 / 13.3 / 13.2, 192 of up to 8 23.7 / 23.8 / 17.4 / 21.5, 400 38.9 / 38.3 / 39.3 / 36.7, 1,600
-// 142.6 / 134.4 / 125.9 / 113.8.)
-static int split_from(long long query_tiles) {
-  if (g_split_min) return g_split_min;
-  return query_tiles <= 74 ? 2 : query_tiles <= 148 ? 4 : query_tiles <= 296 ? 5 : 1 << 30;
-}
+// Key tiles from which a query tile is split over two blocks.  A split tile ends sooner but costs a second start and the
+// exchange: where query tiles leave half of the blocks idle that run at once (296 at head size 64, 148 at 128) splits
+// of three key tiles still pay, beyond that those of five.  (us at head size 64, splits from 2 / 3 / 4 / 5 / none: 48 tiles of
+// up to 4 key tiles 10.1 / 9.1 / 9.5 / 11.1 / 11.0, 100 such 10.4 / 10.3 / 10.1 / 11.6 / 11.5, 192 17.7 / 17.1 / 17.4 / 13.2 / 13.2;
+// at 128, 64 such 11.0 / 10.7 / 11.2 / 13.6 / 13.6, 128 20.3 / 19.9 / 20.3 / 13.6 / 13.7.  No splits at all win by 5 to 10 %
+// where more than 296 tiles are prompts of 1,024 tokens, 33.7 and 35.5, and lose up to 45 % where the portions stand behind
+// a context, 400 tiles of 8 key tiles 73.3 and 55.2: the host knows no contexts.)
+static int split_from(long long query_tiles, int D) { return query_tiles <= (D == 64 ? 148 : 74) ? 3 : 5; }
 
 // Head sizes this kernel takes.
 SGLC_API int sglc_attention_prefill_tc_supports(int D) { return D == 64 || D == 128; }
@@ -829,7 +825,7 @@ static int attention_prefill_run(const void* q, int q_stride, const void* cache,
   a.skip_single = skip_single;
   a.R = R;
   a.pick = skip_single > 1 && skip_single < R ? 1 : 0;
-  a.split_min = split_from((long long)H * ((T + BQ - 1) / BQ));
+  a.split_min = split_from((long long)H * ((T + BQ - 1) / BQ), D);
   a.kv_shared = kv_shared;
   a.chunk = chunk;
   a.sinks = sinks;
