@@ -1451,16 +1451,20 @@ def gated_gather(z, tokens, table, first, dst, err_flag=None):
 EXT_MAX_SPLITS = 16         # blocks a token's keys are dealt to at most (attention_ext in a step of single tokens)
 
 
-def attention_ext_splits(max_keys, window=None, chunk=None, n_blocks=None):
-    """How many blocks share a token's keys in a step of single tokens: a tile of 32 keys a block, two where there are
-    few of them, up to EXT_MAX_SPLITS (1: the plain launch).  n_blocks: the launch's blocks without the split (tokens
-    times key/value heads): no more shares than keep all blocks resident at once.  Measured, 12 heads over 3 of 64, shares
-    of two tiles and of one: 8 tokens of 128 / 256 / 512 keys 10.5 -> 8.4, 10.2 -> 9.4, 11.9 -> 11.4 us, 32 tokens of 128 keys
-    11.8 -> 9.4; 64 keys are best left whole (7.0, two shares 8.7)."""
+def attention_ext_splits(max_keys, window=None, chunk=None, n_blocks=None, width=128):
+    """How many blocks share a token's keys in a step of single tokens, up to EXT_MAX_SPLITS (1: the plain launch).  n_blocks:
+    the launch's blocks without the split (tokens times key/value heads): no more shares than keep all blocks resident
+    at once; width: entries of a key and a value.  A tile of 32 keys a block where every tile can have one (wide heads: in
+    half of the room), else two: a few more shares than half the tiles only add to what is merged.  Measured, shares of
+    two tiles and of one: 12 heads over 3 of 64, 8 tokens of 128 / 256 / 512 keys 10.7 -> 8.9, 10.1 -> 9.9, 11.8 -> 11.2 us, 32
+    tokens of 128 11.8 -> 9.4, but 16 of 512 (8 and 9 shares) 12.8 -> 13.5; 16 heads, 4 of 256 (4 and 6) 9.5 -> 10.4; 8 heads
+    over 1 of 128, 16 of 100 14.9 -> 11.7, but 32 of 256 13.8 -> 15.0; 64 keys are best left whole (7.0, two shares 8.7)."""
     seen = min(int(max_keys), int(window or max_keys), int(chunk or max_keys))
-    tiles = (seen + 31) // 32 + 1
-    most = EXT_MAX_SPLITS if n_blocks is None else max(1, EXT_RESIDENT_BLOCKS // int(n_blocks))
-    return max(1, min(EXT_MAX_SPLITS, tiles if tiles > 4 else tiles // 2, most))
+    full = (seen + 31) // 32                      # (and one more where they do not start at a tile's edge)
+    blocks = int(n_blocks) if n_blocks is not None else 1
+    most = max(1, EXT_RESIDENT_BLOCKS // blocks)
+    each = full > 3 and blocks * min(full, EXT_MAX_SPLITS) <= EXT_RESIDENT_BLOCKS * 128 // max(128, int(width))
+    return max(1, min(EXT_MAX_SPLITS, full + 1 if each else (full + 1) // 2, most))
 
 
 EXT_RESIDENT_BLOCKS = 3 * 148
@@ -1496,7 +1500,7 @@ def attention_ext(q, cache, block_table, token_req, positions, out, n_heads, n_k
         splits = 1
         if max_q_len == 1:
             workspace = _tc_buffers(q.device)[0]
-            splits = min(attention_ext_splits(max_keys, window, chunk, T * n_kv_heads),
+            splits = min(attention_ext_splits(max_keys, window, chunk, T * n_kv_heads, dim + v_dim),
                          workspace.numel() // (T * n_heads * (v_dim + 2)))
             if splits < 1:
                 splits, workspace = 1, None

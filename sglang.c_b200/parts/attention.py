@@ -556,7 +556,7 @@ class RotaryAttention(Part):
         # (also one share a token, where query heads that share keys gain from staging them once)
         splits, ws = 1, None
         if ctx.max_q_len == 1:
-            splits = ops.attention_ext_splits(ctx.max_keys, p.get("window"), p.get("chunk"), T * G)
+            splits = ops.attention_ext_splits(ctx.max_keys, p.get("window"), p.get("chunk"), T * G, D + V)
             if splits > 1 or 2 <= H // G <= 8:
                 ws = ctx.alloc((T * H * splits * (V + 2),), torch.float32)
         ops.attention_ext(q, cache.tensor, grp.block_table, ctx.token_req, ctx.positions, o, H, G, D, V, grp.page_size,
