@@ -553,6 +553,39 @@ attention_f32_single_kernel(const F32Args a) {
   }
 }
 
+// Which kernel takes a 32-bit launch without extensions: the general one, or one of the two above (the same bits from each).
+//   Portions: the kernel of four tokens a warp needs a quarter of the blocks for four times the tokens, so it pays where the
+//   general kernel's blocks (eight tokens of a head) would take more than one round of the 444 that run at once, and
+//   where a block's tokens belong to few requests, for runs of different requests take turns in a block.  Measured, head
+//   sizes 64 and 128, general kernel and this one: one prompt of 128 tokens, 12 heads (192 general blocks) 13.7 and 20.6 us,
+//   384 (576) 51.9 and 59.3, 512 (768) 79.8 and 73.3, 1,000 (1,500) 246 and 142; 16 portions of 16 tokens behind 640 keys 77
+//   and 131, of 32 149 and 98; two tokens each of 16 requests of 640 keys 133 and 680; 31 single tokens of 640 keys beside a
+//   portion of 481 364 and 1,236.  At head size 32 tiles are small: 8 x 120 (1,440) 33 and 36, 2 x 320 (960) 48 and 43.
+//   Single tokens: a block of the pipelined kernel is two to three times as fast as a general one, but an SM holds fewer of
+//   them (two at head size 64, one beyond, the general kernel's four): it pays as long as its rounds are no more than the
+//   general kernel's.  Blocks, head size, keys: 192 / 64 / 140 11.5 and 8.3 us, 384 / 64 / 140 12.8 and 14.8, 768 / 64 / 140
+//   26.5 and 21.8, 3,072 / 64 / 140 72.9 and 77.2; 128 / 128 / 140 14.4 and 8.7, 384 / 128 / 140 18.3 and 24.5, 2,048 / 128 /
+//   140 77.5 and 128; 3,072 / 32 / 140 57.7 and 39.6.
+// n_portions: how many requests the tokens belong to where each brings several (0: not known, or single tokens among
+// them).
+enum { F32_GENERAL = 0, F32_PORTIONS = 1, F32_SINGLES = 2 };
+static size_t f32_single_smem(int D) { return ((size_t)3 * 64 * (2 * D + 4) + D) * sizeof(float); }
+static int f32_form(int T, int H, int D, int max_q_len, int n_portions) {
+  if (D % 4 != 0 || D > 128) return F32_GENERAL;
+  if (max_q_len <= 1) {
+    const long long blocks = (long long)T * H;
+    const int here = (int)(228 * 1024 / (f32_single_smem(D) + 1024));            // blocks an SM holds
+    const long long rounds = (blocks + 148 * here - 1) / (148 * here), general = (blocks + 591) / 592;
+    return here >= 4 || rounds == 1 || (here >= 2 && rounds <= 3 && rounds * here < general * 4) ? F32_SINGLES : F32_GENERAL;
+  }
+  const long long blocks = (long long)((T + 7) / 8) * H;
+  if (n_portions <= 0 || (T + FP_W - 1) / FP_W > 65535) return F32_GENERAL;
+  return (D >= 64 ? blocks >= 640 && T >= 32 * n_portions : blocks >= 960 && T >= 160 * n_portions) ? F32_PORTIONS : F32_GENERAL;
+}
+SGLC_API int sglc_attention_f32_form(int T, int H, int D, int max_q_len, int n_portions) {
+  return f32_form(T, H, D, max_q_len, n_portions);
+}
+
 template <typename K>
 static int launch_f32(K* kernel, dim3 grid, int threads, size_t smem, const F32Args& a, cudaStream_t stream) {
   if (smem > 48 * 1024) {
@@ -568,13 +601,14 @@ static int launch_f32(K* kernel, dim3 grid, int threads, size_t smem, const F32A
 // last one it sees); out: [T][o_stride].  max_keys: the most keys any token of this launch
 // sees.  q/out dtype = act_dtype, cache dtype = cache_dtype.  n_pages and err serve the
 // bounds-check build (page ids are compared with n_pages; err gets the flag).  max_q_len: the
-// longest portion of the step (1: every request brings one token, and a block takes one token).
+// longest portion of the step (1: every request brings one token, and a block takes one token); n_portions:
+// see f32_form.
 static int attention_simt_run(const void* q, int q_stride, const void* cache,
                               const int* block_table, int bt_stride, const int* token_req,
                               const int* positions, void* out, int o_stride, int T, int H,
                               int Hkv, int D, int page_size, float scale, int window,
                               int max_keys, int act_dtype, int cache_dtype, int n_pages, int* err,
-                              int max_q_len, int kv_shared, cudaStream_t stream, bool ext = false, int DV = 0,
+                              int max_q_len, int n_portions, int kv_shared, cudaStream_t stream, bool ext = false, int DV = 0,
                               int chunk = 0, const float* sinks = nullptr, int n_splits = 1, float* part_ws = nullptr,
                               OutGate gate = OutGate{nullptr, 0, 0}) {
   if (T <= 0) return SGLC_OK;
@@ -586,20 +620,19 @@ static int attention_simt_run(const void* q, int q_stride, const void* cache,
   if (H > 65535 || D > (ext ? 768 : 256)) return SGLC_ERR_UNSUPPORTED;
   // single tokens of many requests share nothing: a token a block; portions: eight tokens a block
   const bool single = max_q_len <= 1;
-  if (!ext && act_dtype == SGLC_F32 && cache_dtype == SGLC_F32 && D % 4 == 0 && D <= 128 && ((uintptr_t)cache & 15) == 0) {
+  const int form = !ext && act_dtype == SGLC_F32 && cache_dtype == SGLC_F32 && ((uintptr_t)cache & 15) == 0
+                       ? f32_form(T, H, D, max_q_len, n_portions) : F32_GENERAL;
+  if (form != F32_GENERAL) {
     F32Args a = {};
     a.q = (const float*)q; a.q_stride = q_stride; a.cache = (const float*)cache; a.block_table = block_table;
     a.bt_stride = bt_stride; a.token_req = token_req; a.positions = positions; a.out = (float*)out; a.o_stride = o_stride;
     a.T = T; a.H = H; a.Hkv = Hkv; a.D = D; a.page_size = page_size; a.scale = scale; a.window = window;
     a.n_pages = n_pages; a.kv_shared = kv_shared; a.err = err;
-    if (single) {
-      const size_t smem = ((size_t)3 * 64 * (2 * D + 4) + D) * sizeof(float);
-      return D <= 64 ? launch_f32(attention_f32_single_kernel<1>, dim3(T, H), 128, smem, a, stream)
-                     : launch_f32(attention_f32_single_kernel<2>, dim3(T, H), 128, smem, a, stream);
-    }
+    if (form == F32_SINGLES)
+      return D <= 64 ? launch_f32(attention_f32_single_kernel<1>, dim3(T, H), 128, f32_single_smem(D), a, stream)
+                     : launch_f32(attention_f32_single_kernel<2>, dim3(T, H), 128, f32_single_smem(D), a, stream);
     const size_t smem = ((size_t)2 * 32 * (2 * D + 4) + (size_t)FP_W * (D + 32)) * sizeof(float);
     const dim3 grid(H, (T + FP_W - 1) / FP_W);
-    if (grid.y > 65535) return SGLC_ERR_UNSUPPORTED;
     return D <= 64 ? launch_f32(attention_f32_portion_kernel<2>, grid, 256, smem, a, stream)
                    : launch_f32(attention_f32_portion_kernel<4>, grid, 256, smem, a, stream);
   }
@@ -673,10 +706,10 @@ SGLC_API int sglc_attention_simt(const void* q, int q_stride, const void* cache,
                                  const int* positions, void* out, int o_stride, int T, int H,
                                  int Hkv, int D, int page_size, float scale, int window,
                                  int max_keys, int act_dtype, int cache_dtype, int n_pages, int* err,
-                                 int max_q_len, cudaStream_t stream) {
+                                 int max_q_len, int n_portions, cudaStream_t stream) {
   return attention_simt_run(q, q_stride, cache, block_table, bt_stride, token_req, positions, out, o_stride,
                             T, H, Hkv, D, page_size, scale, window, max_keys, act_dtype, cache_dtype,
-                            n_pages, err, max_q_len, 0, stream);
+                            n_pages, err, max_q_len, n_portions, 0, stream);
 }
 
 // The same over a cache whose pages hold one block of rows [Hkv][page_size][D] that serve as keys
@@ -686,10 +719,10 @@ SGLC_API int sglc_attention_simt_shared(const void* q, int q_stride, const void*
                                         const int* positions, void* out, int o_stride, int T, int H,
                                         int Hkv, int D, int page_size, float scale, int window,
                                         int max_keys, int act_dtype, int cache_dtype, int n_pages, int* err,
-                                        int max_q_len, cudaStream_t stream) {
+                                        int max_q_len, int n_portions, cudaStream_t stream) {
   return attention_simt_run(q, q_stride, cache, block_table, bt_stride, token_req, positions, out, o_stride,
                             T, H, Hkv, D, page_size, scale, window, max_keys, act_dtype, cache_dtype,
-                            n_pages, err, max_q_len, 1, stream);
+                            n_pages, err, max_q_len, n_portions, 1, stream);
 }
 
 // The extended form: values of size DV beside keys of size D (cache [n_pages][Hkv x page_size x D keys |
@@ -708,7 +741,7 @@ SGLC_API int sglc_attention_simt_ext(const void* q, int q_stride, const void* ca
                                      int gate_per_head, cudaStream_t stream) {
   return attention_simt_run(q, q_stride, cache, block_table, bt_stride, token_req, positions, out, o_stride,
                             T, H, Hkv, D, page_size, scale, window, max_keys, act_dtype, cache_dtype,
-                            n_pages, err, max_q_len, kv_shared, stream, true, DV, chunk, sinks, 1, nullptr,
+                            n_pages, err, max_q_len, 0, kv_shared, stream, true, DV, chunk, sinks, 1, nullptr,
                             OutGate{gate, gate_stride, gate_per_head});
 }
 
@@ -764,7 +797,7 @@ SGLC_API int sglc_attention_simt_ext_split(const void* q, int q_stride, const vo
   if (!part_ws || n_splits < 1) return SGLC_ERR_ARGUMENT;
   const int code = attention_simt_run(q, q_stride, cache, block_table, bt_stride, token_req, positions, out, o_stride,
                                       T, H, Hkv, D, page_size, scale, window, max_keys, act_dtype, cache_dtype,
-                                      n_pages, err, 1, kv_shared, stream, true, DV, chunk, nullptr, n_splits, part_ws);
+                                      n_pages, err, 1, 0, kv_shared, stream, true, DV, chunk, nullptr, n_splits, part_ws);
   if (code != SGLC_OK) return code;
   const dim3 grid((unsigned)(((long long)T * H + 3) / 4));
   const OutGate g{gate, gate_stride, gate_per_head};

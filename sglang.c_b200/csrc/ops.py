@@ -277,11 +277,12 @@ def _gate_args(gate, T, n_heads, width, what):
 
 
 def attention_simt(q, cache, block_table, token_req, positions, out, n_heads, scale, window,
-                   max_keys, max_q_len=None, kv_shared=False):
+                   max_keys, max_q_len=None, kv_shared=False, n_portions=0):
     """Causal attention of T tokens over the paged cache, 32-bit arithmetic.
     q: [T, n_heads*head_dim] view; out likewise; block_table int32 [R, max_blocks].
     max_q_len: the longest portion among the tokens (1 when every request brings one token;
-    unknown: None); it only decides how many tokens share a block.
+    unknown: None); n_portions: how many requests the tokens belong to where each brings several (0:
+    unknown, or single tokens among them).  Both only decide which kernel works, and how many tokens share a block.
     kv_shared: cache is [n_pages, 1, n_kv_heads, page_size, head_dim], rows that are keys and
     values at once."""
     _need_cuda(q, cache, block_table, token_req, positions, out)
@@ -302,8 +303,15 @@ def attention_simt(q, cache, block_table, token_req, positions, out, n_heads, sc
               out.stride(0), T, n_heads, Hkv, D, page_size, ctypes.c_float(scale),
               int(window or 0), int(max_keys), _dt(q, "attention q"),
               _dt(cache, "cache"), n_pages, _ptr(tc_error_flag(q.device)),
-              int(max_q_len) if max_q_len else 2, _stream())
+              int(max_q_len) if max_q_len else 2, int(n_portions), _stream())
     _check(lib, code, f"attention_simt (head_dim {D}, up to {max_keys} keys)")
+
+
+def attention_f32_form(n_tokens, n_heads, dim, max_q_len, n_portions=0):
+    """Which kernel attention_simt takes for such a 32-bit step without extensions: "general", "portions" or "singles"."""
+    lib = build.load("attention_simt")
+    return ("general", "portions", "singles")[lib.sglc_attention_f32_form(int(n_tokens), int(n_heads), int(dim), int(max_q_len),
+                                                                          int(n_portions))]
 
 
 # ---------------------------------------------------------------------------

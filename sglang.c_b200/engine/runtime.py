@@ -100,7 +100,7 @@ class Runtime:
                                      n_tokens=ctx.n_decode)
             return
         ops.attention_simt(q, cache, grp.block_table, ctx.token_req, ctx.positions, out, n_heads,
-                           scale, window, ctx.max_keys, max_q_len=ctx.max_q_len)
+                           scale, window, ctx.max_keys, max_q_len=ctx.max_q_len, n_portions=0 if ctx.n_decode else ctx.R)
 
     def attend_shared(self, ctx, q, binding, grp, out, n_heads, head_dim, scale, window, sinks=None, gate=None):
         """Causal attention of the step's queries over a cache whose rows are keys and values at
@@ -136,4 +136,5 @@ class Runtime:
                               max_q_len=ctx.max_q_len, splits=None, kv_shared=True, gate=gate)
             return
         ops.attention_simt(q, cache, grp.block_table, ctx.token_req, ctx.positions, out, n_heads,
-                           scale, window, ctx.max_keys, max_q_len=ctx.max_q_len, kv_shared=True)
+                           scale, window, ctx.max_keys, max_q_len=ctx.max_q_len, kv_shared=True,
+                           n_portions=0 if ctx.n_decode else ctx.R)

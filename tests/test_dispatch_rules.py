@@ -1,7 +1,11 @@
 """Rules by which launches choose a kernel or a split, at the sizes that they were measured at (no GPU)."""
+from types import SimpleNamespace
+
 import pytest
+import torch
 
 from sglang_c_b200.csrc import ops
+from sglang_c_b200.engine.runtime import Runtime
 
 
 @pytest.mark.parametrize("keys,blocks,width,splits", [
@@ -12,3 +16,30 @@ def test_a_tile_a_share_only_where_every_tile_has_one(keys, blocks, width, split
     assert ops.attention_ext_splits(keys, None, None, blocks, width) == splits
     assert ops.attention_ext_splits(4 * keys, keys, None, blocks, width) == splits          # (a window)
     assert ops.attention_ext_splits(4 * keys, None, keys, blocks, width) == splits          # (a chunk)
+
+
+@pytest.mark.parametrize("tokens,heads,dim,longest,portions,form", [
+    (128, 12, 64, 128, 1, "general"), (384, 12, 64, 384, 1, "general"), (512, 12, 64, 512, 1, "portions"), (256, 25, 64, 256, 1, "portions"),
+    (512, 8, 128, 512, 1, "general"), (640, 8, 128, 640, 1, "portions"), (512, 12, 64, 16, 32, "general"), (512, 12, 64, 32, 16, "portions"),
+    (32, 12, 64, 2, 16, "general"), (512, 12, 64, 481, 0, "general"), (1000, 12, 32, 1000, 1, "portions"), (960, 12, 32, 120, 8, "general"),
+    (512, 12, 66, 512, 1, "general"), (512, 12, 132, 512, 1, "general"), (1 << 22, 1, 64, 1 << 22, 1, "general"),
+    (8, 12, 64, 1, 0, "singles"), (24, 12, 64, 1, 0, "singles"), (32, 12, 64, 1, 0, "general"), (64, 12, 64, 1, 0, "singles"),
+    (128, 12, 64, 1, 0, "general"), (256, 12, 64, 1, 0, "general"), (16, 8, 128, 1, 0, "singles"), (24, 8, 128, 1, 0, "general"),
+    (64, 8, 128, 1, 0, "general"), (256, 12, 32, 1, 0, "singles")])
+def test_32_bit_attention_takes_the_kernel_that_was_faster(tokens, heads, dim, longest, portions, form):
+    assert ops.attention_f32_form(tokens, heads, dim, longest, portions) == form
+
+
+@pytest.mark.parametrize("singles", [0, 1, 31])
+def test_a_step_with_single_tokens_is_no_step_of_portions(monkeypatch, singles):
+    """What the runtime tells the 32-bit kernels of a step: single tokens beside portions would take turns with them."""
+    told = []
+    monkeypatch.setattr(ops, "attention_simt", lambda *a, n_portions=0, **kw: told.append(n_portions))
+    rt = Runtime.__new__(Runtime)
+    rt.dtype = "float32"
+    q = torch.zeros(4, 8)
+    ctx = SimpleNamespace(n_decode=singles, R=2 + singles, max_q_len=9, token_req=None, positions=None, max_keys=9)
+    grp, binding = SimpleNamespace(block_table=None, slots=None), SimpleNamespace(tensor=torch.zeros(1, 2, 1, 4, 8), write=False)
+    rt.attend(ctx, q, q, q, binding, grp, q, 1, 1, 8, 1.0, None)
+    rt.attend_shared(ctx, q, binding, grp, q, 1, 8, 1.0, None)
+    assert told == ([0, 0] if singles else [2, 2])

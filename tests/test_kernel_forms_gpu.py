@@ -62,6 +62,24 @@ def test_attention_f32_has_the_same_bits_in_every_cut(H, Hkv, D, ps, window):
         assert torch.equal(out, whole[pick]), longest
 
 
+@pytest.mark.parametrize("H,Hkv,D,ps,window", [(16, 4, 64, 16, None), (16, 16, 128, 8, 40), (30, 2, 36, 16, 33), (30, 30, 4, 32, None)])
+def test_attention_f32_portions_have_the_general_kernels_bits(H, Hkv, D, ps, window):
+    """Portions of several requests in blocks of 32 tokens, against the kernel of a token a warp and float64: prompts and a
+    portion behind a context, lengths off the edges of tiles and blocks."""
+    ops = _ops()
+    lens, q_lens = [330, 97, 333], [330, 97, 63] if D >= 64 else [330, 97, 133]
+    c = _paged_case(lens, q_lens, H, Hkv, D, ps, torch.float32, seed=D)
+    T, scale, outs = sum(q_lens), 1.3 / math.sqrt(D), []
+    assert ops.attention_f32_form(T, H, D, 330, 3) == "portions" and ops.attention_f32_form(T, H, D, 330, 0) == "general"
+    for n_portions in (0, 3):
+        out = torch.full((T, H * D), float("nan"), device=DEV)
+        ops.attention_simt(c["q"], c["cache"], c["bt"], c["token_req"], c["positions"], out, H, scale, window, 333, max_q_len=330,
+                           n_portions=n_portions)
+        outs.append(out)
+    assert torch.equal(*outs)
+    assert float((outs[0].double().cpu() - _attention_reference(c, H, Hkv, D, scale, window)).abs().max()) < 2e-5
+
+
 @pytest.mark.parametrize("D,at", [(64, 9), (64, 61), (128, 40)])
 def test_attention_f32_keeps_a_bad_value_from_the_tokens_before_it(D, at):
     """A value that is infinite or no number reaches the tokens that see it, and no other token of its tile or block."""
@@ -72,8 +90,10 @@ def test_attention_f32_keeps_a_bad_value_from_the_tokens_before_it(D, at):
 
     def run():
         out = torch.zeros(T, H * D, device=DEV)
-        ops.attention_simt(c["q"], c["cache"], c["bt"], c["token_req"], c["positions"], out, H, 0.1, None, 640, max_q_len=600)
+        ops.attention_simt(c["q"], c["cache"], c["bt"], c["token_req"], c["positions"], out, H, 0.1, None, 640, max_q_len=600, n_portions=2)
         return out
+
+    assert ops.attention_f32_form(T, H, D, 600, 2) == "portions"
 
     clean = run()
     for bad in (float("inf"), float("nan")):
