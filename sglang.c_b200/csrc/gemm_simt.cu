@@ -304,6 +304,66 @@ gemm_simt_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, 
   }
 }
 
+// 9 to 16 rows of some thousand features: with few features a block and 128 threads to it enough weights are on their way
+// without any of a lane's chains being longer.  A block takes 16 rows of 16 features; tiles of 32 k come through a ring of
+// eight shared-memory stages by asynchronous 16-byte copies, seven tiles ahead of the arithmetic; a thread owns two
+// rows of one feature, k ascending: the same bits again.  16 rows, this kernel and the best of one-warp blocks: 2,304 columns
+// over K 768 8.3 and 9.0 us, 3,072 10.6 and 11.3, 4,096 over 1,024 13.9 and 15.8.
+constexpr int FEW_M = 16, FEW_N = 16, FEW_K = 32, FEW_ST = 8, FEW_PITCH = FEW_K + 4;
+
+__global__ void __launch_bounds__(128)
+gemm_simt_few_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias,
+                     float* __restrict__ out, float* __restrict__ residual, int M, int N, int K, int lda,
+                     int ldo, int act) {
+  __shared__ __align__(16) float As[FEW_ST][FEW_M][FEW_PITCH];
+  __shared__ __align__(16) float Ws[FEW_ST][FEW_N][FEW_PITCH];
+  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+  const int m0 = blockIdx.y * FEW_M, n0 = blockIdx.x * FEW_N;
+  const int lrow = tid / 8, lk = (tid % 8) * 4;      // this thread's 16-byte piece of a tile row
+  const int n_tiles = (K + FEW_K - 1) / FEW_K;
+  auto issue = [&](int tile) {
+    if (tile < n_tiles) {
+      const int st = tile % FEW_ST, k = tile * FEW_K + lk;
+      const bool kin = k < K;                        // (K is a multiple of 4: a piece lies inside or outside)
+      const int m = m0 + lrow;
+      cp_async16_zfill(&As[st][lrow][lk], A + (size_t)(m < M ? m : 0) * lda + (kin ? k : 0), kin && m < M);
+      const int n = n0 + lrow;
+      cp_async16_zfill(&Ws[st][lrow][lk], W + (size_t)(n < N ? n : 0) * K + (kin ? k : 0), kin && n < N);
+    }
+    cp_async_commit();
+  };
+  for (int t = 0; t < FEW_ST - 1; t++) issue(t);
+  float acc[2] = {0.0f, 0.0f};
+  for (int tile = 0; tile < n_tiles; tile++) {
+    cp_async_wait<FEW_ST - 2>();
+    __syncthreads();                                 // tile `tile` has landed; the stage of tile-1 is free
+    issue(tile + FEW_ST - 1);
+    const int st = tile % FEW_ST;
+#pragma unroll
+    for (int k = 0; k < FEW_K; k += 4) {
+      const float4 a0 = *reinterpret_cast<const float4*>(&As[st][2 * ty][k]);
+      const float4 a1 = *reinterpret_cast<const float4*>(&As[st][2 * ty + 1][k]);
+      const float4 w0 = *reinterpret_cast<const float4*>(&Ws[st][tx][k]);
+      acc[0] = fmaf(a0.x, w0.x, acc[0]); acc[1] = fmaf(a1.x, w0.x, acc[1]);
+      acc[0] = fmaf(a0.y, w0.y, acc[0]); acc[1] = fmaf(a1.y, w0.y, acc[1]);
+      acc[0] = fmaf(a0.z, w0.z, acc[0]); acc[1] = fmaf(a1.z, w0.z, acc[1]);
+      acc[0] = fmaf(a0.w, w0.w, acc[0]); acc[1] = fmaf(a1.w, w0.w, acc[1]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int m = m0 + 2 * ty + i;
+    const int n = n0 + tx;
+    if (m >= M || n >= N) continue;
+    float v = acc[i];
+    if (bias) v += bias[n];
+    v = apply_act(v, act);
+    const size_t o = (size_t)m * ldo + n;
+    if (residual) residual[o] = residual[o] + v;
+    else out[o] = v;
+  }
+}
+
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   unsigned long long r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
@@ -461,6 +521,11 @@ int launch_tile(const SimtArgs& p, cudaStream_t stream) {
                      stream, 1, false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K, p.lda, p.ldo, p.act);
 }
 
+int launch_few(const SimtArgs& p, cudaStream_t stream) {
+  return sglc_launch(gemm_simt_few_kernel, dim3((p.N + FEW_N - 1) / FEW_N, (p.M + FEW_M - 1) / FEW_M), dim3(128), 0, stream, 1,
+                     false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K, p.lda, p.ldo, p.act);
+}
+
 template <int BMT, int BNT, int BLOCKS>
 int launch_pair(const SimtArgs& p, cudaStream_t stream) {
   return sglc_launch(gemm_simt_pair_kernel<BMT, BNT, BLOCKS>, dim3((p.N + BNT - 1) / BNT, (p.M + BMT - 1) / BMT),
@@ -470,7 +535,7 @@ int launch_pair(const SimtArgs& p, cudaStream_t stream) {
 
 // Tuning hook: 0 (default) lets the launcher choose the kernel.
 int g_simt_form = 0;
-enum { FORM_ROWS = 1, FORM_ROWS_WIDE, FORM_TILE, FORM_PAIR, FORM_PAIR_WIDE };
+enum { FORM_ROWS = 1, FORM_ROWS_WIDE, FORM_TILE, FORM_PAIR, FORM_PAIR_WIDE, FORM_FEW };
 
 int choose_form(int M, int N) {
   if (M <= 64) return FORM_ROWS;
@@ -497,6 +562,7 @@ int simt_f32(const SimtArgs& p, cudaStream_t stream) {
     case FORM_TILE: return launch_tile(p, stream);
     case FORM_PAIR: return launch_pair<128, 64, 3>(p, stream);
     case FORM_PAIR_WIDE: return launch_pair<128, 128, 2>(p, stream);
+    case FORM_FEW: return launch_few(p, stream);
   }
   // Few rows, by the narrowest: the chain of K multiply-adds bounds a product, so a lane has one output; wider
   // ones, where shared-memory reads do, more; the vocabulary's head, where enough weights have to be on their way,
@@ -504,7 +570,17 @@ int simt_f32(const SimtArgs& p, cudaStream_t stream) {
   // 4.8 (a row a lane) / 9.1 / 11.4, over K 3,072 12.6 / 29.9 / 37.9, 2,304 columns 7.5 / 9.5 / 11.9, 50,257
   // columns 67.9 / 52.7 / 43.8.)
   if (p.M <= 4) return p.N <= 8192 ? launch_rows<1, 1, 10>(p, stream) : launch_rows<1, 2, 4>(p, stream);
-  if (p.N > 8192) return p.M <= 8 ? launch_rows<2, 4, 3>(p, stream) : launch_rows<4, 4, 3>(p, stream);
+  if (p.M <= 8) {
+    if (p.N > 8192) return launch_rows<2, 4, 3>(p, stream);
+  } else if (p.M <= 16) {
+    // (us at 16 rows, 8 rows of 8 features a block, of 16, of 32 and 16 rows of 32: 4,800 columns over K 1,600 30.6 / 23.9 /
+    // 26.2 / 42.1, 6,400 over 1,600 41.0 / 27.3 / 26.4 / 31.5, 8,200 over 768 21.8 / 19.3 / 17.6 / 21.8, 12,288 - / 28.0 / 23.8 / 22.3.)
+    if (p.N > 10240) return launch_rows<4, 4, 3>(p, stream);
+    if (p.N > 4608) return launch_rows<2, 4, 3>(p, stream);
+    if (p.N > 1792) return launch_few(p, stream);
+  } else if (p.N > 8192) {
+    return launch_rows<4, 4, 3>(p, stream);
+  }
   if (p.M <= 16) {
     if (p.N <= 1024) return launch_rows<1, 1, 10>(p, stream);
     return p.N <= 2304 ? launch_rows<2, 1, 10>(p, stream) : launch_rows<2, 2, 8>(p, stream);
