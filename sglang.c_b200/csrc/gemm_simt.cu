@@ -117,7 +117,8 @@ gemm_simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, 
   const int m0 = blockIdx.y * BMT, n0 = blockIdx.x * BNT;
   const int n_tiles = (K + LK - 1) / LK;
   const int crow = tid / 8, ck = (tid % 8) * 4;
-  // (rows beyond the last are copies of it: their outputs are not stored)
+  // (weight rows beyond the last are copies of it, their outputs are not stored; token rows beyond the last are zeros, for
+  // every block would ask for the same lines again: 65 tokens of 12,288 columns over K 768 122.8 -> 68.8 us)
   auto ask_w = [&](int tile, int st) {
     float* to = ring + st * STAGE + BMT * LPITCH + crow * LPITCH + ck;
     const int k = tile * LK + ck;
@@ -134,7 +135,7 @@ gemm_simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     const float* from = A + (on ? k : 0);
 #pragma unroll
     for (int r = 0; r < BMT / STEP; r++)
-      cp_async16_zfill(to + r * STEP * LPITCH, from + (size_t)min(m0 + crow + r * STEP, M - 1) * lda, on);
+      cp_async16_zfill(to + r * STEP * LPITCH, from + (size_t)min(m0 + crow + r * STEP, M - 1) * lda, on && m0 + crow + r * STEP < M);
   };
   for (int t = 0; t < ST; t++) {
     if (t < n_tiles) { ask_a(t, t); ask_w(t, t); }
