@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 # -- 32-bit products -----------------------------------------------------------------------------
-ROWS, ROWS_WIDE, TILE, PAIR, PAIR_WIDE, FEW = 1, 2, 3, 4, 5, 6
+ROWS, ROWS_WIDE, TILE, PAIR, PAIR_WIDE, FEW, BLOCK = 1, 2, 3, 4, 5, 6, 7
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (8, 9, 60), (9, 2305, 68), (16, 8193, 36), (3, 8200, 68), (8, 8200, 100), (12, 4700, 68),
@@ -28,7 +28,7 @@ def test_gemm_simt_forms_give_the_same_bits(M, N, K):
     ref = a.double() @ w.double().t() + bias.double()
     first = None
     try:
-        for form in (ROWS, ROWS_WIDE, TILE, PAIR, PAIR_WIDE, FEW, 0):
+        for form in (ROWS, ROWS_WIDE, TILE, PAIR, PAIR_WIDE, FEW, BLOCK, 0):
             lib.sglc_gemm_simt_set_form(form)
             out = torch.full((M, N), float("nan"), device=DEV)
             ops.gemm_simt(a, w, bias, out=out)
