@@ -1029,6 +1029,32 @@ bool get_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, u
   return true;
 }
 
+// Whether the device holds a cluster of 16 blocks of the few-token kernel (more than eight is an opt-in size that a device
+// may lack, as a part of one may): asked once, for the largest shared memory a block of it takes.
+int widest_cluster() {
+  static const int widest = [] {
+    constexpr int SMEM = 96 * 1024 + (BM + 16) * (16 + 4) * 4 + 1024;
+    auto* kernel = gemm_tc_kernel<16, false>;
+    int n = 0;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 16;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, 16);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
+                    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaFuncSetAttribute(gemm_tc_kernel<16, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    if (!ok) cudaGetLastError();
+    return ok ? 16 : 8;
+  }();
+  return widest;
+}
+
 template <int BN, bool XI>
 int launch(const CUtensorMap& mp, const CUtensorMap& mq, const CUtensorMap& mo, const GemmArgs& a,
            dim3 grid, cudaStream_t stream) {
@@ -1040,7 +1066,6 @@ int launch(const CUtensorMap& mp, const CUtensorMap& mq, const CUtensorMap& mo, 
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, XI>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    cudaFuncSetAttribute(gemm_tc_kernel<BN, XI>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);    // (clusters of 16)
     // ask for the largest shared-memory split of the SM, so that two blocks fit side by side
     // (one block's epilogue then overlaps the other's main loop)
     cudaFuncSetAttribute(gemm_tc_kernel<BN, XI>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1169,13 +1194,17 @@ static int long_k_split(int M, int N, int kb_total) {
   if (tiles * 3 <= 264) return tiles * 8 <= 264 ? 8 : (int)(264 / tiles);
   return tiles * 2 <= 296 ? 2 : 0;
 }
-// deal_k: false for the projections that write the cache, which only the many-token kernels do.
 // Few tokens and features over a long K: clusters of 16 blocks where 8 leave every other SM without one; the weights
 // of a block's share then all find room in its ring, ahead of the wait for the kernel before.  Measured, us with 8
-// and with 16, up to 16 tokens: 768 columns over K 2,048 / 3,072 / 8,192 4.4 / 5.0 / 7.9 and 4.8 / 4.9 / 6.5, 1,024 over
-// 4,096 5.8 and 5.2, 1,152 over 4,608 6.2 and 5.7; 32 tokens, 1,024 over 4,096 6.3 and 9.8 (not all clusters fit at once).
-static bool wide_split(int M, int tiles_p, int kb_total) { return M <= 16 && tiles_p <= 9 && kb_total >= 48; }
-static void plan(int M, int N, int K, bool deal_k, int* swap, int* bn, int* splits, int* kb_per_split,
+// and with 16, up to 16 tokens: 256 columns over K 3,008 / 3,072 / 8,192 4.9 / 4.9 / 7.7 and 4.9 / 4.4 / 5.8, 768 over 3,072 / 4,096 /
+// 8,192 5.1 / 5.7 / 8.0 and 5.0 / 5.2 / 6.5; of 1,024 and 1,152 over 3,072 5.3 and 5.3 or 5.4, over 3,584 5.6 and 5.1 or
+// 5.3; 32 tokens, 1,024 over 4,096 6.3 and 9.8 (not all clusters fit at once).
+static bool wide_split(int M, int tiles_p, int kb_total) {
+  return M <= 16 && kb_total >= 48 && (tiles_p <= 6 || (tiles_p <= 9 && kb_total >= 56));
+}
+// deal_k: false for the projections that write the cache, which only the many-token kernels do; widest: the largest
+// cluster the device holds.
+static void plan(int M, int N, int K, bool deal_k, int widest, int* swap, int* bn, int* splits, int* kb_per_split,
                  int* tiles_p, int* tiles_q) {
   int kb_total = (K + BK - 1) / BK;
   if (const int want = deal_k ? long_k_split(M, N, kb_total) : 0) {
@@ -1193,7 +1222,7 @@ static void plan(int M, int N, int K, bool deal_k, int* swap, int* bn, int* spli
     // enough blocks to put most SMs on the weights, but few enough partial sums that the
     // last block's reduction stays short
     int want = (2 * 148) / (*tiles_p);
-    if (want > 8) want = wide_split(M, *tiles_p, kb_total) ? 16 : 8;
+    if (want > 8) want = widest >= 16 && wide_split(M, *tiles_p, kb_total) ? 16 : 8;
     if (want < 1) want = 1;
     if (want > kb_total) want = kb_total;
     int per = (kb_total + want - 1) / want;
@@ -1256,7 +1285,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   if (K % 8 != 0 || lda % 8 != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15))
     return SGLC_ERR_UNSUPPORTED;
   int swap, bn, splits, per, tp, tq;
-  plan(M, N, K, kv == nullptr, &swap, &bn, &splits, &per, &tp, &tq);
+  plan(M, N, K, kv == nullptr, widest_cluster(), &swap, &bn, &splits, &per, &tp, &tq);
   const bool xi = act_is_xielu(act);          // the epilogue's other instantiation
   GemmArgs a;
   a.M = M; a.N = N; a.K = K;
@@ -1359,13 +1388,20 @@ SGLC_API int sglc_gemm_tc_kv(const void* A, const void* W, const float* bias, vo
   return gemm_tc_run(A, W, bias, out, nullptr, M, N, K, lda, ldo, 0, act, err, &kv, stream);
 }
 
+// Into how many shares of K a product is dealt where the device holds clusters of `widest` blocks (1: none; for tests).
+SGLC_API int sglc_gemm_tc_shares(int M, int N, int K, int widest) {
+  int swap, bn, splits, per, tp, tq;
+  plan(M, N, K, true, widest, &swap, &bn, &splits, &per, &tp, &tq);
+  return splits;
+}
+
 // Which kernel sglc_gemm_tc takes for a product whose output a tensor map can address (rows 16-byte
 // aligned; any product of few tokens): 0 the few-token kernel, 1 the many-token kernel with one
 // block a tile, 2 the many-token kernel on pairs of SMs.  (Tests ask, so that the sizes they
 // choose for a kernel do reach it.)
 SGLC_API int sglc_gemm_tc_form(int M, int N, int K, int act) {
   int swap, bn, splits, per, tp, tq;
-  plan(M, N, K, true, &swap, &bn, &splits, &per, &tp, &tq);
+  plan(M, N, K, true, 8, &swap, &bn, &splits, &per, &tp, &tq);       // (the form does not follow the widest cluster)
   if (swap) return 0;
   return (bn == 128 && pair_pays(M, N, K, act, tp, tq)) ? 2 : 1;
 }

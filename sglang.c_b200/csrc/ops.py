@@ -418,6 +418,11 @@ def gemm_tc_kv(a, w, bias, out, cache, slots, n_heads, n_kv_heads, head_dim):
     return True
 
 
+def gemm_tc_shares(M, N, K, widest=16):
+    """Into how many shares of K gemm_tc deals such a product, where the device holds clusters of `widest` blocks."""
+    return build.load("gemm_tc").sglc_gemm_tc_shares(int(M), int(N), int(K), int(widest))
+
+
 def gemm_tc_form(M, N, K, act=None):
     """Which of gemm_tc's kernels a product of these sizes takes: "few" (up to 128 tokens: weights on
     the MMA's 128-row side, split-K over a cluster), "stream" (many tokens, one block a tile) or "pair"

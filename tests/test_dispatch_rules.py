@@ -43,3 +43,17 @@ def test_a_step_with_single_tokens_is_no_step_of_portions(monkeypatch, singles):
     rt.attend(ctx, q, q, q, binding, grp, q, 1, 1, 8, 1.0, None)
     rt.attend_shared(ctx, q, binding, grp, q, 1, 8, 1.0, None)
     assert told == ([0, 0] if singles else [2, 2])
+
+
+@pytest.mark.parametrize("M,N,K,shares", [(1, 768, 3072, 16), (16, 768, 3072, 16), (17, 768, 3072, 8), (16, 768, 3008, 8), (16, 1024, 3072, 8),
+                                          (16, 1024, 3584, 14), (16, 1152, 4608, 15), (16, 1160, 4608, 8), (8, 128, 8200, 15)])
+def test_shares_of_a_long_k(M, N, K, shares):
+    """Clusters of more than eight blocks only where the device holds them, and where they pay."""
+    assert ops.gemm_tc_shares(M, N, K) == shares
+    assert ops.gemm_tc_shares(M, N, K, 8) == 8
+
+
+@pytest.mark.parametrize("M,N,K,shares", [(129, 768, 3072, 8), (256, 768, 3072, 5), (320, 768, 4096, 4), (400, 768, 3072, 3), (512, 768, 3072, 2),
+                                          (256, 1024, 4096, 4), (768, 768, 3072, 2), (800, 768, 3072, 1), (129, 2048, 3072, 3), (512, 768, 2048, 1)])
+def test_shares_of_many_tokens(M, N, K, shares):
+    assert ops.gemm_tc_shares(M, N, K) == shares
