@@ -1140,16 +1140,24 @@ def state_chunks(q, k, v, weights, A_log, out, state, q_start, state_slots, n_re
 DELTA_CHUNKS_MAX_DIM = 64        # key sizes of the chunks of the delta rule and the fixed decay (state_chunks.cu)
 
 
-def delta_chunks_pay(mode, n_tokens, n_requests, max_q_len, n_heads, dim):
+def delta_chunks_pay(mode, n_tokens, n_requests, max_q_len, n_heads, dim, v_dim):
     """Whether a step's delta rule (or recurrence of fixed decay) is worked on in chunks.  A walk takes the time of
-    its longest portion, chunks that of all of them on the whole chip.  Measured, heads of 64, walk against chunks:
-    delta rule, 12 heads, 1 x 128 tokens 30 and 36 us, 8 x 128 51 and 53, 12 x 160 70 and 78, 2 x 192 46 and 39,
-    1 x 256 56 and 37, 2 x 1,024 232 and 80; fixed decay, 3 heads, 1 x 64 tokens 14 and 19, 8 x 100 22 and 20,
-    1 x 128 25 and 19, 2 x 1,024 174 and 21."""
+    its longest portion, longer where more heads and columns walk at once than SMs have room for; chunks that of all (chunk,
+    head, 64 value columns) on the whole chip, and no less than their three launches.  Both in us, fitted to 550 measured
+    steps (1 to 64 heads of 7 to 64, values of 5 to 256, 1 to 16 portions of 64 to 2,000 tokens).  Walk against chunks:
+    delta rule, 12 heads of 64, 1 x 150 tokens 35 and 37, 1 x 256 56 and 37, 8 x 128 50 and 52, 8 x 256 86 and 76, 2 x 1,024
+    227 and 80, 32 heads of 64 x 128, 2 x 1,024 418 and 318, 4 x 512 226 and 320; fixed decay, 3 heads of 64, 1 x 100 29 and 28,
+    2 x 1,024 229 and 30, 64 heads of 64 x 16, 1 x 128 34 and 38, 4 x 512 176 and 226."""
     if dim > DELTA_CHUNKS_MAX_DIM or n_requests > n_tokens // STATE_CHUNK:
         return False
-    work = (n_tokens // STATE_CHUNK + n_requests // 2) * n_heads         # about the (chunk, head) pairs
-    return max_q_len >= (150 + work // 2 if mode == "delta" else 96 + work // 6)
+    pairs = (n_tokens // STATE_CHUNK + n_requests // 2) * n_heads * -(-v_dim // 64)      # about
+    at_once = n_tokens * n_heads * v_dim / (64 * max_q_len)          # heads of 64 columns that walk side by side, on average
+    crowd = 1.0 if at_once < 48 else 1.3 + at_once / 350
+    if mode == "delta":
+        walk, chunks = 3 + 0.208 * max_q_len, max(36, 25 + 0.145 * pairs)
+    else:
+        walk, chunks = (5 + 0.22 * max_q_len) * (1.4 if dim <= 16 else 1.0), max(28, 20 + 0.09 * pairs)
+    return walk * crowd > 1.08 * chunks
 
 
 def delta_chunks_workspace(mode, n_tokens, n_requests, n_heads, v_dim):

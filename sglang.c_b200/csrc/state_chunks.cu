@@ -449,7 +449,11 @@ struct DcArgs {
   int* err;
 };
 
-__device__ __forceinline__ float dc_silu(float v) { return v / (1.0f + expf(-v)); }
+// (a division of zero is a slow one, and rows and columns beyond a tile's are zeros: they divide a one)
+__device__ __forceinline__ float dc_silu(float v) {
+  const float x = v == 0.0f ? 1.0f : v, y = x / (1.0f + expf(-x));
+  return v == 0.0f ? v : y;
+}
 
 // 64 rows of src, columns c0 .. c0 + 63 of rows that end at column n, into dst; zeros outside.
 template <int NT>      // NT: the block's threads

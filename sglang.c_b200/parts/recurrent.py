@@ -71,7 +71,7 @@ def _chunk_bytes(rt, mode, H, D, V):
     return 4 * ops.delta_chunks_workspace(mode, ops.STATE_CHUNK, 1, H, V) // ops.STATE_CHUNK
 
 
-def _form(ctx, T, mode, H, D):
+def _form(ctx, T, mode, H, D, V):
     """How a step's recurrence is worked on: "step" (one token a request, in a pass over the states), "chunks" (long
     portions, side by side) or "walk" (token by token).  In the 32-bit path always the walk: each form has an order
     of additions of its own, and there a request's bits must not depend on what else is in its step."""
@@ -79,13 +79,13 @@ def _form(ctx, T, mode, H, D):
         return "walk"
     if ctx.max_q_len == 1:
         return "step"
-    return "chunks" if ops.delta_chunks_pay(mode, T, ctx.R, ctx.max_q_len, H, D) else "walk"
+    return "chunks" if ops.delta_chunks_pay(mode, T, ctx.R, ctx.max_q_len, H, D, V) else "walk"
 
 
 def _matrix_state(ctx, mode, q, k, v, out, state, H, G, D, V, **kw):
     """The recurrence over the step's tokens."""
     T = out.shape[0]
-    form = _form(ctx, T, mode, H, D)
+    form = _form(ctx, T, mode, H, D, V)
     if form == "step" and ops.delta_step_fits(state, D, V):
         ops.delta_step(mode, q, k, v, out, state, ctx.state_slots, H, G, D, V, **kw)
     elif form == "chunks":
@@ -156,7 +156,7 @@ class GatedDeltaRule(Part):
             + _chunk_bytes(self.rt, "delta", H, D, V)
 
     def launch_form(self, ctx):
-        return _form(ctx, ctx.T, "delta", self.params["n_heads"], self.params["dim"])
+        return _form(ctx, ctx.T, "delta", *(self.params[k] for k in ("n_heads", "dim", "v_dim")))
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params
@@ -216,7 +216,7 @@ class LinearDecayAttention(Part):
         return 4 * (2 * H * D + 2 * H * V) + 4 * H * V + act * H * V + 1024 + _chunk_bytes(self.rt, "decay", H, D, V)
 
     def launch_form(self, ctx):
-        return _form(ctx, ctx.T, "decay", self.params["n_heads"], self.params["dim"])
+        return _form(ctx, ctx.T, "decay", *(self.params[k] for k in ("n_heads", "dim", "v_dim")))
 
     def forward(self, ctx, h, residual, cache, position=None, out=None):
         p = self.params

@@ -57,3 +57,27 @@ def test_shares_of_a_long_k(M, N, K, shares):
                                           (256, 1024, 4096, 4), (768, 768, 3072, 2), (800, 768, 3072, 1), (129, 2048, 3072, 3), (512, 768, 2048, 1)])
 def test_shares_of_many_tokens(M, N, K, shares):
     assert ops.gemm_tc_shares(M, N, K) == shares
+
+
+# (walk and chunks measured, in us, beside each)
+@pytest.mark.parametrize("mode,lens,heads,dim,v_dim,chunks", [
+    ("delta", [150], 12, 64, 64, False),               # 35, 37
+    ("delta", [200], 12, 64, 64, True),                # 45, 37
+    ("delta", [512] * 4, 12, 64, 64, True),            # 158, 75
+    ("delta", [200] * 8, 12, 64, 64, False),           # 72, 75
+    ("delta", [1024] * 2, 12, 64, 64, True),           # 227, 80
+    ("delta", [512] * 4, 16, 32, 32, False),           # 96, 100
+    ("delta", [512] * 4, 32, 64, 128, False),          # 226, 320
+    ("delta", [1024] * 2, 32, 64, 128, True),          # 418, 318
+    ("delta", [200], 12, 65, 64, False),               # (no form in chunks)
+    ("delta", [2] * 30 + [900], 12, 64, 64, False),    # (more requests than chunks)
+    ("decay", [100], 3, 64, 64, False),                # 29, 28
+    ("decay", [128], 3, 64, 64, True),                 # 34, 28
+    ("decay", [134, 133, 133], 32, 64, 128, False),    # 63, 66
+    ("decay", [200, 100, 100], 32, 64, 128, True),     # 87, 62
+    ("decay", [128], 64, 64, 16, False),               # 34, 36
+    ("decay", [512] * 4, 64, 64, 16, False),           # 176, 226
+    ("decay", [100] * 8, 64, 64, 16, False),           # 55, 116
+    ("decay", [1024] * 2, 3, 64, 64, True)])           # 229, 30
+def test_recurrences_go_in_chunks_where_those_are_faster(mode, lens, heads, dim, v_dim, chunks):
+    assert ops.delta_chunks_pay(mode, sum(lens), len(lens), max(lens), heads, dim, v_dim) == chunks
