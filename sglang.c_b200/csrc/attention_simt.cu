@@ -586,13 +586,15 @@ SGLC_API int sglc_attention_f32_form(int T, int H, int D, int max_q_len, int n_p
   return f32_form(T, H, D, max_q_len, n_portions);
 }
 
-template <typename K>
-static int launch_f32(K* kernel, dim3 grid, int threads, size_t smem, const F32Args& a, cudaStream_t stream) {
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <void (*KERNEL)(const F32Args)>
+static int launch_f32(dim3 grid, int threads, size_t smem, const F32Args& a, cudaStream_t stream) {
+  static size_t configured = 48 * 1024;
+  if (smem > configured) {
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
+    configured = smem;
   }
-  return sglc_launch(kernel, grid, dim3(threads), smem, stream, 1, true, a);
+  return sglc_launch(KERNEL, grid, dim3(threads), smem, stream, 1, true, a);
 }
 
 // q: first query element of token 0 (rows q_stride apart, heads side by side); cache: one
@@ -629,12 +631,12 @@ static int attention_simt_run(const void* q, int q_stride, const void* cache,
     a.T = T; a.H = H; a.Hkv = Hkv; a.D = D; a.page_size = page_size; a.scale = scale; a.window = window;
     a.n_pages = n_pages; a.kv_shared = kv_shared; a.err = err;
     if (form == F32_SINGLES)
-      return D <= 64 ? launch_f32(attention_f32_single_kernel<1>, dim3(T, H), 128, f32_single_smem(D), a, stream)
-                     : launch_f32(attention_f32_single_kernel<2>, dim3(T, H), 128, f32_single_smem(D), a, stream);
+      return D <= 64 ? launch_f32<attention_f32_single_kernel<1>>(dim3(T, H), 128, f32_single_smem(D), a, stream)
+                     : launch_f32<attention_f32_single_kernel<2>>(dim3(T, H), 128, f32_single_smem(D), a, stream);
     const size_t smem = ((size_t)2 * 32 * (2 * D + 4) + (size_t)FP_W * (D + 32)) * sizeof(float);
     const dim3 grid(H, (T + FP_W - 1) / FP_W);
-    return D <= 64 ? launch_f32(attention_f32_portion_kernel<2>, grid, 256, smem, a, stream)
-                   : launch_f32(attention_f32_portion_kernel<4>, grid, 256, smem, a, stream);
+    return D <= 64 ? launch_f32<attention_f32_portion_kernel<2>>(grid, 256, smem, a, stream)
+                   : launch_f32<attention_f32_portion_kernel<4>>(grid, 256, smem, a, stream);
   }
   const int W = single ? 1 : 8;
   const size_t smem = ((size_t)32 * (D % 4 == 0 ? D + 4 : D + 1) + (size_t)32 * DV + (size_t)W * D + (size_t)W * 32) * sizeof(float);

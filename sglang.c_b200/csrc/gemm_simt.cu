@@ -586,9 +586,11 @@ template <int MR, int NF, int ST>
 int launch_rows(const SimtArgs& p, cudaStream_t stream) {
   constexpr int smem = ST * (4 * MR + 8 * NF) * PITCH * 4;
   auto* kernel = gemm_simt_rows_kernel<MR, NF, ST>;
-  if (smem > 48 * 1024) {
+  static bool configured = false;
+  if (smem > 48 * 1024 && !configured) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
+    configured = true;
   }
   return sglc_launch(kernel, dim3((p.N + 8 * NF - 1) / (8 * NF), (p.M + 4 * MR - 1) / (4 * MR)), dim3(32), smem, stream, 1,
                      false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K, p.lda, p.ldo, p.act);
@@ -596,8 +598,12 @@ int launch_rows(const SimtArgs& p, cudaStream_t stream) {
 
 int launch_tile(const SimtArgs& p, cudaStream_t stream) {
   constexpr int smem = TILE_ST * (TILE_M + TILE_N) * LPITCH * 4;
-  const cudaError_t e = cudaFuncSetAttribute(gemm_simt_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return (int)e;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_simt_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
   return sglc_launch(gemm_simt_tile_kernel, dim3((p.N + TILE_N - 1) / TILE_N, (p.M + TILE_M - 1) / TILE_M), dim3(128), smem,
                      stream, 1, false, p.A, p.W, p.bias, p.out, p.residual, p.M, p.N, p.K, p.lda, p.ldo, p.act);
 }

@@ -881,6 +881,27 @@ delta_read_kernel(const DcArgs p) {
   }
 }
 
+// (no early start of the later two behind one another: blocks that wait take up the room of running ones unevenly)
+template <bool DELTA>
+static int launch_delta_chunks(const DcArgs& p, dim3 grid, dim3 pass, cudaStream_t stream) {
+  constexpr int smem = 4 * DC_TILE * 4, pass_smem = DELTA ? DC_PASS_RING * DC_TILE * 4 : 0;
+  static bool configured = false;
+  if (!configured) {
+    auto allow = [](auto* kernel, int bytes) {
+      return bytes > 48 * 1024 ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : cudaSuccess;
+    };
+    cudaError_t e = allow(delta_terms_kernel<DELTA>, smem);
+    if (e == cudaSuccess) e = allow(delta_read_kernel<DELTA>, smem);
+    if (e == cudaSuccess) e = allow(delta_pass_kernel<DELTA>, pass_smem);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  int rc = sglc_launch(delta_terms_kernel<DELTA>, grid, dim3(DC_TERM_THREADS), smem, stream, 1, true, p);
+  if (rc == SGLC_OK) rc = sglc_launch(delta_pass_kernel<DELTA>, pass, dim3(SC_THREADS), pass_smem, stream, 1, false, p);
+  if (rc == SGLC_OK) rc = sglc_launch(delta_read_kernel<DELTA>, grid, dim3(SC_THREADS), smem, stream, 1, false, p);
+  return rc;
+}
+
 // gates: the delta rule's [T][2H] (b, then the decays), or null with head_decay [H]: the decay form.  silu_in:
 // silu of q, k and v first.  ws: float, n_chunks * H * (1 + 4096 * (delta rule: 3 + 2 tiles; decay form: 1 + tiles))
 // entries, tiles = ceil(V / 64), n_chunks being at least the chunks of the step.
@@ -912,21 +933,8 @@ SGLC_API int sglc_delta_chunks(const float* q, long long q_stride, const float* 
   auto al = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
   if (!al(ws)) return SGLC_ERR_ARGUMENT;
   p.vec = D % 4 == 0 && V % 4 == 0 && (q_stride | k_stride | v_stride | out_stride) % 4 == 0 && al(q) && al(k) && al(v) && al(out);
-  constexpr int smem = 4 * DC_TILE * 4;
   const dim3 grid(n_chunks, H, tiles), pass(R, H, pieces);
-  auto go = [&](auto* terms, auto* over, auto* read) {
-    cudaFuncSetAttribute(terms, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(read, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    // (no early start behind one another: blocks that wait take up the room of running ones unevenly)
-    const int pass_smem = gates ? DC_PASS_RING * DC_TILE * 4 : 0;
-    cudaFuncSetAttribute(over, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_PASS_RING * DC_TILE * 4);
-    int rc = sglc_launch(terms, grid, dim3(DC_TERM_THREADS), smem, stream, 1, true, p);
-    if (rc == SGLC_OK) rc = sglc_launch(over, pass, dim3(SC_THREADS), pass_smem, stream, 1, false, p);
-    if (rc == SGLC_OK) rc = sglc_launch(read, grid, dim3(SC_THREADS), smem, stream, 1, false, p);
-    return rc;
-  };
-  return gates ? go(delta_terms_kernel<true>, delta_pass_kernel<true>, delta_read_kernel<true>)
-               : go(delta_terms_kernel<false>, delta_pass_kernel<false>, delta_read_kernel<false>);
+  return gates ? launch_delta_chunks<true>(p, grid, pass, stream) : launch_delta_chunks<false>(p, grid, pass, stream);
 }
 
 // Every request brings one token (token r is request r's).  Grid (requests, H, column tiles of SS_COLS); a
