@@ -430,9 +430,8 @@ struct StreamArgs {
   Args b;
   int n_items;        // tokens served x heads
   int n_stages;
-  int n_split;        // blocks (a cluster) that share an item's keys; with more than 1 a cluster has one item
 };
-constexpr int S_MAX_SPLIT = 4;
+constexpr int S_SPLIT = 2;                 // blocks of a cluster that shares items (it then has one item)
 constexpr int S_WARPS = 4;                  // consumer warps; warp S_WARPS produces
 constexpr int S_THREADS = (S_WARPS + 1) * 32;
 constexpr int S_MAX_STAGES = 8;
@@ -454,7 +453,7 @@ __device__ __forceinline__ ItemGeom item_geom(int pos, int window, int ps) {
   return g;
 }
 
-// SPLIT: clusters share items (StreamArgs::n_split above 1); the plain form is compiled without it.
+// SPLIT: clusters share items; the plain form is compiled without it.
 template <int D, bool SPLIT>
 __global__ void __launch_bounds__(S_THREADS)
 attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const StreamArgs sa) {
@@ -478,7 +477,7 @@ attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const
   __shared__ float s_scores[2][S_TILE];     // a stage's scores, written by quarters, read by all
   __shared__ int s_abort;
   __shared__ __align__(8) uint64_t merge_bar;          // block 0 of a cluster: the others' shares are there
-  __shared__ float recs[SPLIT ? (S_MAX_SPLIT - 1) * (D + 2) : 1];  // ... and lie here: (max, sum, D unnormalised results)
+  __shared__ float recs[SPLIT ? (S_SPLIT - 1) * (D + 2) : 1];  // ... and lie here: (max, sum, D unnormalised results)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int H = a.H, G = a.H / a.Hkv, rank = blockIdx.z;
@@ -488,7 +487,7 @@ attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], S_WARPS);
     }
-    if (SPLIT) mbar_init(&merge_bar, (sa.n_split - 1) * S_WARPS);
+    if (SPLIT) mbar_init(&merge_bar, (S_SPLIT - 1) * S_WARPS);
     s_abort = 0;
     mbar_fence_init();
   }
@@ -500,11 +499,11 @@ attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const
   auto shared_item = [&](const ItemGeom& g) { return SPLIT && g.n_tiles > S_WHOLE_TILES; };
   auto first_tile = [&](const ItemGeom& g) {
     if (!shared_item(g)) return SPLIT && rank != 0 ? g.n_tiles : 0;
-    return min(g.n_tiles, rank * ((g.n_tiles + sa.n_split - 1) / sa.n_split));
+    return min(g.n_tiles, rank * ((g.n_tiles + S_SPLIT - 1) / S_SPLIT));
   };
   auto last_tile = [&](const ItemGeom& g) {
     if (!shared_item(g)) return g.n_tiles;
-    return min(g.n_tiles, (rank + 1) * ((g.n_tiles + sa.n_split - 1) / sa.n_split));
+    return min(g.n_tiles, (rank + 1) * ((g.n_tiles + S_SPLIT - 1) / S_SPLIT));
   };
   auto token_of = [&](int item) { int ti = item / H; return a.token_list ? a.token_list[ti] : ti; };
   // A block's items: one of every run of gridDim.x, counted from the front in even runs and from
@@ -794,7 +793,7 @@ attention_decode_stream_kernel(const __grid_constant__ CUtensorMap map_kv, const
         break;
       }
       l_run = warp_sum(l_run);
-      for (int x = 0; x < sa.n_split - 1; x++) {
+      for (int x = 0; x < S_SPLIT - 1; x++) {
         const float* rec = recs + x * (D + 2);
         if (rec[1] == 0.0f) continue;                    // (an empty run of keys; a sum that is no number goes into the result)
         const float m_new = fmaxf(m_run, rec[0]), c0 = ex2(m_run - m_new), c1 = ex2(rec[0] - m_new);
@@ -974,26 +973,26 @@ SGLC_API int sglc_attention_decode_stream(const void* q, int q_stride, void* cac
   if (per_sm > 3) per_sm = 3;
   if (per_sm < 1) per_sm = 1;
   int grid = n_sm * per_sm;
-  // Items that leave half of the resident blocks without work are shared by clusters of two blocks: 208 items of 350 to 700
+  // Items of 64 entries that leave half of the resident blocks without work are shared by clusters of two blocks (of 128 they
+  // would be fewer than come here): 208 items of 350 to 700
   // keys 14.3 -> 9.7 us a launch (28 MB of keys and values, 4.3 us at the copy rate).  An item of up to S_WHOLE_TILES tiles
   // stays with its cluster's first block, and where no item can have more the launch is the plain one (its items
   // have the same bits; a cluster costs it 0.2 to 1.2 us: 192 items of 32 / 100 / 200 keys 4.3 / 5.1 / 7.3 us plain, 5.0 /
   // 6.1 / 7.7 in pairs; from 272 on the pairs win, 8.4 -> 7.6).  So a token's bits follow its own keys and the number of
   // items, and not max_keys.
-  sa.n_split = 1;
   const int most_rows = (window > 0 && window < max_keys ? window + page_size - 1 : max_keys) - 1;
-  if (sa.n_items * 2 <= grid && most_rows > S_WHOLE_TILES * S_TILE) sa.n_split = 2;
-  if (sa.n_split > 1 || grid > sa.n_items) grid = sa.n_items;
-  const bool split = sa.n_split > 1;
-  auto kern = D == 64 ? (split ? attention_decode_stream_kernel<64, true> : attention_decode_stream_kernel<64, false>)
-                      : (split ? attention_decode_stream_kernel<128, true> : attention_decode_stream_kernel<128, false>);
-  static size_t configured[4] = {0, 0, 0, 0};
-  size_t& conf = configured[(D == 64 ? 0 : 2) + (split ? 1 : 0)];
+  const bool split = D == 64 && sa.n_items * 2 <= grid && most_rows > S_WHOLE_TILES * S_TILE;
+  if (split || grid > sa.n_items) grid = sa.n_items;
+  auto kern = split ? attention_decode_stream_kernel<64, true>
+              : D == 64 ? attention_decode_stream_kernel<64, false>
+                        : attention_decode_stream_kernel<128, false>;
+  static size_t configured[3] = {0, 0, 0};
+  size_t& conf = configured[split ? 2 : D == 64 ? 0 : 1];
   if (smem > 48 * 1024 && smem > conf) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     conf = smem;
   }
-  return sglc_launch(kern, dim3(grid, 1, sa.n_split), dim3(S_THREADS), smem, stream, sa.n_split, true, mkv, sa);
+  return sglc_launch(kern, dim3(grid, 1, split ? S_SPLIT : 1), dim3(S_THREADS), smem, stream, split ? S_SPLIT : 1, true, mkv, sa);
 }
