@@ -13,6 +13,8 @@
 // memory (a block of eight consecutive tokens of a prompt portion reads them once instead of
 // eight times: the reference's kernel, one block per token, reads them per token).  This is the
 // kernel of the 32-bit path and the general fallback of the bfloat16 path.
+#include <limits.h>
+
 #include <type_traits>
 
 #include "common.cuh"
@@ -285,7 +287,7 @@ __device__ __forceinline__ const float* f32_row(const F32Args& a, const int* bt,
 // an SM: 194 us.  The last tokens of a prompt, which see the most keys, go first.
 constexpr int FP_Q = 4, FP_W = 8 * FP_Q;
 template <int NA>      // head sizes up to 32 NA
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 attention_f32_portion_kernel(const F32Args a) {
   extern __shared__ __align__(16) float smem[];
   __shared__ int s_req[FP_W], s_lo[FP_W], s_pos[FP_W];
@@ -399,38 +401,49 @@ attention_f32_portion_kernel(const F32Args a) {
 #pragma unroll
           for (int n = 0; n < NA; n++)
             if (on[i]) acc[i][n] *= corr[i];
-        // (A tile that some of the warp's tokens see in part: their sums leave the other keys out, for the weight zero times an
-        // infinite value is not zero.)
-        auto add_values = [&](auto whole) {
-#pragma unroll 2
-          for (int j = 0; j < 32; j += 4) {
-            float4 p4[FP_Q];
+        // Four keys' values at a time.  In a tile that some of the warp's tokens see in part, their sums leave the other keys
+        // out (the weight zero times an infinite value is not zero), and keys that none of them sees are passed over.
+        auto add_four = [&](int j, auto whole) {
+          float4 p4[FP_Q];
 #pragma unroll
-            for (int i = 0; i < FP_Q; i++) p4[i] = *reinterpret_cast<const float4*>(pv + i * 32 + j);
+          for (int i = 0; i < FP_Q; i++) p4[i] = *reinterpret_cast<const float4*>(pv + i * 32 + j);
 #pragma unroll
-            for (int n = 0; n < NA; n++) {
-              const int d = min(lane + 32 * n, D - 1);                  // (lanes beyond the head size: not stored)
-              const float v0 = vs[j * D + d], v1 = vs[(j + 1) * D + d], v2 = vs[(j + 2) * D + d], v3 = vs[(j + 3) * D + d];
+          for (int n = 0; n < NA; n++) {
+            const int d = min(lane + 32 * n, D - 1);                    // (lanes beyond the head size: not stored)
+            const float v0 = vs[j * D + d], v1 = vs[(j + 1) * D + d], v2 = vs[(j + 2) * D + d], v3 = vs[(j + 3) * D + d];
 #pragma unroll
-              for (int i = 0; i < FP_Q; i++)
-                if (on[i]) {
-                  const int key4 = key0 + j;
-                  auto sees = [&](int e) { return decltype(whole)::value || (key4 + e >= my_lo[i] && key4 + e <= my_pos[i]); };
-                  float x = acc[i][n];
-                  if (sees(0)) x = fmaf(p4[i].x, v0, x);
-                  if (sees(1)) x = fmaf(p4[i].y, v1, x);
-                  if (sees(2)) x = fmaf(p4[i].z, v2, x);
-                  if (sees(3)) x = fmaf(p4[i].w, v3, x);
-                  acc[i][n] = x;
-                }
-            }
+            for (int i = 0; i < FP_Q; i++)
+              if (on[i]) {
+                const int key4 = key0 + j;
+                auto sees = [&](int e) { return decltype(whole)::value || (key4 + e >= my_lo[i] && key4 + e <= my_pos[i]); };
+                float x = acc[i][n];
+                if (sees(0)) x = fmaf(p4[i].x, v0, x);
+                if (sees(1)) x = fmaf(p4[i].y, v1, x);
+                if (sees(2)) x = fmaf(p4[i].z, v2, x);
+                if (sees(3)) x = fmaf(p4[i].w, v3, x);
+                acc[i][n] = x;
+              }
           }
         };
-        bool whole = true;
+        int any_lo = INT_MAX, any_pos = -1, all_lo = 0, all_pos = INT_MAX;       // keys that some, that all of the tokens see
 #pragma unroll
-        for (int i = 0; i < FP_Q; i++) whole = whole && (!on[i] || (key0 >= my_lo[i] && key0 + 31 <= my_pos[i]));
-        if (whole) add_values(std::true_type{});
-        else add_values(std::false_type{});
+        for (int i = 0; i < FP_Q; i++)
+          if (on[i]) {
+            any_lo = min(any_lo, my_lo[i]); any_pos = max(any_pos, my_pos[i]);
+            all_lo = max(all_lo, my_lo[i]); all_pos = min(all_pos, my_pos[i]);
+          }
+        if (key0 >= all_lo && key0 + 31 <= all_pos) {
+#pragma unroll 2
+          for (int j = 0; j < 32; j += 4) add_four(j, std::true_type{});
+        } else {
+#pragma unroll 1
+          for (int j = 0; j < 32; j += 4) {
+            const int key4 = key0 + j;
+            if (key4 + 3 < any_lo || key4 > any_pos) continue;
+            if (key4 >= all_lo && key4 + 3 <= all_pos) add_four(j, std::true_type{});
+            else add_four(j, std::false_type{});
+          }
+        }
         __syncwarp();
       }
       __syncthreads();                                // everybody is done with tile kt: the next but one may come
