@@ -449,11 +449,7 @@ struct DcArgs {
   int* err;
 };
 
-// (a division of zero is a slow one, and rows and columns beyond a tile's are zeros: they divide a one)
-__device__ __forceinline__ float dc_silu(float v) {
-  const float x = v == 0.0f ? 1.0f : v, y = x / (1.0f + expf(-x));
-  return v == 0.0f ? v : y;
-}
+__device__ __forceinline__ float dc_silu(float v) { return v / (1.0f + expf(-v)); }
 
 // 64 rows of src, columns c0 .. c0 + 63 of rows that end at column n, into dst; zeros outside.
 template <int NT>      // NT: the block's threads
@@ -474,9 +470,17 @@ __device__ __forceinline__ void dc_stage(const float* src, long long stride, int
 __device__ __forceinline__ void dc_stage64(const float* src, float* dst) {        // a whole tile of the workspace
   for (int x = threadIdx.x; x < 64 * 16; x += blockDim.x) copy16(dst + (x >> 4) * DC_LD + (x & 15) * 4, src + x * 4, true);
 }
+// (rows and columns beyond a tile's are zeros and stay so: a division of zero is a slow one)
 template <int NT>
-__device__ __forceinline__ void dc_silu_tile(float* t) {
-  for (int x = threadIdx.x; x < 64 * 64; x += NT) t[(x >> 6) * DC_LD + (x & 63)] = dc_silu(t[(x >> 6) * DC_LD + (x & 63)]);
+__device__ __forceinline__ void dc_silu_tile(float* t, int rows, int cols) {
+  if (rows >= 64 && cols >= 64) {
+    for (int x = threadIdx.x; x < 64 * 64; x += NT) t[(x >> 6) * DC_LD + (x & 63)] = dc_silu(t[(x >> 6) * DC_LD + (x & 63)]);
+    return;
+  }
+  for (int x = threadIdx.x; x < 64 * 64; x += NT) {
+    float* e = t + (x >> 6) * DC_LD + (x & 63);
+    if ((x >> 6) < rows && (x & 63) < cols) *e = dc_silu(*e);
+  }
 }
 // A sum of short sums rounds less than one long one, as the walk's partial sums do: 64 entries go eight at a time, in
 // pairs; and what a sum is added to, it is added to once.  (Against 64 bits, six draws of gates, keys and
@@ -624,9 +628,9 @@ delta_terms_kernel(const DcArgs p) {
   copies_wait<0>();
   __syncthreads();
   if (p.silu_in) {
-    dc_silu_tile<DC_TERM_THREADS>(ks);
-    if (z == 0) dc_silu_tile<DC_TERM_THREADS>(qs);
-    dc_silu_tile<DC_TERM_THREADS>(vs);
+    dc_silu_tile<DC_TERM_THREADS>(ks, ck.len, p.D);
+    if (z == 0) dc_silu_tile<DC_TERM_THREADS>(qs, ck.len, p.D);
+    dc_silu_tile<DC_TERM_THREADS>(vs, ck.len, p.V - z * 64);
     __syncthreads();
   }
   const size_t at = ((size_t)c * p.H + h) * 4096, atz = (((size_t)c * p.H + h) * p.tiles + z) * 4096;
@@ -840,8 +844,8 @@ delta_read_kernel(const DcArgs p) {
     for (int i = 0; i < 64; i++) { r *= gs[i]; cs[i] = r; }
   }
   if (p.silu_in) {
-    dc_silu_tile<SC_THREADS>(qs);
-    if (!DELTA) dc_silu_tile<SC_THREADS>(us);
+    dc_silu_tile<SC_THREADS>(qs, ck.len, p.D);
+    if (!DELTA) dc_silu_tile<SC_THREADS>(us, ck.len, p.V - z * 64);
     __syncthreads();
   }
   if (DELTA) {                                           // U0 - W S
