@@ -19,8 +19,8 @@ ROWS, ROWS_WIDE, TILE, PAIR, PAIR_WIDE, FEW, BLOCK = 1, 2, 3, 4, 5, 6, 7
                                    (16, 10300, 36), (24, 8200, 36), (64, 65, 772), (65, 63, 128),
                                    (129, 200, 1028), (200, 130, 16)])
 def test_gemm_simt_forms_give_the_same_bits(M, N, K):
-    """Remainders of rows, features and k in every form; the residual form; strided rows.  Error: K roundings of
-    a sum of about sqrt(K) in size, each half a unit: below 1e-7 K."""
+    """Remainders of rows, features and k in every form, and the sizes at which the rule takes each of the few-row forms; the
+    residual form; strided rows.  Error: K roundings of 2^-24 of sums that stay below sum |a w|, a random walk of them."""
     from sglang_c_b200.csrc import build
     ops, lib = _ops(), build.load("gemm_simt")
     wide = _rand(M, K + 12, seed=M)
@@ -39,7 +39,8 @@ def test_gemm_simt_forms_give_the_same_bits(M, N, K):
             assert torch.equal(out, first), form
     finally:
         lib.sglc_gemm_simt_set_form(0)
-    assert float((first.double() - ref).abs().max()) < 1e-7 * K * math.sqrt(K) + 1e-6
+    bound = float((a.double().abs() @ w.double().abs().t() + bias.double().abs()).max()) * 2.0 ** -24 * (K + 1) ** 0.5
+    assert float((first.double() - ref).abs().max()) < bound
 
 
 # -- 32-bit attention ------------------------------------------------------------------------------
@@ -132,6 +133,47 @@ def test_prompt_attention_follows_a_growing_maximum(D, window, grow):
     assert float((out.double().cpu() - ref).abs().max()) < 2.5e-2
 
 
+@pytest.mark.parametrize("H,Hkv,D", [(40, 1, 64), (20, 2, 128)])
+def test_prompt_attention_of_many_query_tiles(H, Hkv, D):
+    """More query tiles than half of the blocks that run at once: tiles of five key tiles are split, shorter ones are not."""
+    ops = _ops()
+    lens, q_lens, ps = [600, 129, 40, 700], [130, 129, 40, 200], 16
+    c = _paged_case(lens, q_lens, H, Hkv, D, ps, torch.bfloat16, seed=H)
+    q_start = torch.tensor(np.concatenate([[0], np.cumsum(q_lens)]), dtype=torch.int32, device=DEV)
+    kv_len = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    out = torch.full((sum(q_lens), H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    scale = 1.0 / math.sqrt(D)
+    ops.attention_prefill_tc(c["q"], c["cache"], c["bt"], q_start, kv_len, out, H, scale, None, len(lens), max(q_lens))
+    # bfloat16 weights and results of size below one: 2^-8 each
+    assert float((out.double().cpu() - _attention_reference(c, H, Hkv, D, scale, None)).abs().max()) < 1.2e-2
+
+
+@pytest.mark.parametrize("kv_shared", [False, True])
+@pytest.mark.parametrize("q_lens", [[1, 1, 1, 44], [70, 1, 1, 1, 1], [1] * 33 + [129] + [1] * 3, [1] * 40 + [2], [3] + [1] * 31 + [5] + [1] * 31 + [140],
+                                    [1, 9, 1, 9]])
+def test_a_launch_for_the_portions_alone(q_lens, kv_shared):
+    """The number of single tokens is known: portions first, last, beyond the 32nd and the 64th request and between single
+    tokens are all found, and no single token's row is written."""
+    ops = _ops()
+    H, D, ps = 3, 64, 16
+    lens = [n + (37 * r) % 150 for r, n in enumerate(q_lens)]
+    c = _paged_case(lens, q_lens, H, 1, D, ps, torch.bfloat16, seed=len(q_lens))
+    if kv_shared:                                       # (rows that are keys and values at once)
+        c["cache"], c["Vs"] = c["cache"][:, :1].contiguous(), c["Ks"]
+    starts = np.concatenate([[0], np.cumsum(q_lens)])
+    q_start = torch.tensor(starts, dtype=torch.int32, device=DEV)
+    kv_len = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    out = torch.full((sum(q_lens), H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    singles = [int(s) for s, n in zip(starts, q_lens) if n == 1]
+    ops.attention_prefill_tc(c["q"], c["cache"], c["bt"], q_start, kv_len, out, H, 0.1, None, len(lens), max(q_lens), skip_single=len(singles),
+                             kv_shared=kv_shared)
+    rows = torch.ones(sum(q_lens), dtype=torch.bool)
+    rows[singles] = False
+    assert bool(torch.isnan(out[~rows]).all())
+    ref = _attention_reference(c, H, 1, D, 0.1, None)
+    assert float((out.double().cpu() - ref)[rows].abs().max()) < 2e-2
+
+
 # -- single tokens: items shared by clusters -------------------------------------------------------------
 @pytest.mark.parametrize("T,H,Hkv,D,window", [(9, 12, 12, 64, None), (13, 16, 4, 64, None), (18, 12, 12, 64, 200), (6, 16, 16, 128, None),
                                               (3, 16, 2, 64, None)])
@@ -197,11 +239,13 @@ def _walk(mode, q, k, v, gates, decay, H, G, D, V, S):
     return out.reshape(n, H * V), S
 
 
+@pytest.mark.parametrize("silu", [False, True])
 @pytest.mark.parametrize("mode,H,G,D,V,rate", [("delta", 4, 2, 64, 64, 0.1), ("delta", 3, 3, 40, 100, 0.002), ("delta", 2, 1, 7, 9, 3.0),
                                                ("decay", 2, 2, 64, 64, 0.05), ("decay", 2, 2, 33, 70, 0.5)])
-def test_recurrences_in_chunks(mode, H, G, D, V, rate):
+def test_recurrences_in_chunks(mode, H, G, D, V, rate, silu):
     """Portions of 1 to 200 tokens over shuffled slots: chunk edges, states carried in, decays near one, far from it
-    and zero, sizes no vector load fits.  The chunks may not be further off than 2 x the walk token by token."""
+    and zero, sizes no vector load fits, silu of the inputs.  The chunks may not be further off than 2 x the walk token by
+    token."""
     ops = _ops()
     g = torch.Generator().manual_seed(D)
     lens = [200, 1, 64, 65, 127]
@@ -215,7 +259,8 @@ def test_recurrences_in_chunks(mode, H, G, D, V, rate):
     S0 = torch.randn(R + 2, H, D, V, generator=g).to(DEV)
     starts, slots = np.concatenate([[0], np.cumsum(lens)]), [3, 0, 6, 1, 4]
     i32 = lambda x: torch.tensor(np.asarray(x), dtype=torch.int32, device=DEV)      # noqa: E731
-    kw = dict(gates=gates) if mode == "delta" else dict(head_decay=decay)
+    kw = dict(gates=gates, silu_in=silu) if mode == "delta" else dict(head_decay=decay, silu_in=silu)
+    act = (lambda x: torch.nn.functional.silu(x.double())) if silu else (lambda x: x)
     got = {}
     for way in ("walk", "chunks"):
         S, o = S0.clone(), torch.full((T, H * V), float("nan"), device=DEV)
@@ -227,7 +272,7 @@ def test_recurrences_in_chunks(mode, H, G, D, V, rate):
         got[way] = (o, S)
     for r, slot in enumerate(slots):
         at = slice(starts[r], starts[r + 1])
-        want, state = _walk(mode, q[at], k[at], v[at], gates[at], decay, H, G, D, V, S0[slot].double())
+        want, state = _walk(mode, act(q[at]), act(k[at]), act(v[at]), gates[at], decay, H, G, D, V, S0[slot].double())
         for i, (ref, pick) in enumerate(((want, lambda t: t[0][at]), (state, lambda t: t[1][slot]))):
             err = {w: float((pick(got[w]).double() - ref).norm() / ref.norm()) for w in got}
             assert err["chunks"] < max(2.0 * err["walk"], 5e-7), (r, i, err)
@@ -403,6 +448,26 @@ def test_cache_writing_projection_over_a_long_k():
     got = torch.cat([out[:, :H * D].double()] + [cache[slots.long() // ps, i, 0, slots.long() % ps].double() for i in range(2)], 1)
     # half a unit of bfloat16 a value and the 32-bit sums before it
     assert float((got - want).abs().max()) < float(want.abs().max()) * 2.0 ** -8
+
+
+@pytest.mark.parametrize("M,N,K,shares", [(129, 768, 3072, 8), (170, 768, 3104, 7), (160, 1000, 3072, 6), (250, 768, 3072, 5), (320, 700, 4096, 4),
+                                          (400, 768, 3080, 3), (129, 2048, 2120, 3), (768, 768, 3072, 2), (4700, 60, 2304, 2)])
+def test_many_tokens_over_a_long_k(M, N, K, shares):
+    """K dealt to two to eight blocks, tokens off the edges of tiles of 32, features off those of 128."""
+    ops = _ops()
+    assert ops.gemm_tc_shares(M, N, K) == shares
+    g = torch.Generator().manual_seed(M)
+    a, w = (torch.randn(n, K, generator=g).mul_(s).to(DEV, torch.bfloat16) for n, s in ((M, 1.0), (N, 0.02)))
+    bias, x = torch.randn(N, generator=g).to(DEV), torch.randn(M, N, generator=g).to(DEV)
+    plain = a.double() @ w.double().T + bias.double()
+    want = x.double() + plain
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.gemm_tc(a, w, bias, out=out)
+    ops.gemm_tc(a, w, bias, residual=x)
+    # 32-bit sums of K products: K roundings of 2^-24 of sums that stay below sum |a w|, a random walk of them
+    bound = float((a.double().abs() @ w.double().abs().T).max()) * 2.0 ** -24 * K ** 0.5
+    assert float((x.double() - want).abs().max()) < bound
+    assert float((out.double() - plain).abs().max()) < float(plain.abs().max()) * 2.0 ** -8      # half a unit of bfloat16
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 3072), (16, 1152, 4608), (5, 100, 3080), (16, 768, 8200), (17, 768, 3072), (16, 1160, 3072)])

@@ -604,7 +604,8 @@ def test_attention_decode_writes_new_keys_itself(case_id):
     assert torch.equal(holed, want_cache)
 
 
-def test_attention_kernels_share_a_mixed_step():
+@pytest.mark.parametrize("known", [False, True])
+def test_attention_kernels_share_a_mixed_step(known):
     """Portions of some requests beside single tokens of others: the tile kernel serves the
     portions and skips the single tokens, the split-key kernel serves exactly those."""
     ops = _ops()
@@ -618,7 +619,7 @@ def test_attention_kernels_share_a_mixed_step():
     token_list = torch.tensor(singles + [0, 0], dtype=torch.int32, device=DEV)
     out = torch.full((T, H * D), float("nan"), dtype=torch.bfloat16, device=DEV)
     ops.attention_prefill_tc(c["q"], c["cache"], c["bt"], q_start, kv_len, out, H, scale, None, len(lens),
-                             max(q_lens), skip_single=True)
+                             max(q_lens), skip_single=len(singles) if known else True)
     torch.cuda.synchronize()
     assert all(bool(torch.isnan(out[t]).all()) for t in singles)          # left for the other kernel
     ops.attention_decode(c["q"], c["cache"], c["bt"], c["token_req"], c["positions"], out, H, scale, None,
