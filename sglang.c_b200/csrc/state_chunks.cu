@@ -471,12 +471,17 @@ __device__ __forceinline__ void dc_stage64(const float* src, float* dst) {      
   for (int x = threadIdx.x; x < 64 * 16; x += blockDim.x) copy16(dst + (x >> 4) * DC_LD + (x & 15) * 4, src + x * 4, true);
 }
 // (rows and columns beyond a tile's are zeros and stay so: a division of zero is a slow one)
-template <int NT>
+// FAST: whole tiles a few entries at a time; without it the least code, for the delta rule, which no layer asks for a silu:
+// its kernels run straight through code that has to be fetched (the terms of 2 x 1,024 tokens in a layer's chain of
+// launches 38.2 us, 44.8 with both loops unrolled).
+template <int NT, bool FAST>
 __device__ __forceinline__ void dc_silu_tile(float* t, int rows, int cols) {
-  if (rows >= 64 && cols >= 64) {
+  if (FAST && rows >= 64 && cols >= 64) {
+#pragma unroll 4
     for (int x = threadIdx.x; x < 64 * 64; x += NT) t[(x >> 6) * DC_LD + (x & 63)] = dc_silu(t[(x >> 6) * DC_LD + (x & 63)]);
     return;
   }
+#pragma unroll 1
   for (int x = threadIdx.x; x < 64 * 64; x += NT) {
     float* e = t + (x >> 6) * DC_LD + (x & 63);
     if ((x >> 6) < rows && (x & 63) < cols) *e = dc_silu(*e);
@@ -628,9 +633,9 @@ delta_terms_kernel(const DcArgs p) {
   copies_wait<0>();
   __syncthreads();
   if (p.silu_in) {
-    dc_silu_tile<DC_TERM_THREADS>(ks, ck.len, p.D);
-    if (z == 0) dc_silu_tile<DC_TERM_THREADS>(qs, ck.len, p.D);
-    dc_silu_tile<DC_TERM_THREADS>(vs, ck.len, p.V - z * 64);
+    dc_silu_tile<DC_TERM_THREADS, !DELTA>(ks, ck.len, p.D);
+    if (z == 0) dc_silu_tile<DC_TERM_THREADS, !DELTA>(qs, ck.len, p.D);
+    dc_silu_tile<DC_TERM_THREADS, !DELTA>(vs, ck.len, p.V - z * 64);
     __syncthreads();
   }
   const size_t at = ((size_t)c * p.H + h) * 4096, atz = (((size_t)c * p.H + h) * p.tiles + z) * 4096;
@@ -844,8 +849,8 @@ delta_read_kernel(const DcArgs p) {
     for (int i = 0; i < 64; i++) { r *= gs[i]; cs[i] = r; }
   }
   if (p.silu_in) {
-    dc_silu_tile<SC_THREADS>(qs, ck.len, p.D);
-    if (!DELTA) dc_silu_tile<SC_THREADS>(us, ck.len, p.V - z * 64);
+    dc_silu_tile<SC_THREADS, !DELTA>(qs, ck.len, p.D);
+    if (!DELTA) dc_silu_tile<SC_THREADS, !DELTA>(us, ck.len, p.V - z * 64);
     __syncthreads();
   }
   if (DELTA) {                                           // U0 - W S
