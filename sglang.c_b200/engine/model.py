@@ -89,8 +89,9 @@ class Model:
         for layer in self.layers:
             parts += [layer.block] + list(layer.parts.values())
         self.graph_safe = all(getattr(p, "graph_safe", True) for p in parts)
-        self._formed = [m for m in (layer.the_mixer for layer in self.layers)
-                        if isinstance(m, Part) and type(m).launch_form is not Part.launch_form]
+        # one mixer of each kind and parameters speaks for its like
+        self._formed = list({(type(m), repr(m.params)): m for m in (layer.the_mixer for layer in self.layers)
+                             if isinstance(m, Part) and type(m).launch_form is not Part.launch_form}.values())
         self.largest_layer_matrix = 0     # elements of the largest matrix a layer holds (set by load)
 
     def load(self, model_dir):
