@@ -186,7 +186,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_kv, const Ar
   // Every warp walks its own keys with a maximum and a sum of its own, four groups of rows at a time so that
   // their reads, their sums over the lanes and their exponentials do not wait for one another; the warps meet once.
   // (With the block's maximum and sum taken first, between barriers, and one group at a time a launch took 7.9 us in
-  // the chain of a step of eight requests at context 512, now 6.0, and 5.8 for one request, now 4.9.  What is left is a
+  // the chain of a step of eight requests at context 512, now 5.9, and 5.8 for one request, now 4.8.  What is left is a
   // chain: the dependency's return, the query's way from L2, two passes, the cluster's exchange.)
   // A pass takes as many groups as are left, up to four: one of four for the last few keys costs their instructions all the
   // same (eight requests of 320 keys, 80 a block: 6.3 us instead of 5.8; of 272, 5.8 instead of 5.5).

@@ -204,10 +204,9 @@ gemm_simt_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, 
 // dependent multiply-adds (four clocks each), which is what bounds the narrow products.  A block is one
 // warp with 4 MR rows of 8 NF features, a lane MR x NF outputs, with no barrier between warps, and few
 // instructions beside the chain.  Tiles of 64 k come through a ring of ST stages by asynchronous
-// 16-byte copies; the first stages' weights are asked for before the wait for the kernel ahead.  A
-// 16-byte read costs one pass for the eight features all quarters of the warp share and four for the
-// four rows (rows lie 68 floats apart: no bank conflicts).  k ascending, one accumulator: the same bits
-// as the kernels above.
+// 16-byte copies.  A 16-byte read costs one pass for the eight features all quarters of the warp share and
+// four for the four rows (rows lie 68 floats apart: no bank conflicts).  k ascending, one accumulator: the
+// same bits as the kernels above.
 // 8 rows: 768 columns 7.4 -> 4.8 us, over K 3,072 23.6 -> 12.6 us (its chain alone 6.4), 50,257 columns 84 -> 44 us (154 MB:
 // 24 us at the copy rate).
 constexpr int SK = 64, PITCH = SK + 4;

@@ -423,8 +423,8 @@ SGLC_API int sglc_state_chunks(const float* q, long long q_stride, const float* 
 // (matrix_state.cu) is a chain of T dependent steps of 215 ns with most of the GPU idle; this does about twice
 // the multiply-adds with every SM at work.  2 x 1,024 tokens: delta rule, 12 heads of 64, 232 -> 80 us (38, 24 and 21:
 // the first bound by shared memory reads and the chain of the triangular system, the second a chain of 16 chunks, 1.4
-// us each); fixed decay, 3 heads, 174 -> 21.  Key sizes up to 64 (three blocks' tiles then fit into an SM's shared
-// memory); value columns in tiles of 64.
+// us each); fixed decay with silu of its inputs, 3 heads, 174 -> 35 (20, 5 and 10).  Key sizes up to 64 (three blocks'
+// tiles then fit into an SM's shared memory); value columns in tiles of 64.
 constexpr int DC_LD = 64 + SC_PAD, DC_TILE = 64 * DC_LD;
 constexpr int DC_PASS_COLS = 8, DC_PASS_RING = 4;
 constexpr int DC_TERM_THREADS = 128;      // (three blocks an SM: 34 chunks of 12 heads then take one round)
