@@ -244,6 +244,58 @@ def gemm_simt(a, w, bias, out=None, residual=None, act=None):
     _check(lib, code, f"gemm_simt M={M} N={N} K={K}")
 
 
+def gemm_f32_supported(a, w):
+    """Whether the 32-bit path takes gemm_f32 for this product.  (Nothing here follows the number of rows, so that a
+    token's results do not either.)"""
+    return a.dtype == torch.float32 and w.dtype == torch.float32 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 \
+        and a.stride(1) == 1 and w.is_contiguous() \
+        and bool(build.load("gemm_f32").sglc_gemm_f32_supports(w.shape[0], w.shape[1], a.stride(0)))
+
+
+def gemm_f32(a, w, bias, out=None, residual=None, act=None):
+    """gemm_simt's product for 32-bit operands on the tensor cores, each number as three bfloat16 pieces: out =
+    act(a·wᵀ + bias), or residual += act(a·wᵀ + bias).  An output's bits do not depend on the number of rows."""
+    _need_cuda(a, w, bias, out, residual)
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K or not w.is_contiguous() or a.stride(1) != 1 or a.dtype != torch.float32 or w.dtype != torch.float32:
+        raise KernelError(f"gemm_f32: a {tuple(a.shape)}/{a.dtype} and w {tuple(w.shape)}/{w.dtype} do not match")
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
+        raise KernelError("gemm_f32: bias must be a float32 vector of N")
+    dst = residual if residual is not None else out
+    if dst is None or dst.shape[0] < M or dst.shape[1] != N or dst.stride(1) != 1 or dst.dtype != torch.float32:
+        raise KernelError("gemm_f32: output does not match a float32 [M,N]")
+    lib = build.load("gemm_f32")
+    code = lib.sglc_gemm_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), _ptr(residual), M, N, K, a.stride(0), dst.stride(0),
+                             _act(act), _ptr(tc_error_flag(a.device)), _stream())
+    _check(lib, code, f"gemm_f32 M={M} N={N} K={K}")
+
+
+def gemm_f32_kv(a, w, bias, out, cache, slots, n_heads, n_kv_heads, head_dim):
+    """gemm_f32's query/key/value projection with the cache write in its epilogue: out[:, :n_heads*head_dim] takes the
+    queries; keys and values go straight into the paged cache [n_pages, 2, n_kv_heads, page_size, head_dim] at
+    slots[token].  Returns False, having launched nothing, for products gemm_f32 does not take."""
+    _need_cuda(a, w, bias, out, cache, slots)
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K or not gemm_f32_supported(a, w) or out.dtype != torch.float32 or cache.dtype != torch.float32 \
+            or out.shape[0] < M or out.shape[1] != N or out.stride(1) != 1 or not cache.is_contiguous() \
+            or N != (n_heads + 2 * n_kv_heads) * head_dim:
+        return False
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
+        raise KernelError("gemm_f32_kv: bias must be a float32 vector of N")
+    _i32(slots, "slots")
+    n_pages, two, Hkv, page_size, D = cache.shape
+    if two != 2 or Hkv != n_kv_heads or D != head_dim or slots.numel() < M:
+        raise KernelError("gemm_f32_kv: the cache or the slots do not match the projection")
+    lib = build.load("gemm_f32")
+    code = lib.sglc_gemm_f32_kv(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), M, N, K, a.stride(0), out.stride(0), _ptr(cache),
+                                _ptr(slots), n_heads * head_dim, n_kv_heads, head_dim, page_size, n_pages,
+                                _ptr(tc_error_flag(a.device)), _stream())
+    _check(lib, code, f"gemm_f32_kv M={M} N={N} K={K}")
+    return True
+
+
 def kv_write(k_src, v_src, cache, slots, n_kv_heads, head_dim):
     """Scatter keys and values of T tokens into one layer's pages.
     k_src, v_src: [T, n_kv_heads*head_dim] views (row stride free); cache:

@@ -31,6 +31,11 @@ typedef int (*fn_layernorm)(const float*, const int*, const float*, const float*
                             cudaStream_t);
 typedef int (*fn_gemm_simt)(const void*, const void*, const float*, void*, float*, int, int, int, int, int, int, int,
                             int, cudaStream_t);
+typedef int (*fn_gemm_f32_supports)(int, int, int);
+typedef int (*fn_gemm_f32)(const float*, const float*, const float*, float*, float*, int, int, int, int, int, int, int*,
+                           cudaStream_t);
+typedef int (*fn_gemm_f32_kv)(const float*, const float*, const float*, float*, int, int, int, int, int, float*, const int*,
+                              int, int, int, int, int, int*, cudaStream_t);
 typedef int (*fn_gemm_tc)(const void*, const void*, const float*, void*, float*, int, int, int, int, int, int, int,
                           int*, cudaStream_t);
 typedef int (*fn_gemm_tc_kv)(const void*, const void*, const float*, void*, int, int, int, int, int, int, void*,
@@ -65,6 +70,9 @@ struct Bound {
   fn_embed embed;
   fn_layernorm layernorm;
   fn_gemm_simt gemm_simt;
+  fn_gemm_f32_supports gemm_f32_supports;
+  fn_gemm_f32 gemm_f32;
+  fn_gemm_f32_kv gemm_f32_kv;
   fn_gemm_tc gemm_tc;
   fn_gemm_tc_kv gemm_tc_kv;
   fn_gemm_few_supports gemm_few_supports;
@@ -80,7 +88,7 @@ struct Bound {
   fn_attention_decode_stream attention_decode_stream;
 } g = {};
 
-const char* const NAMES[] = {"sglc_embed", "sglc_layernorm", "sglc_gemm_simt", "sglc_gemm_tc", "sglc_gemm_tc_kv",
+const char* const NAMES[] = {"sglc_embed", "sglc_layernorm", "sglc_gemm_simt", "sglc_gemm_f32_supports", "sglc_gemm_f32", "sglc_gemm_f32_kv", "sglc_gemm_tc", "sglc_gemm_tc_kv",
                              "sglc_gemm_few_supports", "sglc_gemm_few", "sglc_kv_write", "sglc_attention_simt",
                              "sglc_attention_prefill_tc", "sglc_attention_decode_splits",
                              "sglc_attention_decode_scratch", "sglc_attention_decode", "sglc_attention_decode_tma",
@@ -136,6 +144,12 @@ struct Walk {
       }
       check(g.gemm_tc(a, l.w, l.bias, out, residual, M, l.N, l.K, lda, ldo, out_f32 ? 1 : 0, act, s.tc_err, s.stream),
             "gemm_tc");
+      return;
+    }
+    if (!m.bf16 && ((uintptr_t)a & 15) == 0 && ((uintptr_t)l.w & 15) == 0 && g.gemm_f32_supports(l.N, l.K, lda)) {
+      check(g.gemm_f32((const float*)a, (const float*)l.w, l.bias, (float*)out, residual, M, l.N, l.K, lda, ldo, act, s.tc_err,
+                       s.stream),
+            "gemm_f32");
       return;
     }
     const int dst_dt = (residual || out_f32) ? SGLC_F32 : dt();
@@ -201,6 +215,14 @@ struct Walk {
         check(code, "gemm_tc_kv");
         return rc == 0;
       }
+    }
+    if (!m.bf16 && c.write && ((uintptr_t)h & 15) == 0 && ((uintptr_t)L.qkv.w & 15) == 0 &&
+        L.qkv.N == (L.n_heads + 2 * L.n_kv_heads) * L.head_dim && g.gemm_f32_supports(L.qkv.N, L.qkv.K, m.hidden)) {
+      check(g.gemm_f32_kv((const float*)h, (const float*)L.qkv.w, L.qkv.bias, (float*)qkv, T, L.qkv.N, L.qkv.K, m.hidden, wq,
+                          (float*)c.cache, s.slots[c.group], L.n_heads * L.head_dim, L.n_kv_heads, L.head_dim, m.page_size,
+                          c.n_pages, s.tc_err, s.stream),
+            "gemm_f32_kv");
+      return rc == 0;
     }
     gemm(h, T, m.hidden, L.qkv, qkv, wq, false, nullptr, SGLC_ACT_NONE);
     return false;

@@ -63,6 +63,7 @@ class WalkStep(C.Structure):
 
 
 _LIBS = {"sglc_embed": "embed", "sglc_layernorm": "layernorm", "sglc_gemm_simt": "gemm_simt",
+         "sglc_gemm_f32_supports": "gemm_f32", "sglc_gemm_f32": "gemm_f32", "sglc_gemm_f32_kv": "gemm_f32",
          "sglc_gemm_tc": "gemm_tc", "sglc_gemm_tc_kv": "gemm_tc", "sglc_gemm_few_supports": "gemm_few", "sglc_gemm_few": "gemm_few",
          "sglc_kv_write": "kv_cache", "sglc_attention_simt": "attention_simt",
          "sglc_attention_prefill_tc": "attention_prefill_tc", "sglc_attention_decode_splits": "attention_decode",

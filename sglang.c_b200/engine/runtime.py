@@ -1,7 +1,8 @@
 """The runtime: device, precision, and the choice of kernel for each operation.
 
-"float32": weights, activations and cache in 32-bit, every product by plain
-FFMA kernels (no tensor-core mode).  "bfloat16": matrices, activations and
+"float32": weights, activations and cache in 32-bit; products on the tensor cores with every number
+as three bfloat16 pieces (exactly) and 32-bit sums, which is closer to the true product than a chain of
+32-bit multiply-adds (csrc/gemm_f32.cu), or by such chains where that kernel does not take the sizes.  "bfloat16": matrices, activations and
 cache in bfloat16 with 32-bit accumulation; the residual stream, norms' and
 softmax statistics stay 32-bit in both.
 """
@@ -51,16 +52,22 @@ class Runtime:
             if few_ok and a.shape[0] <= ops.FEW_MAX_TOKENS and w.numel() <= ops.FEW_MAX_WEIGHT:
                 return ops.gemm_few(a, w, bias, out=out, residual=residual, act=act)
             return ops.gemm_tc(a, w, bias, out=out, residual=residual, act=act, supported=True)
+        if self.dtype == "float32" and ops.gemm_f32_supported(a, w):
+            return ops.gemm_f32(a, w, bias, out=out, residual=residual, act=act)
         return ops.gemm_simt(a, w, bias, out=out, residual=residual, act=act)
 
     def project_qkv(self, ctx, h, linear, qkv, binding, grp, n_heads, n_kv_heads, head_dim):
-        """qkv = h·Wᵀ + b for a mixer that owns its cache.  In a step with prompt portions the
-        tensor-core product writes the keys and values into the cache from its epilogue (they
+        """qkv = h·Wᵀ + b for a mixer that owns its cache.  In the 32-bit path, and in a step with prompt
+        portions, the tensor-core product writes the keys and values into the cache from its epilogue (they
         are not needed in `qkv` then: the attention kernels of such a step read the cache);
         returns whether it did, for attend()."""
         if self.dtype == "bfloat16" and binding.write and ctx.max_q_len > 1 \
                 and ops.gemm_tc_kv(h, linear.weight, linear.bias, qkv, binding.tensor, grp.slots, n_heads,
                                    n_kv_heads, head_dim):
+            return True
+        if self.dtype == "float32" and binding.write \
+                and ops.gemm_f32_kv(h, linear.weight, linear.bias, qkv, binding.tensor, grp.slots, n_heads,
+                                    n_kv_heads, head_dim):
             return True
         linear.forward(ctx, h, out=qkv)
         return False

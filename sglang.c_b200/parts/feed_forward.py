@@ -39,7 +39,7 @@ class MLP(Part):
             softplus = lambda v: max(v, 0.0) + math.log1p(math.exp(-abs(v)))
             self.act_params = (softplus(p), 0.5 + softplus(q))
             if self.rt is not None:
-                libs = ["gemm_simt"] + (["gemm_tc", "gemm_few"] if self.rt.dtype == "bfloat16" else [])
+                libs = ["gemm_simt"] + (["gemm_tc", "gemm_few"] if self.rt.dtype == "bfloat16" else ["gemm_f32"])
                 self.act_slot = ops.register_act_params(*self.act_params, libs)
 
     act_params = act_slot = None
