@@ -42,6 +42,7 @@ constexpr int BK = 64;    // K per stage: 128 bytes of bfloat16, one swizzle row
 constexpr int UMMA_K = 16;
 constexpr int THREADS = 192;   // warp 0: TMA, warp 1: MMA + TMEM, warps 2-5: epilogue
 constexpr int MAX_STAGES = 8;
+constexpr int FEW_BUDGET = 96 * 1024;      // the few-token kernel's ring
 constexpr int PAIR_THREADS = 64 + 256;   // the two-SM kernel: warp 0 TMA, warp 1 MMA, two groups of four epilogue warps
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -1176,10 +1177,8 @@ int pairs_at_once() { return g_pairs_at_once; }
 }  // namespace
 
 // Orientation, tile width and K split for a problem size.
-// From 65 tokens on, a product over a short K goes to the many-token kernel although its one row
-// of tiles is half empty: the few-token orientation would split K over a cluster and pass
-// 128 x 128 partial sums, 64 KB a block, through distributed shared memory (measured at 96 and
-// 128 tokens: a decode step 15-17 % shorter; at 64 tokens and fewer the split wins or ties).
+// From 65 tokens on, a product over a short K may go to the many-token kernel although its one row
+// of tiles is half empty (`few_tokens` compares the two).
 constexpr int DIRECT_MIN_M = 65, DIRECT_MAX_KB = 32;
 // More tokens than that over a long K, with few features: the many-token kernel has few tiles, each a long walk
 // over K by one SM while the others idle.  The few-token orientation with tiles of 32 tokens deals K to a cluster as
@@ -1202,6 +1201,37 @@ static int long_k_split(int M, int N, int kb_total) {
 static bool wide_split(int M, int tiles_p, int kb_total) {
   return M <= 16 && kb_total >= 48 && (tiles_p <= 6 || (tiles_p <= 9 && kb_total >= 56));
 }
+// Up to 128 tokens, weights on the MMA's 128-row side: tiles of 16 or 32 tokens, and K dealt to a cluster of one to eight
+// blocks, by an estimate of the time in us.  What it is made of: a block's walk over its K blocks; the rounds in which a
+// block's threads finish the rows it owns (from four blocks on at 16 tokens, eight at 32, there is one); what passes through
+// distributed shared memory, which grows with all blocks together; and rounds of blocks where not all are resident at once,
+// which cost most (by shared memory two, three or four are on an SM, and clusters leave up to an eighth of the places empty).
+// Fitted to 8,000 launches with a layer norm between them (19 sizes from 256 x 768 to 16,384 x 768 and 1,600 x 6,400, 2 to
+// 128 tokens; 8 % rms), where it is 0.6 % from the best choice of each size.  Before, more than 48 tokens took tiles of 32
+// and K was always dealt as far as eight.  Before and now, us with the norm's 1.9: 2,304 x 768 at 64 tokens 9.3, 7.3, 3,072 x
+// 768 at 45 9.5, 7.3, 768 x 768 at 64 7.9, 6.5, 1,024 x 1,024 at 128 9.6, 7.1, 3,072 x 1,024 at 13 7.1, 6.6, 4,800 x 1,600 at
+// 13 12.4, 7.9 and at 64 21.4, 11.4.
+static double few_tokens(int M, int N, int kb_total, int bn, int splits, int* per_out, int* splits_out) {
+  const int per = (kb_total + splits - 1) / splits, s = (kb_total + per - 1) / per;
+  const int rows = (BM + s - 1) / s, rounds = s > 1 ? (rows * bn / 4 + 127) / 128 : 2;
+  const int stage = BM * BK * 2 + bn * BK * 2;
+  int stages = FEW_BUDGET / stage;
+  if (stages > MAX_STAGES) stages = MAX_STAGES;
+  if (stages > per) stages = per;
+  const int smem = stages * stage + (s > 1 ? rows * s * (bn + 4) * 4 : 0) + 2400;
+  int here = 228 * 1024 / smem;
+  if (here > 8) here = 8;
+  const int at_once = (int)(148 * here * (s == 1 ? 1.0 : s == 2 ? 0.97 : s == 3 ? 0.92 : 0.88));
+  const long long blocks = (long long)((N + BM - 1) / BM) * ((M + bn - 1) / bn) * s;
+  const double together = (double)(blocks < at_once ? blocks : at_once);
+  const bool wide = bn > 16;
+  *per_out = per;
+  *splits_out = s;
+  return (double)((blocks + at_once - 1) / at_once) * (4.87 + 0.29 * per + 0.42 * (rounds - 1) + (wide ? 0.74 + 0.05 * per : 0.0)) +
+         together * (0.0056 + (s > 1 ? 0.0001 * s : 0.0) + (wide ? 0.0017 : 0.0));
+}
+// Many features (the head over the vocabulary) keep the old choice: no split, all tiles resident by a shallow ring.
+constexpr int FEW_MAX_TILES = 200;
 // deal_k: false for the projections that write the cache, which only the many-token kernels do; widest: the largest
 // cluster the device holds.
 static void plan(int M, int N, int K, bool deal_k, int widest, int* swap, int* bn, int* splits, int* kb_per_split,
@@ -1216,7 +1246,39 @@ static void plan(int M, int N, int K, bool deal_k, int widest, int* swap, int* b
     *splits = (kb_total + *kb_per_split - 1) / *kb_per_split;
     return;
   }
-  if (M <= 128 && !(M >= DIRECT_MIN_M && kb_total <= DIRECT_MAX_KB)) {
+  const int rows128 = (N + BM - 1) / BM;
+  if (M <= 128 && rows128 <= FEW_MAX_TILES && !(widest >= 16 && wide_split(M, rows128, kb_total)) &&
+      (deal_k || M < DIRECT_MIN_M || kb_total > DIRECT_MAX_KB)) {
+    double best = 1e30;
+    if (M >= DIRECT_MIN_M && kb_total <= DIRECT_MAX_KB) {
+      // (the many-token kernel's tiles are 128 tokens high: 65 as well as 128 of them take 8.4 us over K 768, 9.5 over 1,024,
+      // 12.1 over 1,600)
+      const int wide = (rows128 >= 74 || N <= 64) ? 128 : 64;
+      best = (double)(((N + wide - 1) / wide + 147) / 148) * (5.0 + 0.285 * kb_total) - 0.2;
+    }
+    *swap = 0;
+    // Up to 16 tokens blocks were dealt to all SMs twice, as far as eight times, and that stays unless a fourteenth is won:
+    // the estimate's launches stand alone, and in a step more and smaller blocks leave the next launch's more room to start
+    // in (a prompt of 14 tokens 398 us, and 406 by the estimate alone).
+    const int dealt = M <= 16 ? (2 * 148 / rows128 < 1 ? 1 : 2 * 148 / rows128 > 8 ? 8 : 2 * 148 / rows128) : 0;
+    for (int b = 16; b <= 32; b += 16)
+      for (int want = 1; want <= 8 && want <= kb_total; want++) {
+        int per, s;
+        double us = few_tokens(M, N, kb_total, b, want, &per, &s);
+        if (b == 16 && (want == dealt || (want == kb_total && want < dealt))) us *= 0.93;
+        if (us >= best) continue;
+        best = us;
+        *swap = 1;
+        *bn = b;
+        *splits = s;
+        *kb_per_split = per;
+      }
+    if (*swap) {
+      *tiles_p = rows128;
+      *tiles_q = (M + *bn - 1) / *bn;
+      return;
+    }
+  } else if (M <= 128 && !(M >= DIRECT_MIN_M && kb_total <= DIRECT_MAX_KB)) {
     *swap = 1;
     *tiles_p = (N + BM - 1) / BM;
     // enough blocks to put most SMs on the weights, but few enough partial sums that the
@@ -1228,20 +1290,11 @@ static void plan(int M, int N, int K, bool deal_k, int widest, int* swap, int* b
     int per = (kb_total + want - 1) / want;
     *kb_per_split = per;
     *splits = (kb_total + per - 1) / per;
-    // The tokens' side of the tile: what a block passes through distributed shared memory for
-    // the split-K sum grows with it (a 128 x 64 tile of partial sums is 32 KB a block: 3 us of
-    // each product), so more than 16 tokens are dealt to several tiles of 16 or 32 (the weights of
-    // the later ones come from L2) as long as all blocks of the product still find room on the
-    // SMs at once (two a SM); tiles of 64 are not used at all.  Measured on decode steps of 24
-    // to 128 requests: 5 to 13 % shorter at GPT-2 small's widths, about even at medium and XL
-    // widths, where the blocks are many already and the rule mostly keeps the wide tiles.
-    auto blocks = [&](int b) { return (long long)(*tiles_p) * ((M + b - 1) / b) * (*splits); };
-    if (M <= 16) *bn = 16;
-    else if (M <= 48) *bn = blocks(16) <= 2 * 148 ? 16 : 32;
-    else if (M <= 64) *bn = 32;
-    else *bn = blocks(32) <= 2 * 148 ? 32 : 128;
+    *bn = M <= 16 ? 16 : M <= 64 ? 32 : 128;
     *tiles_q = (M + *bn - 1) / *bn;
-  } else {
+    return;
+  }
+  {
     *swap = 0;
     int tiles128 = ((M + BM - 1) / BM) * ((N + 127) / 128);
     // a block of the many-token kernel walks its tiles one after the other: wide tiles (fewer
@@ -1342,8 +1395,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
     return bn == 128 ? launch_stream<128, false, false>(mp, mq, mo, a, none, stream) : launch_stream<64, false, false>(mp, mq, mo, a, none, stream);
   }
   int stage_bytes = BM * BK * 2 + bn * BK * 2;
-  int budget = swap ? 96 * 1024 : (bn == 128 ? 100 * 1024 : 100 * 1024);
-  int stages = budget / stage_bytes;
+  int stages = FEW_BUDGET / stage_bytes;
   if (stages > MAX_STAGES) stages = MAX_STAGES;
   if (stages > per) stages = per;
   // Many tiles and no split (the head over the vocabulary, a few tokens): with a deep ring two
@@ -1361,7 +1413,6 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* ou
   switch (bn) {
     case 16: return xi ? launch<16, true>(mp, mq, mo, a, grid, stream) : launch<16, false>(mp, mq, mo, a, grid, stream);
     case 32: return xi ? launch<32, true>(mp, mq, mo, a, grid, stream) : launch<32, false>(mp, mq, mo, a, grid, stream);
-    case 64: return xi ? launch<64, true>(mp, mq, mo, a, grid, stream) : launch<64, false>(mp, mq, mo, a, grid, stream);
     case 128: return xi ? launch<128, true>(mp, mq, mo, a, grid, stream) : launch<128, false>(mp, mq, mo, a, grid, stream);
   }
   return SGLC_ERR_ARGUMENT;

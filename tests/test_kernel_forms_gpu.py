@@ -482,3 +482,21 @@ def test_few_tokens_over_a_long_k(M, N, K):
     # 32-bit sums of K products: K roundings of 2^-24 of sums that stay below sum |a w|, a random walk of them
     bound = float((a.double().abs() @ w.double().abs().T).max()) * 2.0 ** -24 * K ** 0.5
     assert float((x.double() - want).abs().max()) < bound
+
+
+@pytest.mark.parametrize("M,N,K", [(45, 2304, 768), (64, 768, 768), (56, 16400, 128), (65, 1000, 776), (128, 1030, 1024), (97, 1600, 1608),
+                                   (33, 130, 3080), (70, 770, 3072), (13, 4800, 1600), (24, 100, 64)])
+def test_few_tokens_in_tiles_of_16_and_32(M, N, K):
+    """Tokens, features and K off the tiles' edges, K whole and in two to eight shares, more blocks than are resident at once."""
+    ops = _ops()
+    assert ops.gemm_tc_form(M, N, K) == "few"
+    a, w, bias, x = _rand(M, K, dtype=torch.bfloat16, seed=1), _rand(N, K, dtype=torch.bfloat16, seed=2), _rand(N, seed=3), _rand(M, N, seed=4)
+    plain = a.double() @ w.double().t() + bias.double()
+    want = x.double() + plain
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.gemm_tc(a, w, bias, out=out)
+    ops.gemm_tc(a, w, bias, residual=x)
+    # 32-bit sums of K products: K roundings of 2^-24 of sums that stay below sum |a w|, a random walk of them
+    bound = float((a.double().abs() @ w.double().abs().t()).max()) * 2.0 ** -24 * K ** 0.5 + 1e-5
+    assert float((x.double() - want).abs().max()) < bound
+    assert float((out.double() - plain).abs().max()) < float(plain.abs().max()) * 2.0 ** -8      # half a unit of bfloat16
