@@ -920,6 +920,52 @@ SGLC_API int sglc_attention_decode_stream_supports(int D, int page_size, int max
   return 1;
 }
 
+// Which of this file's kernels takes heads of 64: the split-key kernel with so many blocks an item (1 to 8), or (0) the
+// streaming one; -1 where the rules by items and blocks stand.  By an estimate of the time in us, of what was measured behind
+// a layer norm (17 numbers of items from 12 to 768, contexts of 60 to 960, alike and ragged, pages of 16): a block's walk over
+// its keys, the merge in a cluster, what all blocks together do, and rounds of blocks where shared memory, sized by
+// max_keys, does not hold all of them at once (clusters leave up to an eighth of the places empty).  Before, an item had a
+// block for every 64 to 128 keys whatever was resident, and from 160 items on all went to the streaming kernel.  Before and
+// now, us with the norm's 1.9: 96 items of 700 keys (of at most 1,024) 11.4, 7.5 and of 960 12.8, 8.5; 12 of 60 5.2, 4.3; 192
+// of 200 9.2, 6.7, of 350 9.1, 7.7; 208 of 512 10.2, 9.2; 336 of 200 9.4, 7.0; 480 of 100 10.9, 6.4, of 200 15.7, 11.7; 144 of
+// 700 13.0, 11.3.
+SGLC_API int sglc_attention_decode_form(int T, int H, int D, int page_size, int max_keys, int window) {
+  if (D != 64 || page_size < 1 || page_size > 64 || (page_size * D * 2) % 128 != 0 || T <= 0 || H <= 0 || max_keys <= 0) return -1;
+  const long long n = (long long)T * H;
+  const int eff = window > 0 && window < max_keys ? window : max_keys;
+  const double keys = 0.8 * eff;
+  int best = -1;
+  double best_us = 1e30;
+  if (sglc_attention_decode_stream_supports(D, page_size, max_keys, window) && n >= 24) {
+    const long long rounds = (n + 443) / 444;
+    best_us = n * 2 <= 444 && eff > 256 ? 5.3 + 0.01 * keys : 1.0 + (double)rounds * (4.6 + 0.0155 * keys);
+    best = 0;
+  }
+  // (the share that attention_decode.cu's rule deals stays where the two are about even)
+  int dealt = (int)((2 * 148 + n - 1) / n);
+  if (dealt < (max_keys + 127) / 128) dealt = (max_keys + 127) / 128;
+  if (dealt > (max_keys + 63) / 64) dealt = (max_keys + 63) / 64;
+  if (dealt > 8) dealt = 8;
+  const int nb = (max_keys + page_size - 1) / page_size;
+  for (int s = 1; s <= 8 && n * s <= 1536; s++) {
+    const int chunk = (eff + s - 1) / s, rows = ((chunk + page_size - 1) / page_size + 1) * page_size;
+    const int smem = 2 * rows * D * 2 + (WARPS * D + nb + 8 * (D + 2)) * 4;
+    if (smem > 200 * 1024) continue;
+    int here = 227 * 1024 / (smem + 2048);
+    if (here > 10) here = 10;
+    const int at_once = (int)(148 * here * (s == 1 ? 1.0 : s == 2 ? 0.97 : s == 3 ? 0.92 : 0.88));
+    const long long blocks = n * s, rounds = (blocks + at_once - 1) / at_once;
+    double us = (double)rounds * ((s == 1 ? 3.5 : 4.75) + 0.0135 * keys / s) + 0.0027 * (double)(blocks < at_once ? blocks : at_once);
+    if (rounds > 1 && s > 1) us *= 1.7;               // (clusters of a second round wait for whole groups of places)
+    if (s == dealt) us -= 0.3;
+    if (us < best_us) {
+      best_us = us;
+      best = s;
+    }
+  }
+  return best;
+}
+
 // Same arguments and result as sglc_attention_decode_tma (n_splits has no meaning here: a block
 // walks whole (token, head) items).  Meant for many items; any number is served.
 SGLC_API int sglc_attention_decode_stream(const void* q, int q_stride, void* cache, const int* block_table,

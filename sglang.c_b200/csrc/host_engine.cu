@@ -114,6 +114,7 @@ const char* const LAUNCHER_LIB[][2] = {
     {"sglc_attention_decode_scratch", "attention_decode"}, {"sglc_attention_decode", "attention_decode"},
     {"sglc_attention_decode_tma", "attention_decode_tma"},
     {"sglc_attention_decode_stream_supports", "attention_decode_tma"},
+    {"sglc_attention_decode_form", "attention_decode_tma"},
     {"sglc_attention_decode_stream", "attention_decode_tma"}};
 
 struct Kernels {

@@ -530,8 +530,9 @@ def attention_decode(q, cache, block_table, token_req, positions, out, n_heads, 
     `token_list` (int32, its first `n_tokens` entries) names the tokens to serve; a list of all
     tokens is an order in which the streaming kernel takes them (long contexts first balance
     its blocks).
-    Three kernels serve it, chosen by the size of the launch (or named by `variant`, for tests
-    and tuning: "stream", "tma", "register")."""
+    Three kernels serve it, chosen by the size of the launch (sglc_attention_decode_form, or by the
+    items and blocks where that has no answer), or named by `variant`, for tests and tuning: "stream", "tma",
+    "register"."""
     _need_cuda(q, cache, block_table, token_req, positions, out, k_new, v_new, slots, token_list)
     for t, nm in ((block_table, "block_table"), (positions, "positions")):
         _i32(t, nm)
@@ -569,7 +570,14 @@ def attention_decode(q, cache, block_table, token_req, positions, out, n_heads, 
         new_stride = k_new.stride(0)
     if variant not in (None, "stream", "tma", "register"):
         raise KernelError(f"attention_decode: unknown variant {variant!r}")
-    if variant == "stream" or (variant is None and USE_TMA_DECODE and T * n_heads >= STREAM_MIN_ITEMS):
+    form = -1
+    if variant is None and not n_splits and USE_TMA_DECODE and D == 64:
+        form = build.load("attention_decode_tma").sglc_attention_decode_form(T, n_heads, D, page_size, int(max_keys),
+                                                                             int(window or 0))
+        if form > 0:
+            splits = form
+    if variant == "stream" or (variant is None and USE_TMA_DECODE
+                               and (form == 0 or form < 0 and T * n_heads >= STREAM_MIN_ITEMS)):
         # many (token, head) items: resident blocks stream them through a ring of TMA stages
         tlib = build.load("attention_decode_tma")
         if tlib.sglc_attention_decode_stream_supports(D, page_size, int(max_keys), int(window or 0)) \
@@ -588,7 +596,7 @@ def attention_decode(q, cache, block_table, token_req, positions, out, n_heads, 
     if order_only:
         token_list = None
     if D in (64, 128) and splits <= 8 and (page_size * D * 2) % 128 == 0 and page_size <= 256 \
-            and ((variant is None and USE_TMA_DECODE and T * n_heads * splits <= 1536) or variant == "tma"):
+            and ((variant is None and USE_TMA_DECODE and (form > 0 or T * n_heads * splits <= 1536)) or variant == "tma"):
         # keys and values staged through shared memory by TMA (measured faster up to about a
         # thousand blocks; beyond, the register-staged kernel is a few percent ahead)
         tlib = build.load("attention_decode_tma")

@@ -59,6 +59,7 @@ typedef int (*fn_attention_decode_tma)(const void*, int, void*, const int*, int,
                                        int, int, int, int, int, float, int, int, int, const void*, const void*, int,
                                        const int*, int*, const int*, int, cudaStream_t);
 typedef int (*fn_stream_supports)(int, int, int, int);
+typedef int (*fn_decode_form)(int, int, int, int, int, int);
 typedef int (*fn_attention_decode_stream)(const void*, int, void*, const int*, int, const int*, const int*, void*,
                                           int, int, int, int, int, int, float, int, int, const void*, const void*,
                                           int, const int*, int*, const int*, int, cudaStream_t);
@@ -85,6 +86,7 @@ struct Bound {
   fn_attention_decode attention_decode;
   fn_attention_decode_tma attention_decode_tma;
   fn_stream_supports stream_supports;
+  fn_decode_form decode_form;
   fn_attention_decode_stream attention_decode_stream;
 } g = {};
 
@@ -92,7 +94,8 @@ const char* const NAMES[] = {"sglc_embed", "sglc_layernorm", "sglc_gemm_simt", "
                              "sglc_gemm_few_supports", "sglc_gemm_few", "sglc_kv_write", "sglc_attention_simt",
                              "sglc_attention_prefill_tc", "sglc_attention_decode_splits",
                              "sglc_attention_decode_scratch", "sglc_attention_decode", "sglc_attention_decode_tma",
-                             "sglc_attention_decode_stream_supports", "sglc_attention_decode_stream"};
+                             "sglc_attention_decode_stream_supports", "sglc_attention_decode_form",
+                             "sglc_attention_decode_stream"};
 constexpr int N_BOUND = sizeof(NAMES) / sizeof(NAMES[0]);
 static_assert(sizeof(Bound) == N_BOUND * sizeof(void*), "one pointer per name");
 
@@ -175,7 +178,9 @@ struct Walk {
     int need_c = 0;
     g.decode_scratch(T, H, D, splits, &need_ws, &need_c);
     if (need_ws > s.tc_ws_floats || need_c > s.tc_n_counters) splits = 1;
-    if (s.use_tma_decode && T * H >= s.stream_min_items && g.stream_supports(D, ps, s.max_keys, L.window) &&
+    const int form = s.use_tma_decode && D == 64 ? g.decode_form(T, H, D, ps, s.max_keys, L.window) : -1;
+    if (form > 0) splits = form;
+    if (s.use_tma_decode && (form == 0 || (form < 0 && T * H >= s.stream_min_items)) && g.stream_supports(D, ps, s.max_keys, L.window) &&
         (ps * D * 2) % 128 == 0) {
       check(g.attention_decode_stream(q, q_stride, c.cache, bt, s.bt_stride, token_req, s.positions, out, o_stride, T,
                                       H, Hkv, D, ps, L.scale, L.window, s.max_keys, k_new, v_new, new_stride, slots,
@@ -185,7 +190,7 @@ struct Walk {
     }
     if (order_only) token_list = nullptr;
     if ((D == 64 || D == 128) && splits <= 8 && (ps * D * 2) % 128 == 0 && ps <= 256 && s.use_tma_decode &&
-        T * H * splits <= 1536) {
+        (form > 0 || T * H * splits <= 1536)) {
       const int code = g.attention_decode_tma(q, q_stride, c.cache, bt, s.bt_stride, token_req, s.positions, out,
                                               o_stride, T, H, Hkv, D, ps, L.scale, L.window, s.max_keys, splits, k_new,
                                               v_new, new_stride, slots, s.tc_err, token_list, c.n_pages, s.stream);

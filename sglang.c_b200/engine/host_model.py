@@ -70,6 +70,7 @@ _LIBS = {"sglc_embed": "embed", "sglc_layernorm": "layernorm", "sglc_gemm_simt":
          "sglc_attention_decode_scratch": "attention_decode", "sglc_attention_decode": "attention_decode",
          "sglc_attention_decode_tma": "attention_decode_tma",
          "sglc_attention_decode_stream_supports": "attention_decode_tma",
+         "sglc_attention_decode_form": "attention_decode_tma",
          "sglc_attention_decode_stream": "attention_decode_tma"}
 _bound = {}
 
