@@ -107,6 +107,52 @@ gated_norm_kept_kernel(const float* o, long long o_stride, const float* gate, lo
   }
 }
 
+// Many rows of 64 with bfloat16 results, in whole 16-byte pieces: 16 lanes a row, two rows each, all asked for
+// together.  (For bfloat16 results only: the order of additions is another.)  24,576 rows 7.3 -> 4.5 us, 12,288 4.2 -> 3.5,
+// 4,320 2.3 and 2.5: from 8,192 on.
+constexpr int GN_ROWS = 2;       // of a half warp
+__global__ void __launch_bounds__(128)
+gated_norm_quads_kernel(const float* o, long long o_stride, const float* gate, long long gate_stride, const float* __restrict__ gain,
+                        __nv_bfloat16* __restrict__ y, long long y_stride, long long n_rows, int groups, float eps, int act,
+                        int o_pitch, int gain_rows) {
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, l = lane & 15;
+  const long long first = ((long long)blockIdx.x * 4 + (threadIdx.x >> 5)) * (2 * GN_ROWS) + (lane >> 4);
+  float4 v[GN_ROWS], g[GN_ROWS], w[GN_ROWS];
+  pdl_wait();
+#pragma unroll
+  for (int i = 0; i < GN_ROWS; i++) {
+    const long long row = first + 2 * i;
+    v[i] = g[i] = w[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row >= n_rows) continue;
+    const unsigned t = (unsigned)row / (unsigned)groups, h = (unsigned)row - t * groups;      // (fewer than 2^31 rows)
+    v[i] = *reinterpret_cast<const float4*>(o + t * o_stride + (long long)h * o_pitch + 4 * l);
+    if (act != GN_NONE) g[i] = *reinterpret_cast<const float4*>(gate + t * gate_stride + h * 64 + 4 * l);
+    w[i] = *reinterpret_cast<const float4*>(gain + (gain_rows ? h * 64 : 0) + 4 * l);
+  }
+#pragma unroll
+  for (int i = 0; i < GN_ROWS; i++) {
+    const long long row = first + 2 * i;
+    float ss = (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+#pragma unroll
+    for (int k = 8; k > 0; k >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, k);
+    if (row >= n_rows) continue;
+    const float inv = 1.0f / sqrtf(ss / 64.0f + eps);
+    auto out = [&](float x, float gt, float gn) {
+      x = x * inv * gn;
+      if (act == GN_NONE) return x;
+      float e;                       // (of the fast kind, a few 2^-23: the result is rounded to 2^-9)
+      asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-gt * 1.4426950408889634f));
+      return x * __fdividef(act == GN_SILU ? gt : 1.0f, 1.0f + e);
+    };
+    const __nv_bfloat162 a = __floats2bfloat162_rn(out(v[i].x, g[i].x, w[i].x), out(v[i].y, g[i].y, w[i].y));
+    const __nv_bfloat162 b = __floats2bfloat162_rn(out(v[i].z, g[i].z, w[i].z), out(v[i].w, g[i].w, w[i].w));
+    const unsigned t = (unsigned)row / (unsigned)groups, h = (unsigned)row - t * groups;
+    *reinterpret_cast<uint2*>(y + t * y_stride + h * 64 + 4 * l) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  }
+}
+
 // o, gate: float [T][groups*width] (row strides free); gain: float [width]; y: [T][groups*width]
 // o_pitch: columns between the rows of a token in o (>= width; width + 1 and more with m_run);
 // gain_rows != 0: gain is float [groups*width]; m_run: null, or float [T][groups] (rows m_stride apart).
@@ -126,6 +172,12 @@ SGLC_API int sglc_gated_norm_ext(const float* o, long long o_stride, const float
   if (y_dtype == SGLC_F32)
     return go(width <= 64 ? gated_norm_kept_kernel<float, 2> : width <= 256 ? gated_norm_kept_kernel<float, 8> : gated_norm_kernel<float>,
               (float*)y);
+  auto al = [](const void* q, uintptr_t n) { return (reinterpret_cast<uintptr_t>(q) & (n - 1)) == 0; };
+  if (y_dtype == SGLC_BF16 && width == 64 && !m_run && n_rows >= 8192 && n_rows < 1LL << 31 &&
+      (o_stride | gate_stride | y_stride | o_pitch) % 4 == 0 && al(o, 16) && (act == GN_NONE || al(gate, 16)) && al(gain, 16) && al(y, 8))
+    return sglc_launch(gated_norm_quads_kernel, dim3((unsigned)((n_rows + 8 * GN_ROWS - 1) / (8 * GN_ROWS))), dim3(128), 0, stream, 1,
+                       true, o, o_stride, gate, gate_stride, gain, (__nv_bfloat16*)y, y_stride, n_rows, groups, eps, act, o_pitch,
+                       gain_rows);
   if (y_dtype == SGLC_BF16)
     return go(width <= 64    ? gated_norm_kept_kernel<__nv_bfloat16, 2>
               : width <= 256 ? gated_norm_kept_kernel<__nv_bfloat16, 8>

@@ -500,3 +500,60 @@ def test_few_tokens_in_tiles_of_16_and_32(M, N, K):
     bound = float((a.double().abs() @ w.double().abs().t()).max()) * 2.0 ** -24 * K ** 0.5 + 1e-5
     assert float((x.double() - want).abs().max()) < bound
     assert float((out.double() - plain).abs().max()) < float(plain.abs().max()) * 2.0 ** -8      # half a unit of bfloat16
+
+
+@pytest.mark.parametrize("rows,E,form,gain,bias", [(1024, 768, "rms", True, False), (1025, 8, "layer", True, True), (1031, 1600, "rms", False, False),
+                                                   (1500, 2048, "layer", True, False), (1024, 132, "rms", True, True), (1023, 768, "rms", True, False)])
+def test_norms_of_many_rows(rows, E, form, gain, bias):
+    """A warp a row from 1,024 rows on: widths that end inside a warp's pieces, a gather, a strided source and destination."""
+    ops = _ops()
+    wide = _rand(rows, E + 12, seed=E)
+    x = wide[:, 4:4 + E]
+    g, b = (_rand(E, seed=1) if gain else None), (_rand(E, seed=2) if bias else None)
+    pick = torch.randperm(rows, generator=torch.Generator().manual_seed(3)).to(torch.int32).to(DEV)
+    for rows_of in (None, pick):
+        out = torch.full((rows, E + 8), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.norm_rows(x, g, b, 1e-5, out[:, :E], form, src_rows=rows_of)
+        d = x.double() if rows_of is None else x.double()[rows_of.long()]
+        d = d - d.mean(-1, keepdim=True) if form == "layer" else d
+        want = d / torch.sqrt((d * d).mean(-1, keepdim=True) + 1e-5)
+        want = want * (1.0 if g is None else g.double()) + (0.0 if b is None else b.double())
+        # half a unit of bfloat16, and the 32-bit roundings before it
+        assert float(((out[:, :E].double() - want).abs() - want.abs() * 2.0 ** -8).max()) < 1e-5
+        assert bool(torch.isnan(out[:, E:]).all())
+
+
+@pytest.mark.parametrize("T,groups,act", [(683, 12, "silu"), (2051, 4, "sigmoid"), (8195, 1, "none"), (682, 12, "silu")])
+def test_gated_norm_of_many_rows_of_64(T, groups, act):
+    """Sixteen lanes a row from 8,192 rows on: a number of rows that leaves warps in part, a gain for all rows and one each."""
+    ops = _ops()
+    o, z = _rand(T, groups * 64 + 8, seed=T)[:, :groups * 64], _rand(T, groups * 64, seed=4)
+    for gains in (64, groups * 64):
+        gain = _rand(gains, seed=5)
+        y = torch.empty(T, groups * 64, dtype=torch.bfloat16, device=DEV)
+        ops.gated_norm(o, None if act == "none" else z, gain, y, groups, 64, 1e-5, act)
+        x = o.double().reshape(T, groups, 64)
+        x = (x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5) * gain.double().reshape(-1, 64)).reshape(T, -1)
+        s = torch.sigmoid(z.double())
+        want = x * {"none": 1.0, "sigmoid": s, "silu": s * z.double()}[act]
+        assert float(((y.double() - want).abs() - want.abs() * 2.0 ** -8).max()) < 1e-5
+
+
+@pytest.mark.parametrize("rows,F,per,act", [(3, 8, 8, "silu"), (700, 264, 24, "silu"), (2049, 1024, 128, "silu"), (65, 80, 16, "gelu_tanh"), (300, 4096, 0, "silu")])
+def test_gated_activations_in_16_byte_pieces(rows, F, per, act):
+    """A piece, two pieces and a remainder a thread; weights of blocks of columns, some zero; large and very negative gates."""
+    ops = _ops()
+    src = _rand(rows, 2 * F, dtype=torch.bfloat16, seed=F, scale=4.0)
+    src[0, :4] = torch.tensor([90.0, -90.0, 3.0e4, -3.0e4], device=DEV)
+    w = None
+    if per:
+        w = torch.rand(rows, F // per, generator=torch.Generator().manual_seed(1)).to(DEV)
+        w[::3, 0] = 0.0
+    dst = torch.full((rows, F), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.gated_act(src, dst, weights=w, per=per, act=act)
+    g, u = src[:, :F].double(), src[:, F:].double()
+    want = (g * torch.sigmoid(g) if act == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u
+    if per:
+        want = want * w.double().repeat_interleave(per, 1)
+    # half a unit of bfloat16, and a few 2^-22 of the fast exponential and division (times the gate's size in the exponent)
+    assert float(((dst.double() - want).abs() - want.abs() * (2.0 ** -8)).max()) < 1e-4
