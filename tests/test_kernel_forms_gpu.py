@@ -557,3 +557,92 @@ def test_gated_activations_in_16_byte_pieces(rows, F, per, act):
         want = want * w.double().repeat_interleave(per, 1)
     # half a unit of bfloat16, and a few 2^-22 of the fast exponential and division (times the gate's size in the exponent)
     assert float(((dst.double() - want).abs() - want.abs() * (2.0 ** -8)).max()) < 1e-4
+
+
+@pytest.mark.parametrize("E,groups,form", [(4, 1, "rms"), (512, 1, "layer"), (128, 6, "rms"), (1028, 1, "layer"), (2044, 1, "rms"), (2048, 2, "layer"),
+                                           (4096, 1, "rms"), (4100, 1, "layer")])
+def test_norms_of_a_few_rows(E, groups, form):
+    """Up to two 16-byte pieces a thread, and a row beyond: with a gather, skipped rows, and added to what is there."""
+    ops = _ops()
+    n, W = 5, E * groups
+    x, g, b, there = _rand(n, W + 4, seed=E)[:, :W], _rand(W, seed=1), _rand(W, seed=2), _rand(n + 2, W, seed=3)
+    pick, place = (torch.tensor(v, dtype=torch.int32, device=DEV) for v in ((4, 0, 3, 3, 1), (2, 6, -1, 0, 5)))
+    d = x.double().view(n, groups, E)
+    d = d - d.mean(-1, keepdim=True) if form == "layer" else d
+    want = (d / torch.sqrt((d * d).mean(-1, keepdim=True) + 1e-5)).view(n, W) * g.double() + b.double()
+    tol = 1e-5      # a sum of up to 4,100 squares in 32-bit and a handful of roundings of values below 20
+    got = torch.empty(n, W, device=DEV)
+    ops.norm_rows(x, g, b, 1e-5, got, form, src_rows=pick, groups=groups)
+    assert float((got.double() - want[pick.long()]).abs().max()) < tol
+    added = there.clone()
+    ops.norm_rows(x, g, b, 1e-5, added, form, add=True, dst_rows=place, groups=groups)
+    sure = there.double()
+    for r, p in enumerate(place.tolist()):
+        if p >= 0:
+            sure[p] += want[r]
+    assert float((added.double() - sure).abs().max()) < tol
+    assert torch.equal(added[[1, 3, 4]], there[[1, 3, 4]])
+    half = torch.empty(n, W, dtype=torch.bfloat16, device=DEV)
+    ops.norm_rows(x, None, None, 1e-5, half, form, groups=groups)
+    plain = (d / torch.sqrt((d * d).mean(-1, keepdim=True) + 1e-5)).view(n, W)
+    assert float(((half.double() - plain).abs() - plain.abs() * 2.0 ** -8).max()) < tol
+
+
+@pytest.mark.parametrize("E,K,T", [(1, 8, 3), (8, 768, 8), (17, 1024, 148), (33, 1032, 5), (40, 264, 149), (9, 769, 4)])
+def test_router_makes_its_logits(E, K, T):
+    """Rows that a lane keeps whole and longer ones, more experts than warps, tokens on both sides of the SMs."""
+    ops = _ops()
+    h, w = _rand(T, K, seed=K).bfloat16(), (_rand(E, K, seed=E) / K ** 0.5).bfloat16()
+    top = min(E, 3)
+    dense, ids, wts = torch.empty(T, E, device=DEV), torch.empty(T, top, dtype=torch.int32, device=DEV), torch.empty(T, top, device=DEV)
+    ops.router(None, None, dense, ids, wts, top, rows=h, matrix=w)
+    s = torch.sigmoid(h.double() @ w.double().t())
+    best = torch.topk(s, top, dim=1)
+    # a logit's error is below 2^-24 times the sum of its products' sizes times the additions a lane makes; near ties may fall either way
+    assert float((wts.double() - best.values).abs().max()) < 1e-5
+    assert float((dense.gather(1, ids.long()).double() - torch.gather(s, 1, ids.long())).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("D,V,splits", [(64, 64, 2), (64, 40, 8), (128, 72, 9), (256, 256, 11)])
+def test_merge_of_a_tokens_shares(D, V, splits):
+    """Shares on both sides of the eight that are fetched at once, values that end inside a warp, gates of both kinds and a sink."""
+    ops = _ops()
+    T, H, G, ps, n = 3, 6, 2, 16, 380
+    pages = (n + ps - 1) // ps
+    cache = _rand(pages, G * ps * (D + V), seed=D).bfloat16()
+    q = _rand(T, H * D, seed=V).bfloat16()
+    table = torch.arange(pages, dtype=torch.int32, device=DEV).repeat(T, 1)
+    req, pos = torch.arange(T, dtype=torch.int32, device=DEV), torch.tensor([n - 1, 40, 0], dtype=torch.int32, device=DEV)
+    for sinks, gate in ((None, None), (_rand(H, seed=5), _rand(T, H, seed=6)), (None, _rand(T, H * V, seed=7))):
+        def run(s, **more):
+            out = torch.empty(T, H * V, dtype=torch.bfloat16, device=DEV)
+            ops.attention_ext(q, cache, table, req, pos, out, H, G, D, V, ps, D ** -0.5, None, None, sinks, n, gate=gate, splits=s, **more)
+            return out.double()
+        one = run(1)
+        dealt = run(splits, max_q_len=1, workspace=torch.empty(T * H * splits * (V + 2), device=DEV))
+        # both round a 32-bit result to bfloat16 once: a unit of it apart at most
+        assert float(((dealt - one).abs() - one.abs() * 2.0 ** -7).max()) < 1e-5
+
+
+def test_rotary_rows_have_the_same_bits_beside_many_and_few_tokens():
+    """A warp a row for few tokens, four warps for many; heads wider than what a lane has on its way at once."""
+    ops = _ops()
+    T, H, G, D, V, ps, dims = 150, 7, 2, 272, 40, 16, 96
+    x = _rand(T, H * D + G * (D + V), seed=1)
+    pos, freq = torch.arange(T, dtype=torch.int32, device=DEV) * 7, torch.logspace(0, -4, dims // 2, dtype=torch.float64, device=DEV)
+    def run(lo, hi, q, cache):
+        ops.rotary_kv(x[lo:hi], pos[lo:hi], freq, 1.25, dims, 1e-6, q[lo:hi], cache, torch.arange(lo, hi, dtype=torch.int32, device=DEV), H, G, D, V, ps)
+    made = []
+    for cuts in (((0, T),), ((0, 1), (1, 20), (20, T))):
+        q, cache = torch.zeros(T, H * D, device=DEV), torch.zeros((T + ps - 1) // ps, G * ps * (D + V), device=DEV)
+        for lo, hi in cuts:
+            run(lo, hi, q, cache)
+        made.append((q, cache))
+    assert torch.equal(made[0][0], made[1][0]) and torch.equal(made[0][1], made[1][1])
+    head = x[:, :D].double()
+    a = pos.double()[:, None] * freq
+    u, v = head[:, :dims // 2], head[:, dims // 2:dims]
+    turned = torch.cat([(u * a.cos() - v * a.sin()) * 1.25, (v * a.cos() + u * a.sin()) * 1.25, head[:, dims:]], 1)
+    want = turned / torch.sqrt((turned * turned).mean(-1, keepdim=True) + 1e-6)
+    # the angle is rounded to 32 bits inside one turn: 2^-24 * 2 pi, and a few roundings of values below 6
+    assert float((made[0][0][:, :D].double() - want).abs().max()) < 1e-5
