@@ -762,40 +762,51 @@ SGLC_API int sglc_attention_simt_ext(const void* q, int q_stride, const void* ca
 
 // The merge behind a launch that dealt a token's keys to several blocks (a step of single tokens):
 // the shares' maxima, sums and unnormalised results [T][H][n_splits][DV + 2] become the head's
-// result, the sink (if any) joining the denominator once.  A warp a (token, head).
+// result, the sink (if any) joining the denominator once.  A warp 32 entries of a (token, head), the first
+// eight shares' on their way beside the maxima and sums: one round trip instead of one a 32 entries (8 tokens, 12
+// heads of 64, 5 shares in a decode step 4.1 -> 2.6 us).
+constexpr int MERGE_SHARES = 8;
 template <typename TO>
 __global__ void __launch_bounds__(128)
-attention_merge_kernel(const float* __restrict__ part_ws, int n_splits, const float* __restrict__ sinks,
-                       TO* __restrict__ out, int o_stride, int T, int H, int DV, const OutGate gate) {
+attention_merge_kernel(const float* part_ws, int n_splits, const float* __restrict__ sinks, TO* __restrict__ out, int o_stride,
+                       int T, int H, int DV, const OutGate gate) {
   pdl_launch_dependents();
-  const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  const int chunks = (DV + 31) / 32;
+  const long long at = (long long)blockIdx.x * 4 + (threadIdx.x >> 5), item = at / chunks;
+  const int lane = threadIdx.x & 31, d = (int)(at % chunks) * 32 + lane;
   pdl_wait();
   if (item >= (long long)T * H) return;
   const int t = (int)(item / H), h = (int)(item % H);
+  const bool by_entry = gate.z && !gate.per_head;
   const float* rec = part_ws + (size_t)item * n_splits * (DV + 2);
+  float v[MERGE_SHARES];
+#pragma unroll
+  for (int j = 0; j < MERGE_SHARES; j++) v[j] = j < n_splits && d < DV ? rec[(size_t)j * (DV + 2) + 2 + d] : 0.0f;
   // lane s holds share s's maximum and sum (an empty share: -inf and 0, its results zero)
   const float ms = lane < n_splits ? rec[(size_t)lane * (DV + 2)] : -INFINITY;
   const float ls = lane < n_splits ? rec[(size_t)lane * (DV + 2) + 1] : 0.0f;
   const float sk = sinks ? sinks[h] : -INFINITY;
   const float z_head = gate.z && gate.per_head ? gate.z[t * gate.stride + h] : 0.0f;
+  const float z = by_entry && d < DV ? gate.z[t * gate.stride + (long long)h * DV + d] : 0.0f;
   const float M = fmaxf(warp_max(ls > 0.0f ? ms : -INFINITY), sk);
   const float f = ls > 0.0f ? expf(ms - M) : 0.0f;
   const float L = warp_sum(ls * f) + (sinks ? expf(sk - M) : 0.0f);
   float inv = 1.0f / L;
   if (gate.z && gate.per_head) inv *= 1.0f / (1.0f + expf(-z_head));
-  const bool by_entry = gate.z && !gate.per_head;
-  TO* op = out + (size_t)t * o_stride + (size_t)h * DV;
-  for (int d0 = 0; d0 < DV; d0 += 32) {
-    const int d = d0 + lane;
-    const float z = by_entry && d < DV ? gate.z[t * gate.stride + (long long)h * DV + d] : 0.0f;
-    float o = 0.0f;
-    for (int s = 0; s < n_splits; s++)
-      o = fmaf(d < DV ? rec[(size_t)s * (DV + 2) + 2 + d] : 0.0f, __shfl_sync(0xffffffffu, f, s), o);
-    o *= inv;
-    if (by_entry) o *= 1.0f / (1.0f + expf(-z));
-    if (d < DV) op[d] = from_f32<TO>(o);
+  float o = 0.0f;
+  for (int s0 = 0; s0 < n_splits; s0 += MERGE_SHARES) {
+    if (s0 > 0) {
+#pragma unroll
+      for (int j = 0; j < MERGE_SHARES; j++)
+        v[j] = s0 + j < n_splits && d < DV ? rec[(size_t)(s0 + j) * (DV + 2) + 2 + d] : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < MERGE_SHARES; j++)
+      if (s0 + j < n_splits) o = fmaf(v[j], __shfl_sync(0xffffffffu, f, s0 + j), o);
   }
+  o *= inv;
+  if (by_entry) o *= 1.0f / (1.0f + expf(-z));
+  if (d < DV) out[(size_t)t * o_stride + (size_t)h * DV + d] = from_f32<TO>(o);
 }
 
 // The extended form for a step of single tokens with each token's keys dealt to n_splits blocks:
@@ -814,7 +825,7 @@ SGLC_API int sglc_attention_simt_ext_split(const void* q, int q_stride, const vo
                                       T, H, Hkv, D, page_size, scale, window, max_keys, act_dtype, cache_dtype,
                                       n_pages, err, 1, 0, kv_shared, stream, true, DV, chunk, nullptr, n_splits, part_ws);
   if (code != SGLC_OK) return code;
-  const dim3 grid((unsigned)(((long long)T * H + 3) / 4));
+  const dim3 grid((unsigned)(((long long)T * H * ((DV + 31) / 32) + 3) / 4));
   const OutGate g{gate, gate_stride, gate_per_head};
   if (act_dtype == SGLC_F32)
     return sglc_launch(attention_merge_kernel<float>, grid, dim3(128), 0, stream, 1, true, (const float*)part_ws,
