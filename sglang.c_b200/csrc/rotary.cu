@@ -17,6 +17,7 @@
 SGLC_DEFINE_ERROR_STRING()
 
 constexpr int ROT_WARPS = 4;
+constexpr int ROT_MAX_WARPS = 32;      // of rotary_kv_kernel, where every token has an SM to itself
 constexpr int ROT_MAX_DIM = 512;
 
 // (u, v) -> (u cos a - v sin a, v cos a + u sin a), with the roundings written out: which of the two
@@ -24,20 +25,39 @@ constexpr int ROT_MAX_DIM = 512;
 __device__ __forceinline__ float turn_u(float u, float v, float cs, float sn) { return fmaf(u, cs, -__fmul_rn(v, sn)); }
 __device__ __forceinline__ float turn_v(float u, float v, float cs, float sn) { return fmaf(v, cs, __fmul_rn(u, sn)); }
 
-template <typename TA>
-__global__ void __launch_bounds__(ROT_WARPS * 32)
+// 32 * ROT_AHEAD numbers of a row on their way at once; a loop of loads and stores would wait for each.
+constexpr int ROT_AHEAD = 8;
+template <typename F>
+__device__ __forceinline__ void row_through(const float* src, int n, int lane, F&& put) {
+  for (int d0 = lane; d0 < n; d0 += 32 * ROT_AHEAD) {
+    float v[ROT_AHEAD];
+#pragma unroll
+    for (int j = 0; j < ROT_AHEAD; j++)
+      if (d0 + 32 * j < n) v[j] = src[d0 + 32 * j];
+#pragma unroll
+    for (int j = 0; j < ROT_AHEAD; j++)
+      if (d0 + 32 * j < n) put(d0 + 32 * j, v[j]);
+  }
+}
+
+// FEW: every token has an SM to itself; a warp a row, the row taken into shared memory whole, one round trip instead of one a
+// 32 entries.  8 tokens of 18 rows of 64 in a decode step's chain 5.9 -> 2.5 us (alone 4.6 -> 2.1), of 24 of 128 7.0 ->
+// 2.4.  With many tokens an SM the rows wait beside one another anyway: 2,048 of 18 rows 10.0 us as they are, 11.4 with.
+template <typename TA, bool FEW>
+__global__ void __launch_bounds__((FEW ? ROT_MAX_WARPS : ROT_WARPS) * 32)
 rotary_kv_kernel(const float* x, long long x_stride, const int* __restrict__ positions,
                  const double* __restrict__ freq, float mult, int dims, int norm, float eps,
                  TA* __restrict__ q_out, long long q_stride, TA* __restrict__ cache, const int* __restrict__ slots,
                  int T, int H, int G, int D, int V, int page_size, int n_pages, int* err) {
-  __shared__ float buf[ROT_WARPS][ROT_MAX_DIM];
+  extern __shared__ float row_buf[];           // FEW: D floats a warp, else
+  __shared__ float fixed_buf[FEW ? 1 : ROT_WARPS][FEW ? 1 : ROT_MAX_DIM];
   __shared__ float2 turn[ROT_MAX_DIM / 2];
   pdl_launch_dependents();
-  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = FEW ? blockDim.x >> 5 : ROT_WARPS;
   const int pos = positions[t];                // (the step's own array: no kernel of the step writes it)
   // (cosine, sine) of the token's pairs, once for all of its rows and ahead of the wait (x is not __restrict__: its
-  // loads might move ahead of it).  8 tokens of 15 turned heads in a decode step's chain: 6.5 -> 5.7 us.
-  for (int i = threadIdx.x; i < dims / 2; i += ROT_WARPS * 32) {
+  // loads might move ahead of it).
+  for (int i = threadIdx.x; i < dims / 2; i += warps * 32) {
     double a = (double)pos * freq[i];
     a -= floor(a * 0.15915494309189535) * 6.283185307179586;
     float sn, cs;
@@ -52,18 +72,26 @@ rotary_kv_kernel(const float* x, long long x_stride, const int* __restrict__ pos
   const size_t page_elems = (size_t)G * page_size * (D + V);
   const float* xr = x + (size_t)t * x_stride;
   const int half = dims / 2;
-  float* b = buf[warp];
-  for (int row = warp; row < H + 2 * G; row += ROT_WARPS) {
+  float* b;
+  if constexpr (FEW) b = row_buf + warp * D;
+  else b = fixed_buf[warp];
+  for (int row = warp; row < H + 2 * G; row += warps) {
     if (row >= H + G) {                        // a value head: copied
       const int g = row - H - G;
       if (page_ok) {
         TA* dst = cache + (size_t)page * page_elems + (size_t)G * page_size * D + ((size_t)g * page_size + off) * V;
         const float* src = xr + (size_t)(H + G) * D + (size_t)g * V;
-        for (int d = lane; d < V; d += 32) dst[d] = from_f32<TA>(src[d]);
+        if constexpr (FEW) row_through(src, V, lane, [&](int d, float v) { dst[d] = from_f32<TA>(v); });
+        else for (int d = lane; d < V; d += 32) dst[d] = from_f32<TA>(src[d]);
       }
       continue;
     }
     const float* src = xr + (size_t)row * D;
+    if constexpr (FEW) {
+      row_through(src, D, lane, [&](int d, float v) { b[d] = v; });
+      __syncwarp();
+      src = b;
+    }
     float ss = 0.0f;
     for (int i = lane; i < half; i += 32) {
       const float cs = turn[i].x, sn = turn[i].y;
@@ -74,7 +102,7 @@ rotary_kv_kernel(const float* x, long long x_stride, const int* __restrict__ pos
     }
     for (int d = 2 * half + lane; d < D; d += 32) {
       const float u = src[d];
-      b[d] = u;
+      if (!FEW) b[d] = u;
       ss = fmaf(u, u, ss);
     }
     ss = warp_sum(ss);
@@ -97,14 +125,20 @@ SGLC_API int sglc_rotary_kv(const float* x, long long x_stride, const int* posit
   if (H <= 0 || G <= 0 || D <= 0 || V <= 0 || dims < 0 || dims > D || dims % 2 != 0 || page_size <= 0)
     return SGLC_ERR_ARGUMENT;
   if (D > ROT_MAX_DIM) return SGLC_ERR_UNSUPPORTED;
+  const int rows = H + 2 * G;
+  const bool few = T <= 148;
+  const int most = rows < ROT_MAX_WARPS ? rows : ROT_MAX_WARPS, fit = 10240 / D;      // (40 KB of rows)
+  const int warps = !few || most < ROT_WARPS ? ROT_WARPS : most < fit ? most : fit;
+  auto run = [&](auto* kernel, auto* q, auto* pages) {
+    return sglc_launch(kernel, dim3(T), dim3(warps * 32), few ? (size_t)warps * D * sizeof(float) : 0, stream, 1, true, x, x_stride, positions,
+                       freq, mult, dims, norm, eps, q, q_stride, pages, slots, T, H, G, D, V, page_size, n_pages, err);
+  };
   if (dtype == SGLC_F32)
-    return sglc_launch(rotary_kv_kernel<float>, dim3(T), dim3(ROT_WARPS * 32), 0, stream, 1, true, x, x_stride,
-                       positions, freq, mult, dims, norm, eps, (float*)q_out, q_stride, (float*)cache, slots, T, H, G,
-                       D, V, page_size, n_pages, err);
+    return few ? run(rotary_kv_kernel<float, true>, (float*)q_out, (float*)cache)
+               : run(rotary_kv_kernel<float, false>, (float*)q_out, (float*)cache);
   if (dtype == SGLC_BF16)
-    return sglc_launch(rotary_kv_kernel<__nv_bfloat16>, dim3(T), dim3(ROT_WARPS * 32), 0, stream, 1, true, x,
-                       x_stride, positions, freq, mult, dims, norm, eps, (__nv_bfloat16*)q_out, q_stride,
-                       (__nv_bfloat16*)cache, slots, T, H, G, D, V, page_size, n_pages, err);
+    return few ? run(rotary_kv_kernel<__nv_bfloat16, true>, (__nv_bfloat16*)q_out, (__nv_bfloat16*)cache)
+               : run(rotary_kv_kernel<__nv_bfloat16, false>, (__nv_bfloat16*)q_out, (__nv_bfloat16*)cache);
   return SGLC_ERR_ARGUMENT;
 }
 
