@@ -646,3 +646,17 @@ def test_rotary_rows_have_the_same_bits_beside_many_and_few_tokens():
     want = turned / torch.sqrt((turned * turned).mean(-1, keepdim=True) + 1e-6)
     # the angle is rounded to 32 bits inside one turn: 2^-24 * 2 pi, and a few roundings of values below 6
     assert float((made[0][0][:, :D].double() - want).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("E", [4, 1020, 1024, 1028, 2048, 2052, 4096])
+def test_layer_norm_at_the_edges_of_a_blocks_warps(E):
+    """Blocks of up to 8, 16 and 32 warps, whose partial sums are added in one order: the same bits in both precisions' rounding."""
+    ops = _ops()
+    x, g, b = _rand(5, E, seed=E) + 3.0, _rand(E, seed=1), _rand(E, seed=2)
+    out, half = torch.empty(5, E, device=DEV), torch.empty(5, E, dtype=torch.bfloat16, device=DEV)
+    ops.layernorm(x, g, b, 1e-5, out)
+    ops.layernorm(x, g, b, 1e-5, half)
+    assert torch.equal(out.bfloat16(), half)
+    want = torch.nn.functional.layer_norm(x.double(), (E,), g.double(), b.double(), 1e-5)
+    # sums of up to 4,096 numbers in 32-bit: an error of some 2^-24 * 12 of the mean of 3, times a gain below 5 and 1 / deviation (4 numbers: below 10)
+    assert float((out.double() - want).abs().max()) < 1e-4
