@@ -642,7 +642,7 @@ def measure_model(name, base, n_layer, steps, warmup, pk, points=(1, 64), fp32=T
     r["points"]["prefill_c_api_tok_s"] = \
         (PREFILL_TOKENS - 2) / (time_prefill_c(model_dir, 2, PREFILL_TOKENS // 2 - 1) / 1e3)
     if fp32:
-        # the true 32-bit path (plain FFMA products, 32-bit cache): same step function and scheduler
+        # the true 32-bit path (products of exact bfloat16 pieces, 32-bit cache): same step function and scheduler
         eng = Engine.from_dir(model_dir, dtype="float32", page_size=PAGE, max_tokens=BATCH * (CONTEXT + 256) + 4096,
                               max_requests=BATCH, max_step_tokens=PREFILL_TOKENS)
         t, _, _ = time_decode(eng, BATCH, CONTEXT, steps, warmup)
