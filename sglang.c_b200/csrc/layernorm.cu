@@ -52,13 +52,13 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const int* __restr
 
 // One float4 per thread: the row stays in registers, gain and bias are fetched while the
 // row is in flight, and each reduction costs one barrier (every warp adds the per-warp
-// partial sums itself, in the same order).  NW: the most warps a block has, so that up to 16 partial sums come
+// partial sums itself, in the same order).  NW: the most warps a block has, so that up to 13 partial sums come
 // together and not one after another: 8 rows of 768 1.84 -> 1.58 us, 512 of them 3.13 -> 2.48, 8 of 1,600 2.02 -> 1.80; a decode
-// step is 2 % shorter.  More than 16: 1,023 rows of 4,096 11.0 us one after another, 12.3 together.
+// step is 2 % shorter.  More than 13: 1,023 rows of 2,048 5.05 us one after another, 5.26 together, of 4,096 11.0 and 12.3.
 template <int NW>
 __device__ __forceinline__ float add_up(const float* red, int nw) {
   float sum = 0.0f;
-  if constexpr (NW > 16) {
+  if constexpr (NW > 13) {
     for (int k = 0; k < nw; k++) sum += red[k];
     return sum;
   }
@@ -206,7 +206,7 @@ SGLC_API int sglc_layernorm(const float* x, const int* rows, const float* gamma,
       return sglc_launch(kernel, dim3(n_rows), dim3(th), 0, stream, 1, true, x, rows, gamma, beta, o, n_rows, E, eps);
     };
 #define ROW4_LAUNCH(TO)                                                                                                    \
-  return th <= 256 ? run(layernorm_row4_kernel<TO, 8>, (TO*)out) : th <= 512 ? run(layernorm_row4_kernel<TO, 16>, (TO*)out) \
+  return th <= 256 ? run(layernorm_row4_kernel<TO, 8>, (TO*)out) : th <= 416 ? run(layernorm_row4_kernel<TO, 13>, (TO*)out) \
                                                                              : run(layernorm_row4_kernel<TO, 32>, (TO*)out)
     if (out_dtype == SGLC_F32) ROW4_LAUNCH(float);
     if (out_dtype == SGLC_BF16) ROW4_LAUNCH(__nv_bfloat16);

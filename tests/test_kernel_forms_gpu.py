@@ -648,9 +648,9 @@ def test_rotary_rows_have_the_same_bits_beside_many_and_few_tokens():
     assert float((made[0][0][:, :D].double() - want).abs().max()) < 1e-5
 
 
-@pytest.mark.parametrize("E", [4, 1020, 1024, 1028, 2048, 2052, 4096])
+@pytest.mark.parametrize("E", [4, 1020, 1024, 1028, 1664, 1668, 4096])
 def test_layer_norm_at_the_edges_of_a_blocks_warps(E):
-    """Blocks of up to 8, 16 and 32 warps, whose partial sums are added in one order: the same bits in both precisions' rounding."""
+    """Blocks of up to 8, 13 and 32 warps, whose partial sums are added in one order: the same bits in both precisions' rounding."""
     ops = _ops()
     x, g, b = _rand(5, E, seed=E) + 3.0, _rand(E, seed=1), _rand(E, seed=2)
     out, half = torch.empty(5, E, device=DEV), torch.empty(5, E, dtype=torch.bfloat16, device=DEV)
