@@ -111,14 +111,35 @@ __device__ __forceinline__ void tmem_st_16x256b_x1(uint32_t taddr, uint32_t a, u
   asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d)
                : "memory");
 }
-__device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
-  float s = 0.0f;
-  for (int k = 0; k < K; k++) s = fmaf(a[k], w[k], s);
+__device__ __forceinline__ bool finite(float s) { return fabsf(s) <= 3.402823466e38f; }
+// T tokens' outputs (of which `tokens` exist) as plain chains of multiply-adds, k = 0..K-1 each.
+template <int T> struct Sums { float v[T]; };
+template <int T>
+__device__ __noinline__ Sums<T> plain_sums(const float* a, int lda, int tokens, const float* w, int K) {
+  const float4* row[T];
+#pragma unroll
+  for (int j = 0; j < T; j++) row[j] = reinterpret_cast<const float4*>(a + (size_t)min(j, tokens - 1) * lda);
+  Sums<T> s = {};
+#pragma unroll 8 / T + 2
+  for (int k = 0; k < K / 4; k++) {
+    const float4 y = reinterpret_cast<const float4*>(w)[k];
+#pragma unroll
+    for (int j = 0; j < T; j++) {
+      const float4 x = row[j][k];
+      s.v[j] = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s.v[j]))));
+    }
+  }
   return s;
 }
-__device__ __forceinline__ bool finite(float s) { return fabsf(s) <= 3.402823466e38f; }
-__device__ __forceinline__ float plain_again(const F32Args& p, int m, int n) {
-  return plain_dot(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.K, p.K);
+// Whether there is a NaN among the 16-byte pieces first, first + step, ... of a row.
+__device__ __noinline__ bool any_nan(const float* row, int K, int first, int step) {
+  bool nan = false;
+#pragma unroll 8
+  for (int k = first; k < K / 4; k += step) {
+    const float4 x = reinterpret_cast<const float4*>(row)[k];
+    nan = nan || x.x != x.x || x.y != x.y || x.z != x.z || x.w != x.w;
+  }
+  return nan;
 }
 
 // Blocks walk tiles (features fastest), all of K each; or, CLUSTER, the blocks of a cluster share one tile: rank r takes the
@@ -433,10 +454,20 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         bool all = true;
 #pragma unroll
         for (int j = 0; j < CW; j++) all = all && finite(sum[j]);
-        if (!all) {
+        if (__any_sync(0xffffffffu, !all)) {
+          // A NaN among a token's numbers, which the warp looks for together, or a feature's makes the output NaN without a
+          // chain: in a step whose values have become NaN a chain for every output would take a hundred times the tile.
+          int w_nan = -1;                               // (not looked for yet)
 #pragma unroll
-          for (int j = 0; j < CW; j++)
-            if (f < p.N && mt + j < p.M && !finite(sum[j])) sum[j] = plain_again(p, mt + j, f);
+          for (int j = 0; j < CW; j++) {
+            const bool bad = f < p.N && mt + j < p.M && !finite(sum[j]);
+            if (!__any_sync(0xffffffffu, bad)) continue;
+            const float *a = p.A + (size_t)(mt + j) * p.lda, *w = p.W + (size_t)f * p.K;
+            const bool a_nan = __any_sync(0xffffffffu, any_nan(a, p.K, lane, 32));
+            if (!bad) continue;
+            if (!a_nan && w_nan < 0) w_nan = any_nan(w, p.K, 0, 1);
+            sum[j] = a_nan || w_nan > 0 ? __int_as_float(0x7fffffff) : plain_sums<1>(a, p.lda, 1, w, p.K).v[0];
+          }
         }
         if (p.act != SGLC_ACT_NONE) {
 #pragma unroll
@@ -513,11 +544,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           }
         }
         float v[4] = {s.x, s.y, s.z, s.w};
+        if (m0 + col < p.M && !(finite(v[0]) && finite(v[1]) && finite(v[2]) && finite(v[3]))) {
+          const Sums<4> c = plain_sums<4>(p.A + (size_t)(m0 + col) * p.lda, p.lda, min(4, p.M - m0 - col), p.W + (size_t)f * p.K, p.K);
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            if (!finite(v[j])) v[j] = c.v[j];
+        }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const int m = m0 + col + j;
           if (m >= p.M) break;
-          if (!finite(v[j])) v[j] = plain_again(p, m, f);
           const float y = apply_act(v[j] + bias, p.act);
           if (p.cache && f >= p.q_cols) {
             const long long at = slot_at(p, m);

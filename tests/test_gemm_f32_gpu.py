@@ -102,6 +102,46 @@ def test_gemm_f32_numbers_at_the_edges():
             assert torch.allclose(out[r, :140], chain[r, :140], rtol=1e-6, atol=2.0 ** -133), r
 
 
+@pytest.mark.parametrize("M,K", [(37, 68), (3, 200), (130, 132)])
+def test_gemm_f32_outputs_that_are_no_numbers_at_the_edges(M, K):
+    """NaN and infinities in the last token, k and feature: what a chain of multiply-adds gives, and the other outputs unchanged."""
+    a, w, ops = _rand(M, K, seed=5), _rand(131, K, seed=6), _ops()
+    clean, chain = torch.empty(M, 131, device=DEV), torch.empty(M, 131, device=DEV)
+    ops.gemm_f32(a, w, None, out=clean)
+    a[M - 1, K - 1], a[0, 0], w[130, K - 2], w[129, 1], w[128, 5] = float("nan"), float("inf"), float("nan"), -float("inf"), 3e38
+    ops.gemm_simt(a, w, None, out=chain)
+
+    def run(ops):
+        out = torch.full((M, 131), 5.0, device=DEV)
+        ops.gemm_f32(a, w, None, out=out)
+        return out
+
+    for out in _each(run):
+        assert torch.equal(torch.isnan(out), torch.isnan(chain)) and torch.equal(out[torch.isinf(chain)], chain[torch.isinf(chain)])
+        assert torch.equal(out[1:M - 1, :128], clean[1:M - 1, :128])
+        assert torch.allclose(out[1:M - 1, 128], chain[1:M - 1, 128], rtol=1e-5)
+
+
+def test_gemm_f32_of_nan_takes_a_few_times_the_time_and_no_more():
+    """A step whose values have become NaN still ends soon: a chain for each output took 256 times the product's time (now 5)."""
+    a, w, out, ops = _rand(1872, 768, seed=1), _rand(768, 768, seed=2), torch.empty(1872, 768, device=DEV), _ops()
+
+    def ms(x):
+        best = 1e9
+        for _ in range(5):
+            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            s.record()
+            for _ in range(5):
+                ops.gemm_f32(x, w, None, out=out)
+            e.record()
+            e.synchronize()
+            best = min(best, s.elapsed_time(e))
+        return best
+
+    usual, nan = ms(a), ms(torch.full_like(a, float("nan")))
+    assert bool(torch.isnan(out).all()) and nan < 30 * usual
+
+
 @pytest.mark.parametrize("M,H,Hkv,D,page", [(1, 12, 12, 64, 16), (37, 10, 10, 64, 16), (300, 8, 2, 96, 8), (70, 11, 3, 60, 5)])
 def test_gemm_f32_kv_writes_the_cache(M, H, Hkv, D, page):
     """Queries, keys and values have the bits of the plain product, wherever a tile of 128 columns is cut; slots may be negative."""
