@@ -21,7 +21,7 @@ constexpr int ROT_MAX_WARPS = 32;      // of rotary_kv_kernel, where every token
 constexpr int ROT_MAX_DIM = 512;
 
 // (u, v) -> (u cos a - v sin a, v cos a + u sin a), with the roundings written out: which of the two
-// products is the fused one is then the same in every kernel
+// products is the fused one is then the same in every kernel (rotary_kv_kernel's second sum has the other one)
 __device__ __forceinline__ float turn_u(float u, float v, float cs, float sn) { return fmaf(u, cs, -__fmul_rn(v, sn)); }
 __device__ __forceinline__ float turn_v(float u, float v, float cs, float sn) { return fmaf(v, cs, __fmul_rn(u, sn)); }
 
@@ -96,7 +96,7 @@ rotary_kv_kernel(const float* x, long long x_stride, const int* __restrict__ pos
     for (int i = lane; i < half; i += 32) {
       const float cs = turn[i].x, sn = turn[i].y;
       const float u = src[i], v = src[i + half];
-      const float ru = u * cs - v * sn, rv = v * cs + u * sn;
+      const float ru = turn_u(u, v, cs, sn), rv = fmaf(u, sn, __fmul_rn(v, cs));      // (written out, for equal bits in both forms)
       b[i] = ru; b[i + half] = rv;
       ss = fmaf(ru, ru, fmaf(rv, rv, ss));
     }
@@ -441,7 +441,7 @@ qk_prep_kernel(const float* __restrict__ x, long long x_stride, const int* __res
       const float cs = turn[i].x, sn = turn[i].y;
       const int iu = pairing ? 2 * i : i, iv = pairing ? 2 * i + 1 : i + half;
       const float u = b[iu], v = b[iv];
-      const float ru = turn_u(u, v, cs, sn), rv = turn_v(u, v, cs, sn);
+      const float ru = turn_u(u, v, cs, sn), rv = fmaf(u, sn, __fmul_rn(v, cs));      // (written out, for equal bits in both forms)
       b[iu] = ru; b[iv] = rv;
       ss = fmaf(ru, ru, fmaf(rv, rv, ss));
     }

@@ -648,6 +648,32 @@ def test_rotary_rows_have_the_same_bits_beside_many_and_few_tokens():
     assert float((made[0][0][:, :D].double() - want).abs().max()) < 1e-5
 
 
+@pytest.mark.parametrize("T", [1, 148, 149])
+def test_rotary_rounds_as_it_is_written(T):
+    """u cos - v sin and u sin + v cos with the first product inside the multiply-add and the second one rounded, in each
+    form of the kernel (cosines and sines by turning rows of ones and zeros)."""
+    ops = _ops()
+    H, G, D, ps, dims = 5, 2, 64, 16, 48
+    half, width = dims // 2, (H + G) * D + G * D
+    pos, freq = torch.arange(T, dtype=torch.int32, device=DEV) * 7 + 1, torch.logspace(0, -4, half, dtype=torch.float64, device=DEV)
+
+    def run(x):
+        q, cache = torch.zeros(T, H * D, device=DEV), torch.zeros((T + ps - 1) // ps, G * ps * 2 * D, device=DEV)
+        ops.rotary_kv(x, pos, freq, 1.0, dims, None, q, cache, torch.arange(T, dtype=torch.int32, device=DEV), H, G, D, D, ps)
+        return q.view(T, H, D)
+
+    unit = torch.zeros(T, width, device=DEV)
+    unit.view(T, -1, D)[:, :, :half] = 1.0
+    turn = run(unit).double()
+    cs, sn = turn[..., :half], turn[..., half:dims]
+    x = _rand(T, width, seed=T)
+    rows = x.view(T, -1, D)[:, :H].double()
+    u, v = rows[..., :half], rows[..., half:dims]
+    got, once = run(x), lambda z: z.float().double()          # (a product of two 32-bit numbers is exact in 64 bits)
+    assert torch.equal(got[..., :half], (u * cs - once(v * sn)).float())
+    assert torch.equal(got[..., half:dims], (u * sn + once(v * cs)).float())
+
+
 @pytest.mark.parametrize("E", [4, 1020, 1024, 1028, 1664, 1668, 4096])
 def test_layer_norm_at_the_edges_of_a_blocks_warps(E):
     """Blocks of up to 8, 13 and 32 warps, whose partial sums are added in one order: the same bits in both precisions' rounding."""
