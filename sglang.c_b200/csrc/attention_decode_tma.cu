@@ -929,6 +929,11 @@ SGLC_API int sglc_attention_decode_stream_supports(int D, int page_size, int max
 // now, us with the norm's 1.9: 96 items of 700 keys (of at most 1,024) 11.4, 7.5 and of 960 12.8, 8.5; 12 of 60 5.2, 4.3; 192
 // of 200 9.2, 6.7, of 350 9.1, 7.7; 208 of 512 10.2, 9.2; 336 of 200 9.4, 7.0; 480 of 100 10.9, 6.4, of 200 15.7, 11.7; 144 of
 // 700 13.0, 11.3.
+// Of one to seven items the older rule dealt up to 32 shares, merged through memory, where eight in a cluster are the faster: one
+// item of 1,024 / 2,048 / 4,096 keys 9.9, 6.3 / 11.1, 7.5 / 11.1, 10.0; seven 10.1, 6.5 / 12.1, 7.8 / 12.4, 10.3.  Contexts
+// of 1,100 to 4,000 keys (12 to 500 items, alike and ragged): a second round of clusters costs what a first one does there; with
+// the factor of the shorter ones 48 items of 3,200 went to the streaming kernel in 28.1 (eight shares 19.7), 96 ragged ones
+// of up to 2,048 in 19.7 (16.9).  As it is, it is 1 % from the best of each of 175 such launches.
 SGLC_API int sglc_attention_decode_form(int T, int H, int D, int page_size, int max_keys, int window) {
   if (D != 64 || page_size < 1 || page_size > 64 || (page_size * D * 2) % 128 != 0 || T <= 0 || H <= 0 || max_keys <= 0) return -1;
   const long long n = (long long)T * H;
@@ -956,7 +961,7 @@ SGLC_API int sglc_attention_decode_form(int T, int H, int D, int page_size, int 
     const int at_once = (int)(148 * here * (s == 1 ? 1.0 : s == 2 ? 0.97 : s == 3 ? 0.92 : 0.88));
     const long long blocks = n * s, rounds = (blocks + at_once - 1) / at_once;
     double us = (double)rounds * ((s == 1 ? 3.5 : 4.75) + 0.0135 * keys / s) + 0.0027 * (double)(blocks < at_once ? blocks : at_once);
-    if (rounds > 1 && s > 1) us *= 1.7;               // (clusters of a second round wait for whole groups of places)
+    if (rounds > 1 && s > 1 && eff <= 1024) us *= 1.7;      // (clusters of a second round wait for whole groups of places)
     if (s == dealt) us -= 0.3;
     if (us < best_us) {
       best_us = us;
