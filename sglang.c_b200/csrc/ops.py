@@ -1612,14 +1612,15 @@ GATE_ACTS = {"silu": 0, "gelu_tanh": 1, "clamped": 2}
 
 
 def gated_act(src, dst, weights=None, per=0, act="silu", mult=1.0, n_weighted=None, handed_on=None, slope=None,
-              limit=None):
+              limit=None, sparse=True):
     """dst[r, j] = act(src[r, j]) * src[r, F + j] (* weights[r, j // per]) * mult; src [rows, 2F] holds
     the gate columns, then the up columns; weights: float32 [rows, F // per] or None; act "silu" or
     "gelu_tanh", or "clamped" (dst = g sigmoid(slope g) (u + 1) with g = min(gate, limit), u = up held within
     +-limit; without weights); mult: one more factor of every result, taken in 32-bit.  n_weighted: only the
     first so many columns (a multiple of per) take weights, [rows, n_weighted // per]; the rest take 1.
     handed_on = (h, w, x, add): the same launch forms x[r, :] = w[r] * h[r, :] (added to x if `add`);
-    h [rows, E] in dst's dtype, w float32 [rows], x float32 [rows, E]."""
+    h [rows, E] in dst's dtype, w float32 [rows], x float32 [rows, E].  sparse: whether a quarter of the weights and more are
+    expected to be 0 (it decides which kernel works, no more)."""
     _need_cuda(src, dst, weights)
     rows, F = dst.shape
     if src.shape[1] != 2 * F or src.shape[0] < rows or src.stride(1) != 1 or dst.stride(1) != 1:
@@ -1652,14 +1653,14 @@ def gated_act(src, dst, weights=None, per=0, act="silu", mult=1.0, n_weighted=No
             _ptr(src), ctypes.c_longlong(src.stride(0)), _dt(src, "gated_act source"), _ptr(dst),
             ctypes.c_longlong(dst.stride(0)), _dt(dst, "gated_act destination"), rows, F, _ptr(weights),
             ctypes.c_longlong(weights.stride(0) if weights is not None else 0), int(per), GATE_ACTS[act],
-            ctypes.c_float(mult), nw, _ptr(h), ctypes.c_longlong(h.stride(0)), _ptr(w), _ptr(x),
+            ctypes.c_float(mult), nw, 1 if sparse else 0, _ptr(h), ctypes.c_longlong(h.stride(0)), _ptr(w), _ptr(x),
             ctypes.c_longlong(x.stride(0)), h.shape[1], 1 if add else 0, _stream())
         _check(lib, code, "gated_act")
         return
     code = lib.sglc_gated_act_part(_ptr(src), ctypes.c_longlong(src.stride(0)), _dt(src, "gated_act source"), _ptr(dst),
                                    ctypes.c_longlong(dst.stride(0)), _dt(dst, "gated_act destination"), rows, F,
                                    _ptr(weights), ctypes.c_longlong(weights.stride(0) if weights is not None else 0),
-                                   int(per), GATE_ACTS[act], ctypes.c_float(mult), nw, _stream())
+                                   int(per), GATE_ACTS[act], ctypes.c_float(mult), nw, 1 if sparse else 0, _stream())
     _check(lib, code, "gated_act")
 
 

@@ -212,11 +212,11 @@ class RoutedExperts(Part):
         self.gate_up.forward(ctx, h, out=gu)
         a = ctx.alloc((T, Fall), self.rt.act_dtype)
         if not n_id:
-            ops.gated_act(gu, a, weights=dense, per=F, n_weighted=X * F)
+            ops.gated_act(gu, a, weights=dense, per=F, n_weighted=X * F, sparse=4 * top < 3 * X)
             return self.down.forward(ctx, a, out=out, residual=residual)
         # the identity experts' share goes into the stream (or begins the result), the products add to it
         add = residual is not None
         dst = residual if add else out
         ops.gated_act(gu, a, weights=ctx.columns(dense, 0, X), per=F, n_weighted=X * F,
-                      handed_on=(h, passed, dst[:T], add))
+                      handed_on=(h, passed, dst[:T], add), sparse=4 * top < 3 * (X + n_id))
         return self.down.forward(ctx, a, residual=dst)
