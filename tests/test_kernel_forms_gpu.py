@@ -589,6 +589,22 @@ def test_gated_activations_skip_what_was_not_chosen():
     assert torch.equal(dst, clean) and bool((dst[hole] == 0).all())
 
 
+@pytest.mark.parametrize("rows", [(1 << 30) - 1, (1 << 30) + 5])
+def test_gated_activations_of_a_billion_pieces(rows):
+    """The counters of 32 and of 64 bits on both sides of 2^30 pieces: one piece a row, all rows alike (17 GB of results)."""
+    ops = _ops()
+    one = _rand(1, 16, dtype=torch.bfloat16, seed=1)
+    dst = torch.empty(rows, 8, dtype=torch.bfloat16, device=DEV)
+    for act in ("silu", "gelu_tanh"):
+        for w in (None, torch.full((1, 1), 0.5, device=DEV)):
+            dst.fill_(float("nan"))
+            want = torch.empty(1, 8, dtype=torch.bfloat16, device=DEV)
+            ops.gated_act(one, want, weights=w, per=8, act=act)
+            ops.gated_act(one.expand(rows, 16), dst, weights=None if w is None else w.expand(rows, 1), per=8, act=act)
+            for part in dst.view(torch.int64).split(1 << 28):
+                assert bool((part == want.view(torch.int64)).all())
+
+
 @pytest.mark.parametrize("E,groups,form", [(4, 1, "rms"), (512, 1, "layer"), (128, 6, "rms"), (1028, 1, "layer"), (2044, 1, "rms"), (2048, 2, "layer"),
                                            (4096, 1, "rms"), (4100, 1, "layer")])
 def test_norms_of_a_few_rows(E, groups, form):
@@ -631,6 +647,31 @@ def test_router_makes_its_logits(E, K, T):
     # a logit's error is below 2^-24 times the sum of its products' sizes times the additions a lane makes; near ties may fall either way
     assert float((wts.double() - best.values).abs().max()) < 1e-5
     assert float((dense.gather(1, ids.long()).double() - torch.gather(s, 1, ids.long())).abs().max()) < 1e-5
+
+
+@pytest.mark.parametrize("E,K", [(1, 520), (8, 769), (32, 64), (33, 769), (40, 520)])
+def test_router_makes_its_logits_in_32_bits(E, K):
+    """The 32-bit product: the end of a row inside the loads on their way at once; and a token's weights have the same bits in
+    a launch of 149 tokens, which share SMs, as in launches of a few."""
+    ops = _ops()
+    T, top = 149, min(E, 3)
+    h, w = _rand(T, K + 4, seed=K)[:, :K], _rand(E, K, seed=E) / K ** 0.5
+
+    def run(lo, hi):
+        n = hi - lo
+        dense, ids, wts = torch.empty(n, E, device=DEV), torch.empty(n, top, dtype=torch.int32, device=DEV), torch.empty(n, top, device=DEV)
+        ops.router(None, None, dense, ids, wts, top, rows=h[lo:hi], matrix=w)
+        return dense, ids, wts
+
+    whole = run(0, T)
+    parts = [run(lo, hi) for lo, hi in ((0, 1), (1, 9), (9, T))]
+    for i in range(3):
+        assert torch.equal(whole[i], torch.cat([p[i] for p in parts]))
+    s = torch.sigmoid(h.double() @ w.double().t())
+    best = torch.topk(s, top, dim=1)
+    # a lane adds up to 25 products and the warp 5 times, 2^-24 of sums below 4 each; a near tie may fall either way
+    assert float((whole[2].double() - best.values).abs().max()) < 4 * 30 * 2.0 ** -24
+    assert float((whole[0].gather(1, whole[1].long()).double() - torch.gather(s, 1, whole[1].long())).abs().max()) < 4 * 30 * 2.0 ** -24
 
 
 @pytest.mark.parametrize("D,V,splits", [(64, 64, 2), (64, 40, 8), (128, 72, 9), (256, 256, 11)])
