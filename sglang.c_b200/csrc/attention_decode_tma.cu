@@ -933,7 +933,7 @@ SGLC_API int sglc_attention_decode_stream_supports(int D, int page_size, int max
 // item of 1,024 / 2,048 / 4,096 keys 9.9, 6.3 / 11.1, 7.5 / 11.1, 10.0; seven 10.1, 6.5 / 12.1, 7.8 / 12.4, 10.3.  Contexts
 // of 1,100 to 4,000 keys (12 to 500 items, alike and ragged): a second round of clusters costs what a first one does there; with
 // the factor of the shorter ones 48 items of 3,200 went to the streaming kernel in 28.1 (eight shares 19.7), 96 ragged ones
-// of up to 2,048 in 19.7 (16.9).  As it is, it is 1 % from the best of each of 175 such launches.
+// of up to 2,048 in 19.7 (16.9).  As it is, it is 1 % on average from the best of each of 160 such launches.
 SGLC_API int sglc_attention_decode_form(int T, int H, int D, int page_size, int max_keys, int window) {
   if (D != 64 || page_size < 1 || page_size > 64 || (page_size * D * 2) % 128 != 0 || T <= 0 || H <= 0 || max_keys <= 0) return -1;
   const long long n = (long long)T * H;

@@ -141,7 +141,7 @@ gated_norm_quads_kernel(const float* o, long long o_stride, const float* gate, l
     auto out = [&](float x, float gt, float gn) {
       x = x * inv * gn;
       if (act == GN_NONE) return x;
-      float e;                       // (of the fast kind, a few 2^-23: the result is rounded to 2^-9)
+      float e;                       // (of the fast kind, as in elementwise.cu: silu_fast; the result is rounded to 2^-9)
       asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-gt * 1.4426950408889634f));
       return x * __fdividef(act == GN_SILU ? gt : 1.0f, 1.0f + e);
     };

@@ -43,7 +43,7 @@ using namespace sglc;
 // constants the Python engine shares (csrc/ops.py)
 constexpr long long TC_WS_FLOATS = 8ll << 20;      // split-K partial sums of the decode attention's merge
 constexpr int TC_COUNTERS = 8192;
-constexpr int STREAM_MIN_ITEMS = 160;              // (token, head) items from which the streaming decode kernel is used
+constexpr int STREAM_MIN_ITEMS = 160;              // (csrc/ops.py)
 constexpr int FEW_MAX_TOKENS = 2;
 constexpr long long FEW_MAX_WEIGHT = 3ll << 20;
 constexpr int ORDER_SPREAD = 64;                   // contexts that differ by a stage of keys: their order matters
@@ -769,7 +769,7 @@ class DeviceRunner : public StepRunner {
   // graph serves until the contexts pass it): the next power of two; a step of single tokens in
   // few (token, head) items goes to the decode attention whose blocks' shared memory is sized by
   // the bound, and there it moves in steps of 128 keys up to 1024 and of about an eighth of the
-  // length beyond (parts/attention.py: graph_bound).
+  // length beyond; of more items, whichever kernel takes them, in powers of two (parts/attention.py: graph_bound).
   int graph_bound(const WalkStep& s) const {
     int bound = 128;
     while (bound < s.max_keys) bound *= 2;

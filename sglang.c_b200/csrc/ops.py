@@ -516,7 +516,9 @@ def gemm_few(a, w, bias, out=None, residual=None, act=None):
 
 
 # ---------------------------------------------------------------------------
-STREAM_MIN_ITEMS = 160     # (token, head) items from which the streaming decode kernel is used
+# (token, head) items from which the streaming decode kernel is used where sglc_attention_decode_form has no answer, and from
+# which a step's bound on its keys moves in powers of two (parts/attention.py: graph_bound)
+STREAM_MIN_ITEMS = 160
 USE_TMA_DECODE = True      # tests switch it off to reach the register-staged kernel at head size 64/128
 
 

@@ -40,7 +40,7 @@ typedef struct sglc_sampling {
 
 typedef struct sglc_engine_options {
   int device;                     /* CUDA device index */
-  int bf16;                       /* 1: bfloat16 weights, activations and cache; 0: everything in true 32-bit */
+  int bf16;                       /* 1: bfloat16 weights, activations and cache; 0: everything held and summed in 32-bit */
   int page_size;                  /* positions per cache page */
   long long n_pages;              /* pages of the pool; 0: enough for max_tokens positions */
   long long max_tokens;           /* used when n_pages is 0; 0 as well: max_requests full-length requests */

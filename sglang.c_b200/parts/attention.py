@@ -49,7 +49,8 @@ class CausalAttention(Part):
         # stages a block's whole key range in shared memory sized by the bound, and what a block
         # holds of an SM decides whether it can start, and prefetch, while the kernels ahead still
         # run: there the bound moves in steps of 128 keys up to 1024 and of about an eighth of the
-        # length beyond (a capture every 128 steps costs less than the tighter bound wins).
+        # length beyond (a capture every 128 steps costs less than the tighter bound wins).  Of more
+        # items some go to that kernel as well (csrc/ops.py: attention_decode), with the bound in powers of two.
         from ..csrc import ops
         if ctx.n_decode == ctx.T and ctx.T * self.params["n_heads"] < ops.STREAM_MIN_ITEMS:
             g = 128
