@@ -112,34 +112,55 @@ __device__ __forceinline__ void tmem_st_16x256b_x1(uint32_t taddr, uint32_t a, u
                : "memory");
 }
 __device__ __forceinline__ bool finite(float s) { return fabsf(s) <= 3.402823466e38f; }
-// T tokens' outputs (of which `tokens` exist) as plain chains of multiply-adds, k = 0..K-1 each.
-template <int T> struct Sums { float v[T]; };
-template <int T>
-__device__ __noinline__ Sums<T> plain_sums(const float* a, int lda, int tokens, const float* w, int K) {
-  const float4* row[T];
-#pragma unroll
-  for (int j = 0; j < T; j++) row[j] = reinterpret_cast<const float4*>(a + (size_t)min(j, tokens - 1) * lda);
-  Sums<T> s = {};
-#pragma unroll 8 / T + 2
+// An output as a plain chain of multiply-adds, k = 0..K-1.  (Few loads at once: a function that takes more registers
+// costs the kernels that call it 2 % where none is called.)
+__device__ __noinline__ float plain_dot(const float* a, const float* w, int K) {
+  float s = 0.0f;
+#pragma unroll 2
   for (int k = 0; k < K / 4; k++) {
-    const float4 y = reinterpret_cast<const float4*>(w)[k];
-#pragma unroll
-    for (int j = 0; j < T; j++) {
-      const float4 x = row[j][k];
-      s.v[j] = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s.v[j]))));
-    }
+    const float4 x = reinterpret_cast<const float4*>(a)[k], y = reinterpret_cast<const float4*>(w)[k];
+    s = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s))));
   }
   return s;
 }
 // Whether there is a NaN among the 16-byte pieces first, first + step, ... of a row.
-__device__ __noinline__ bool any_nan(const float* row, int K, int first, int step) {
+__device__ __forceinline__ bool any_nan(const float* row, int K, int first, int step) {
   bool nan = false;
-#pragma unroll 8
+#pragma unroll 4
   for (int k = first; k < K / 4; k += step) {
     const float4 x = reinterpret_cast<const float4*>(row)[k];
     nan = nan || x.x != x.x || x.y != x.y || x.z != x.z || x.w != x.w;
   }
   return nan;
+}
+// A token's outputs of a warp's features (a row of w each) that are no finite numbers, made again (v where `bad` is false).  A NaN among
+// the token's numbers, which the warp looks for together, or among a feature's makes the output NaN without a chain: in a step
+// whose values have become NaN a chain for every output took hundreds of times the tile (1,872 tokens, 768 over 768 5.4 ms,
+// now 0.09, with a NaN in each row of w 0.12, and 0.02 where all is finite; 768 over 3,072 22.4 ms, now 0.25).  w_nan: what
+// was found out about the lane's row of w; -1: nothing yet.
+struct Again { float v; int w_nan; };
+__device__ __noinline__ Again plain_again(const float* a, const float* w, int K, bool bad, float v, int w_nan) {
+  const bool a_nan = __any_sync(0xffffffffu, any_nan(a, K, threadIdx.x & 31, 32));
+  if (bad) {
+    if (!a_nan && w_nan < 0) w_nan = any_nan(w, K, 0, 1);
+    v = a_nan || w_nan > 0 ? __int_as_float(0x7fffffff) : plain_dot(a, w, K);
+  }
+  __syncwarp();
+  return {v, w_nan};
+}
+// The same where blocks share a tile, whose outputs are few: given up where it has become NaN (8 tokens, 768 over 3,072, all NaN
+// 236 -> 17 us).
+__device__ __noinline__ float plain_until_nan(const float* a, const float* w, int K) {
+  float s = 0.0f;
+  for (int k0 = 0; k0 < K && s == s; k0 += FK) {
+    const int n = min(FK, K - k0) / 4;
+#pragma unroll 4
+    for (int k = 0; k < n; k++) {
+      const float4 x = reinterpret_cast<const float4*>(a + k0)[k], y = reinterpret_cast<const float4*>(w + k0)[k];
+      s = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, s))));
+    }
+  }
+  return s;
 }
 
 // Blocks walk tiles (features fastest), all of K each; or, CLUSTER, the blocks of a cluster share one tile: rank r takes the
@@ -455,19 +476,21 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 #pragma unroll
         for (int j = 0; j < CW; j++) all = all && finite(sum[j]);
         if (__any_sync(0xffffffffu, !all)) {
-          // A NaN among a token's numbers, which the warp looks for together, or a feature's makes the output NaN without a
-          // chain: in a step whose values have become NaN a chain for every output would take a hundred times the tile.
-          int w_nan = -1;                               // (not looked for yet)
+          int w_nan = -1;
+          float kept[CW];                               // (in memory: a loop that is not unrolled is the least code beside the usual path)
 #pragma unroll
+          for (int j = 0; j < CW; j++) kept[j] = sum[j];
+#pragma unroll 1
           for (int j = 0; j < CW; j++) {
-            const bool bad = f < p.N && mt + j < p.M && !finite(sum[j]);
+            const float v = kept[j];
+            const bool bad = f < p.N && mt + j < p.M && !finite(v);
             if (!__any_sync(0xffffffffu, bad)) continue;
-            const float *a = p.A + (size_t)(mt + j) * p.lda, *w = p.W + (size_t)f * p.K;
-            const bool a_nan = __any_sync(0xffffffffu, any_nan(a, p.K, lane, 32));
-            if (!bad) continue;
-            if (!a_nan && w_nan < 0) w_nan = any_nan(w, p.K, 0, 1);
-            sum[j] = a_nan || w_nan > 0 ? __int_as_float(0x7fffffff) : plain_sums<1>(a, p.lda, 1, w, p.K).v[0];
+            const Again again = plain_again(p.A + (size_t)(mt + j) * p.lda, p.W + (size_t)f * p.K, p.K, bad, v, w_nan);
+            kept[j] = again.v;
+            w_nan = again.w_nan;
           }
+#pragma unroll
+          for (int j = 0; j < CW; j++) sum[j] = kept[j];
         }
         if (p.act != SGLC_ACT_NONE) {
 #pragma unroll
@@ -544,16 +567,11 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
           }
         }
         float v[4] = {s.x, s.y, s.z, s.w};
-        if (m0 + col < p.M && !(finite(v[0]) && finite(v[1]) && finite(v[2]) && finite(v[3]))) {
-          const Sums<4> c = plain_sums<4>(p.A + (size_t)(m0 + col) * p.lda, p.lda, min(4, p.M - m0 - col), p.W + (size_t)f * p.K, p.K);
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (!finite(v[j])) v[j] = c.v[j];
-        }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const int m = m0 + col + j;
           if (m >= p.M) break;
+          if (!finite(v[j])) v[j] = plain_until_nan(p.A + (size_t)m * p.lda, p.W + (size_t)f * p.K, p.K);
           const float y = apply_act(v[j] + bias, p.act);
           if (p.cache && f >= p.q_cols) {
             const long long at = slot_at(p, m);
@@ -707,11 +725,13 @@ static int start(F32Args& p, cudaStream_t stream) {
 }
 
 // Whether the 32-bit path takes this kernel for a product (else gemm_simt.cu).  Nothing here follows the number of rows, so
-// that a token's results do not either.  From K = 640 on it is the faster one nearly everywhere; below, a step of few rows
-// would lose more than it is worth (us, the kernels of gemm_simt.cu and this one, at 8, 64 and 1,872 rows: 1,024 columns
-// over K 512 3.8 / 4.9, 9.6 / 6.1, 62.5 / 17.3; 768 over 768 4.5 / 5.1, 12.7 / 6.6, 69.3 / 19.3; 2,304 over 768 6.3 / 6.1,
-// 16.2 / 11.5, 154 / 40; 768 over 3,072 12.6 / 8.0, 40.6 / 13.3, 249 / 61; 1,600 over 1,600 10.7 / 7.6, 25.2 / 13.1,
-// 259 / 64; 50,257 over 768 41.8 / 35.0, 195 / 45).
+// that a token's results do not either.  From K = 640 on it is the faster one at most sizes, and a few rows over K 640 to
+// 768 are what it loses at; below, a step of few rows would lose more than it is worth (us, the kernels of gemm_simt.cu and
+// this one, at 8, 64 and 1,872 rows: 1,024 columns over K 512 3.8 / 4.9, 9.6 / 6.1, 62.5 / 17.3; 768 over 768 4.5 / 5.1, 12.7
+// / 6.6, 69.3 / 19.3; 2,304 over 768 6.3 / 6.1, 16.2 / 11.5, 154 / 40; 768 over 3,072 12.6 / 8.0, 40.6 / 13.3, 249 / 61;
+// 1,600 over 1,600 10.7 / 7.6, 25.2 / 13.1, 259 / 64; 50,257 over 768 41.8 / 35.0, 195 / 45).  Narrow products, behind a layer norm
+// of 1.9: 12 columns over K 640 5.9 / 6.7, 6.6 / 6.9, 23.6 / 14.1; over 768 6.2 / 6.1, 7.2 / 6.5, 26.9 / 15.0; over 3,072 13.8 /
+// 8.1, 19.1 / 8.5, 70.7 / 63.6; and 768 over 640 5.7 / 7.2, 12.5 / 8.2, 60 / 18.
 SGLC_API int sglc_gemm_f32_supports(int N, int K, int lda) { return K % 4 == 0 && lda % 4 == 0 && K >= 640; }
 
 // A: [M,K] with row stride lda (elements); W: [N,K] contiguous; bias: float[N] or null; all 32-bit.  If `residual` is
