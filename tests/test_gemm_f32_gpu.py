@@ -34,8 +34,10 @@ def _each(run):
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (15, 127, 60), (17, 129, 64), (33, 128, 68), (129, 300, 772), (200, 65, 1604), (9, 257, 3076),
                                    (97, 20000, 8)])
 def test_gemm_f32_forms_give_the_same_bits(M, N, K):
-    """Remainders of rows, features, k and chunks.  Error: 16 roundings at most inside a chunk and one a chunk, of 2^-23 of sums
-    that stay below sum |a w| (tensor memory cuts), and 2^-21 of each product left out or cut."""
+    """Remainders of rows, features, k and chunks.  An output's error at most: 24 additions into a chunk's sum, which tensor memory
+    cuts, so 2^-23 of the sum of the chunk's |a w| each; 2^-24 of the whole sum a chunk; 2^-21 of each product left out or cut.
+    All outputs' together: 5e-7 of sqrt(sum (a w)^2), three times the most seen; without one of the six products of pieces
+    it is 4e-6 and more."""
     wide = _rand(M, K + 12, seed=M)
     a, w, bias = wide[:, 4:4 + K], _rand(N, K, seed=N), _rand(N, seed=K)
     ref = a.double() @ w.double().t() + bias.double()
@@ -55,10 +57,14 @@ def test_gemm_f32_forms_give_the_same_bits(M, N, K):
     for out, act in each[1:]:
         assert torch.equal(out, each[0][0]) and torch.equal(act, each[0][1])
     out, act = each[0]
-    scale = float((a.double().abs() @ w.double().abs().t() + bias.double().abs()).max())
-    bound = scale * (2.0 ** -23 * (16 + (K + 63) // 64) ** 0.5 + 2.0 ** -21)
-    assert float((out.double() - ref).abs().max()) < bound
-    assert float((act.double() - torch.nn.functional.gelu(ref, approximate="tanh")).abs().max()) < 1.2 * bound + 1e-6
+    scale = a.double().abs() @ w.double().abs().t() + bias.double().abs()
+    bound = scale * (24 * 2.0 ** -23 + ((K + 63) // 64) * 2.0 ** -24 + 2.0 ** -21)
+    assert bool(((out.double() - ref).abs() < bound).all())
+    assert bool(((act.double() - torch.nn.functional.gelu(ref, approximate="tanh")).abs() < 1.2 * bound + 1e-6).all())
+    plain = torch.empty(M, N, device=DEV)
+    _ops().gemm_f32(a, w, None, out=plain)
+    size = (a.double() ** 2 @ (w.double() ** 2).t()).sum().sqrt()
+    assert float((plain.double() - a.double() @ w.double().t()).norm() / size) < 5e-7
 
 
 def test_gemm_f32_is_closer_than_a_chain_of_multiply_adds():
