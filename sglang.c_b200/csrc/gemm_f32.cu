@@ -186,7 +186,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   uint8_t* a_ring = w_ring + W_STAGES * W_BYTES;        // two chunks of A likewise
   float* red = reinterpret_cast<float*>(a_ring + 2 * A_BYTES);             // the sums of all chunks for this block's features
   __shared__ uint64_t ready[2], done[2], read[2],       // a chunk is cut, its MMAs have ended, its sums have been taken
-       w_full[W_STAGES], w_empty[W_STAGES], a_full[2], a_empty[2];
+       w_full[W_STAGES], w_empty[W_STAGES], a_full[2], a_empty[2],
+       taken;                                           // (CLUSTER) all chunks' sums have been taken
   __shared__ uint32_t tmem_s;
   __shared__ int abort_s;
   volatile int* abort_flag = &abort_s;
@@ -209,9 +210,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
       mbar_init(&w_full[i], 1);
       mbar_init(&w_empty[i], WW);
     }
+    mbar_init(&taken, DW);
     abort_s = 0;
     mbar_fence_init();
   }
+  __syncwarp();
+  // A block of a cluster never waits for another one while it holds tensor memory, except for its start, and that is ahead of
+  // the allocation: the columns are given back before the blocks wait for one another's sums.  Otherwise two clusters of
+  // launches in two streams, this kernel's and one of bfloat16 products, could each hold on one SM what the other one's
+  // block waits for there, for good.
+  if (CLUSTER) cluster_arrive_relaxed();                // (waited for ahead of the first store into a peer's memory)
   if (warp == 0) {
     tmem_alloc(&tmem_s, COLS);
     tmem_relinquish();
@@ -222,9 +230,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   // Behind the allocation: blocks of the launch behind, which hold tensor memory while they wait for this one, come
   // only when every block of this one has its own.
   pdl_launch_dependents();
-  if (CLUSTER) cluster_arrive();                        // (waited for ahead of the first store into a peer's memory)
   const uint32_t tmem = tmem_s;
   const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
+  bool held = true;                                     // (warp 0: the columns)
 
   if (warp < WW) {
     // ---- cut W ----
@@ -457,6 +465,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
         __syncwarp();
         if (lane == 0) mbar_arrive(&read[st]);
         if constexpr (CLUSTER) {
+          if (i == n - 1 && lane == 0) mbar_arrive(&taken);
           if (!peers) {
             cluster_wait();
             peers = true;
@@ -551,6 +560,14 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     __syncwarp();
     if (!fin) cluster_wait();                           // (the adding warps have waited for the peers' start)
     cluster_arrive();
+    if (warp == 0) {
+      const bool all = mbar_wait(&taken, 0, abort_flag);
+      if (__all_sync(0xffffffffu, all && !*abort_flag)) {
+        held = false;
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, COLS);
+      }
+    }
     cluster_wait();
     if (!*abort_flag)
       for (int x = t; x < items; x += FIN) {
@@ -583,7 +600,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
   }
   __syncthreads();
   if (tid == 0 && *abort_flag) atomicOr(p.err, SGLC_FLAG_WAIT);
-  if (warp == 0) tmem_dealloc(tmem, COLS);
+  if (warp == 0 && held) tmem_dealloc(tmem, COLS);
 }
 
 constexpr size_t MOST_SMEM = 226 * 1024, TWO_SMEM = 112 * 1024;      // a block's at most; and where two share an SM

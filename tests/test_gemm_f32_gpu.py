@@ -148,6 +148,37 @@ def test_gemm_f32_of_nan_takes_a_few_times_the_time_and_no_more():
     assert bool(torch.isnan(out).all()) and nan < 30 * usual
 
 
+def test_gemm_f32_in_clusters_beside_clusters_of_another_stream():
+    """Blocks that share a tile's K (320 to 512 of an SM's 512 columns of tensor memory) while few-token bfloat16 products, whose
+    blocks share K too, run in another stream: a block gives its columns back before it waits for its peers."""
+    ops, lib = _ops(), _lib()
+    a, w = _rand(64, 768, seed=1), _rand(768, 768, seed=2)
+    b, v = _rand(8, 768, seed=3).bfloat16(), _rand(768, 768, seed=4).bfloat16()
+    n = 200
+    outs = [torch.empty(64, 768, device=DEV) for _ in range(n)]
+    halves = [torch.empty(8, 768, dtype=torch.bfloat16, device=DEV) for _ in range(n)]
+    want, half = torch.empty_like(outs[0]), torch.empty_like(halves[0])
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    try:
+        for form in ((64, 6), (64, 12), (32, 8), (16, 6)):
+            lib.sglc_gemm_f32_set_form(*form)
+            try:
+                ops.gemm_f32(a, w, None, out=want)
+            except ops.KernelError:
+                continue
+            ops.gemm_tc(b, v, None, out=half)
+            torch.cuda.synchronize()
+            for i in range(n):
+                with torch.cuda.stream(one):
+                    ops.gemm_f32(a, w, None, out=outs[i])
+                with torch.cuda.stream(two):
+                    ops.gemm_tc(b, v, None, out=halves[i])
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, want) for o in outs) and all(torch.equal(h, half) for h in halves)
+    finally:
+        lib.sglc_gemm_f32_set_form(0, 0)
+
+
 @pytest.mark.parametrize("M,H,Hkv,D,page", [(1, 12, 12, 64, 16), (37, 10, 10, 64, 16), (300, 8, 2, 96, 8), (70, 11, 3, 60, 5)])
 def test_gemm_f32_kv_writes_the_cache(M, H, Hkv, D, page):
     """Queries, keys and values have the bits of the plain product, wherever a tile of 128 columns is cut; slots may be negative."""
