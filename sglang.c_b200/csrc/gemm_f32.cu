@@ -606,8 +606,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
 constexpr size_t MOST_SMEM = 226 * 1024, TWO_SMEM = 112 * 1024;      // a block's at most; and where two share an SM
 constexpr size_t smem_bytes(int NT, bool cluster, int chunks, int ranks) {
   const size_t rows_per = (FM + ranks - 1) / ranks;
-  // No more blocks on an SM than its tensor memory serves (two of 256 columns, one of 512): a block that waited for
-  // columns would keep its cluster's other blocks, and through them the columns' owners, waiting.
+  // No more blocks on an SM than its tensor memory serves (two of 256 columns, one of 512): one more would only wait for
+  // columns, and keep its cluster's other blocks waiting.
   const size_t least = NT <= 32 ? 76 * 1024 : 114 * 1024;
   const size_t sums = cluster ? chunks * rows_per * (NT + 4) * 4 : 0;
   const size_t need = 1024 + 2 * 3 * NT * 128 + (NT >= 64 ? 2 * NT * FK * 4 : 0) + (cluster || NT == 128 || NT == 16 ? 2 : 3) * W_BYTES + sums;
